@@ -788,11 +788,16 @@ __global__ void k_add_f32(size_t n, double* __restrict__ x, const float* __restr
         x[k] += (double)e[k];
 }
 
-__global__ void k_shift(size_t n, double* __restrict__ x, int pin, const DevScalars* S) {
+// p = x + the constant that puts the pinned cell at its value.  x is only read: every block takes
+// the shift from x[pin], so a block that starts after another has finished must still find the
+// unshifted value there (many small solves at once, as in an ensemble, do start blocks late).
+// Bandwidth-bound, 16 B per cell; it takes the place of an in-place shift and a copy.
+__global__ void k_shift(size_t n, const double* __restrict__ x, double* __restrict__ p, int pin,
+                        const DevScalars* __restrict__ S) {
     pdl_enter();
-    double s = S->pin_value - x[pin];
+    const double s = S->pin_value - x[pin];
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        x[k] += s;
+        p[k] = x[k] + s;
 }
 
 // y = A_ref x (reference pinned matrix) from the device operator.
@@ -1726,18 +1731,18 @@ impec_status pressure_iteration(impec_ctx* ctx, double tol, cudaGraphConditional
     return IMPEC_OK;
 }
 
-// Constant shift to the pinned value and copy to p (launch only).  With CG the reported relres
-// is the true one, from the k_cg_verify that ended the loop.
+// The iterate, shifted by a constant to the pinned value, into p (launch only).  With CG the
+// reported relres is the true one, from the k_cg_verify that ended the loop.
 impec_status pressure_finish(impec_ctx* ctx, double* p) {
-    Level& F = ctx->L[0];
-    const size_t n = F.n();
+    const size_t n = ctx->L[0].n();
     double* x = solve_iterate(ctx);
     if (ctx->singular) {  // the constant that puts the pinned cell at its value
         ++ctx->nlaunch;
-        launch_k(ctx->stream, k_shift, ctx->num_sms * 4, 256, 0, n, x, pin_index(ctx), ctx->dscal);
+        launch_k(ctx->stream, k_shift, ctx->num_sms * 4, 256, 0, n, (const double*)x, p, pin_index(ctx), ctx->dscal);
+        IMPEC_LAUNCH_CHECK();
+    } else {
+        IMPEC_CUDA_TRY(cudaMemcpyAsync(p, x, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    IMPEC_LAUNCH_CHECK();
-    IMPEC_CUDA_TRY(cudaMemcpyAsync(p, x, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     return IMPEC_OK;
 }
 
