@@ -73,14 +73,16 @@ struct Level {
     // FP64 operator (integrated, positive-definite sign convention)
     double* tx = nullptr;    // FACE5: (n1+1)*n2 x-face transmissibilities (boundary faces 0)
     double* ty = nullptr;    // FACE5: n1*(n2+1)
-    double* a9 = nullptr;    // EXP9: 9 planes of n1*n2, folded (no coupling outside the grid)
+    double* a9 = nullptr;    // EXP9: 9 planes of n1*n2, folded (no coupling outside the grid); on a
+                             // FACE5 finest level: the nine-point system that the levels precondition
     double* idiag = nullptr; // 1 / diagonal
     double* diag = nullptr;  // diagonal (FACE5: sum of the four faces + ed; EXP9: plane 0)
     double* ed = nullptr;    // FACE5 with a Dirichlet row: couplings to known cells, moved to the diagonal
     double *x = nullptr, *b = nullptr;
+    double* w4 = nullptr;    // FACE5 below the finest: transfer weights towards E, W, N, S (4 planes of n1*n2)
     // FP32 copies for the mixed-precision cycle
     float *tx32 = nullptr, *ty32 = nullptr, *a932 = nullptr, *idiag32 = nullptr, *diag32 = nullptr;
-    float *x32 = nullptr, *b32 = nullptr;
+    float *x32 = nullptr, *b32 = nullptr, *w432 = nullptr;
     // second iterate buffers of the one-launch red-black sweep (ping-pong; FACE5 levels)
     double* xa = nullptr;
     float* xa32 = nullptr;
@@ -124,7 +126,8 @@ struct DevScalars {
     double fsum, fnorm2, rnorm2, pin_value;  // fsum,fnorm2 adjacent: written as a pair
     double red[8];
     double relres, cn_relres, t_clip;
-    double pcg_rz, pcg_zq;  // (r, z) and (z, q_old) of the current CG iteration (written as a pair)
+    // (r, z), (z, q_old) and the sums of z and r of the current CG iteration (written together)
+    double pcg_rz, pcg_zq, pcg_zsum, pcg_rsum;
     double pcg_pq, pcg_alpha, pcg_rz_old;
     // the iteration's beta (for the direction) and alpha (for the update), each computed once by
     // the last block of the reduction that completes its operands instead of in every thread

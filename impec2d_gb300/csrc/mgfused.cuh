@@ -8,8 +8,8 @@
 
 constexpr int MGC_MAXL = 8;
 
-// Coarsest-level solve x = Dinv b' in FP64 (n <= 64), b' = b with b(0) := 0 for the singular
-// system (whose Dinv, from k_dense_invert, already removes the mean of the result).  Every
+// Coarsest-level solve x = Dinv b in FP64 (n <= 64; for the singular system Dinv, from
+// k_dense_invert, is its pseudo-inverse).  Every
 // thread of the block takes part (the count of loop trips and shuffles is the same for all):
 // row r is summed by the 8 lanes of one lane group, lane g over the columns g, g + 8, g + 16,
 // ... in ascending order; an xor butterfly then adds the 8 partials as
@@ -18,16 +18,13 @@ constexpr int MGC_MAXL = 8;
 // coarse V-cycle kernels all solve the coarsest level here, so they give the same bits.
 // dinv: row-major, row stride n, in global or shared memory.
 template <class T>
-__device__ void dense_coarse_apply(int n, const double* dinv, const T* b, T* x, int singular) {
+__device__ void dense_coarse_apply(int n, const double* dinv, const T* b, T* x) {
     const int t = threadIdx.x, g = t & 7, rows = blockDim.x >> 3;
     for (int base = 0; base < n; base += rows) {
         const int r = base + (t >> 3);
         double s = 0.0;
         if (r < n)
-            for (int c = g; c < n; c += 8) {
-                const double bc = (singular && c == 0) ? 0.0 : (double)b[c];
-                s += dinv[r * n + c] * bc;
-            }
+            for (int c = g; c < n; c += 8) s += dinv[r * n + c] * (double)b[c];
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         s += __shfl_xor_sync(0xffffffffu, s, 4);
@@ -38,75 +35,65 @@ __device__ void dense_coarse_apply(int n, const double* dinv, const T* b, T* x, 
 
 template <class T>
 struct CoarseArgs {
-    int nl, singular, dn;
-    int pre, post;  // smoother sweeps before / after the coarse correction
-    int zero_color;  // restriction skips cells of this colour (their residual is ~0), or -1
+    int nl, dn;
+    int npre, npost;  // smoother colours before / after the coarse correction
+    int post_first;   // five-point: colour of the first one after it
+    int zero_color;   // five-point: restriction skips cells of this colour (their residual is ~0), or -1
     int n1[MGC_MAXL], n2[MGC_MAXL];
     const T* tx[MGC_MAXL];
     const T* ty[MGC_MAXL];
     const T* a9[MGC_MAXL];
     const T* id[MGC_MAXL];
     const T* dg[MGC_MAXL];  // diagonals (FACE5; EXP9 uses plane 0 of a9)
+    const T* w4[MGC_MAXL];  // transfer weights (FACE5, levels below the first), null: plain transfers
     T* x0;           // iterate of the first handled level (global)
     const T* b0;     // its right-hand side (global)
     const double* dinv;
 };
 
+// One colour of a sweep: red-black (0, 1) or four-colour (0..3).
 template <class T, int KIND>
-__device__ void cv_smooth(int n1, int n2, const T* tx, const T* ty, const T* a9, const T* id, const T* b, T* x,
-                          bool reverse, int sweeps) {
+__device__ void cv_colour(int n1, int n2, const T* tx, const T* ty, const T* a9, const T* id, const T* b, T* x, int col) {
     const int n = n1 * n2;
-    for (int s = 0; s < sweeps; ++s) {
-        const int ncol = KIND == FACE5 ? 2 : 4;
-        for (int cc = 0; cc < ncol; ++cc) {
-            const int col = reverse ? ncol - 1 - cc : cc;
-            for (int k = threadIdx.x; k < n; k += blockDim.x) {
-                const int i = k / n2, j = k % n2;
-                if (KIND == FACE5) {
-                    if (((i + j) & 1) != col) continue;
-                    T sm = b[k];
-                    if (i > 0) sm += tx[IX(i, j, n2)] * x[k - n2];
-                    if (i < n1 - 1) sm += tx[IX(i + 1, j, n2)] * x[k + n2];
-                    if (j > 0) sm += ty[IX(i, j, n2 + 1)] * x[k - 1];
-                    if (j < n2 - 1) sm += ty[IX(i, j + 1, n2 + 1)] * x[k + 1];
-                    x[k] = sm * id[k];
-                } else {  // as k_gs4_exp9: s = b - sum_e a_e x_e, x = s * idiag
-                    if ((((i & 1) << 1) | (j & 1)) != col) continue;
-                    T o = 0;
-                    for (int e = 1; e < 9; ++e) {
-                        int ii = i + c_off[e][0], jj = j + c_off[e][1];
-                        if (ii < 0 || ii >= n1 || jj < 0 || jj >= n2) continue;
-                        o += a9[e * n + k] * x[IX(ii, jj, n2)];
-                    }
-                    x[k] = (b[k] - o) * id[k];
-                }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const int i = k / n2, j = k % n2;
+        if (KIND == FACE5) {
+            if (((i + j) & 1) != col) continue;
+            T sm = b[k];
+            if (i > 0) sm += tx[IX(i, j, n2)] * x[k - n2];
+            if (i < n1 - 1) sm += tx[IX(i + 1, j, n2)] * x[k + n2];
+            if (j > 0) sm += ty[IX(i, j, n2 + 1)] * x[k - 1];
+            if (j < n2 - 1) sm += ty[IX(i, j + 1, n2 + 1)] * x[k + 1];
+            x[k] = sm * id[k];
+        } else {  // as k_gs4_exp9: s = b - sum_e a_e x_e, x = s * idiag
+            if ((((i & 1) << 1) | (j & 1)) != col) continue;
+            T o = 0;
+            for (int e = 1; e < 9; ++e) {
+                int ii = i + c_off[e][0], jj = j + c_off[e][1];
+                if (ii < 0 || ii >= n1 || jj < 0 || jj >= n2) continue;
+                o += a9[e * n + k] * x[IX(ii, jj, n2)];
             }
-            __syncthreads();
+            x[k] = (b[k] - o) * id[k];
         }
     }
+    __syncthreads();
 }
 
-// Same arithmetic as resid() of the level kernels: s = b + sum t * x_nb (or b - sum a_e * x_nb),
-// r = s - diag * x.
-template <class T, int KIND>
-__device__ __forceinline__ T cv_resid(int i, int j, int n1, int n2, const T* tx, const T* ty, const T* a9, const T* dg,
-                                      const T* b, const T* x) {
-    const int k = IX(i, j, n2);
-    T s = b[k];
-    if (KIND == FACE5) {
-        if (i > 0) s += tx[k] * x[k - n2];
-        if (i < n1 - 1) s += tx[k + n2] * x[k + n2];
-        if (j > 0) s += ty[IX(i, j, n2 + 1)] * x[k - 1];
-        if (j < n2 - 1) s += ty[IX(i, j + 1, n2 + 1)] * x[k + 1];
-        return s - dg[k] * x[k];
-    }
-    const int n = n1 * n2;
-    for (int e = 1; e < 9; ++e) {
-        int ii = i + c_off[e][0], jj = j + c_off[e][1];
-        if (ii < 0 || ii >= n1 || jj < 0 || jj >= n2) continue;
-        s -= a9[e * n + k] * x[IX(ii, jj, n2)];
-    }
-    return s - a9[k] * x[k];
+// Residual sums of the children of coarse cell (I, J) on its east, west, north and south side
+// (as k_restrict5; the skipped colour counts as zero).
+template <class T>
+__device__ __forceinline__ void cv_sides(int I, int J, int n1, int n2, int zc, const T* tx, const T* ty, const T* dg,
+                                         const T* b, const T* x, T& e, T& w, T& n, T& s) {
+    auto child = [&](int di, int dj) -> T {
+        const int i = 2 * I + di, j = 2 * J + dj;
+        if (((di + dj) & 1) == zc || i >= n1 || j >= n2) return T(0);
+        return resid5<T>(n1, n2, i, j, tx, ty, dg, b, x);
+    };
+    const T r00 = child(0, 0), r01 = child(0, 1), r10 = child(1, 0), r11 = child(1, 1);
+    e = r10 + r11;
+    w = r00 + r01;
+    n = r01 + r11;
+    s = r00 + r10;
 }
 
 template <class T, int KIND>
@@ -114,15 +101,17 @@ __global__ void __launch_bounds__(1024) k_coarse_vcycle(CoarseArgs<T> A) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char cv_raw[];
     T* sm = reinterpret_cast<T*>(cv_raw);
-    T *tx[MGC_MAXL], *ty[MGC_MAXL], *a9[MGC_MAXL], *id[MGC_MAXL], *dg[MGC_MAXL], *x[MGC_MAXL], *b[MGC_MAXL];
+    T *tx[MGC_MAXL], *ty[MGC_MAXL], *a9[MGC_MAXL], *id[MGC_MAXL], *dg[MGC_MAXL], *x[MGC_MAXL], *b[MGC_MAXL],
+        *w4[MGC_MAXL];
     size_t off = 0;
     for (int l = 0; l < A.nl; ++l) {
         const int n1 = A.n1[l], n2 = A.n2[l], n = n1 * n2;
-        tx[l] = ty[l] = a9[l] = dg[l] = nullptr;
+        tx[l] = ty[l] = a9[l] = dg[l] = w4[l] = nullptr;
         if (KIND == FACE5) {
             tx[l] = sm + off; off += (size_t)(n1 + 1) * n2;
             ty[l] = sm + off; off += (size_t)n1 * (n2 + 1);
             dg[l] = sm + off; off += n;
+            if (l > 0 && A.w4[l]) { w4[l] = sm + off; off += (size_t)4 * n; }
         } else {
             a9[l] = sm + off; off += (size_t)9 * n;
         }
@@ -136,6 +125,8 @@ __global__ void __launch_bounds__(1024) k_coarse_vcycle(CoarseArgs<T> A) {
             for (int k = threadIdx.x; k < (n1 + 1) * n2; k += blockDim.x) stage_async(tx[l] + k, A.tx[l] + k);
             for (int k = threadIdx.x; k < n1 * (n2 + 1); k += blockDim.x) stage_async(ty[l] + k, A.ty[l] + k);
             for (int k = threadIdx.x; k < n; k += blockDim.x) stage_async(dg[l] + k, A.dg[l] + k);
+            if (w4[l])
+                for (int k = threadIdx.x; k < 4 * n; k += blockDim.x) stage_async(w4[l] + k, A.w4[l] + k);
         } else {
             for (int k = threadIdx.x; k < 9 * n; k += blockDim.x) stage_async(a9[l] + k, A.a9[l] + k);
         }
@@ -154,41 +145,49 @@ __global__ void __launch_bounds__(1024) k_coarse_vcycle(CoarseArgs<T> A) {
     __syncthreads();
     const int L = A.nl - 1;  // dense level
     for (int l = 0; l < L; ++l) {
-        const int n1 = A.n1[l], n2 = A.n2[l], c1 = A.n1[l + 1], c2 = A.n2[l + 1];
-        cv_smooth<T, KIND>(n1, n2, tx[l], ty[l], a9[l], id[l], b[l], x[l], false, A.pre);
-        for (int K = threadIdx.x; K < c1 * c2; K += blockDim.x) {
+        const int n1 = A.n1[l], n2 = A.n2[l], c1 = A.n1[l + 1], c2 = A.n2[l + 1], nc = c1 * c2;
+        for (int s = 0; s < A.npre; ++s)
+            cv_colour<T, KIND>(n1, n2, tx[l], ty[l], a9[l], id[l], b[l], x[l], KIND == FACE5 ? s & 1 : s & 3);
+        for (int K = threadIdx.x; K < nc; K += blockDim.x) {
             const int I = K / c2, J = K % c2;
             T s = 0;
-            for (int a = 0; a < 2; ++a)
-                for (int bb = 0; bb < 2; ++bb) {
-                    int i = 2 * I + a, j = 2 * J + bb;
-                    if (((i + j) & 1) == A.zero_color) continue;  // as k_restrict
-                    if (i < n1 && j < n2) s += cv_resid<T, KIND>(i, j, n1, n2, tx[l], ty[l], a9[l], dg[l], b[l], x[l]);
-                }
+            if (KIND == FACE5) {  // the neighbours' sides are computed again: few cells, one pass
+                auto sides = [&](int I, int J, T& e, T& w, T& n, T& so) {
+                    cv_sides<T>(I, J, n1, n2, A.zero_color, tx[l], ty[l], dg[l], b[l], x[l], e, w, n, so);
+                };
+                const T* w = w4[l + 1];
+                T e, we, n, so, d0, d1, d2, d3;
+                sides(I, J, e, we, n, so);
+                s = e + we;
+                if (w) s = restrict_sum<T>(e, we, n, so, w[K], w[nc + K], w[2 * nc + K], w[3 * nc + K]);
+                if (w && I > 0) { sides(I - 1, J, d0, d1, d2, d3); s = fma(w[K - c2], d0, s); }
+                if (w && I < c1 - 1) { sides(I + 1, J, d0, d1, d2, d3); s = fma(w[nc + K + c2], d1, s); }
+                if (w && J > 0) { sides(I, J - 1, d0, d1, d2, d3); s = fma(w[2 * nc + K - 1], d2, s); }
+                if (w && J < c2 - 1) { sides(I, J + 1, d0, d1, d2, d3); s = fma(w[3 * nc + K + 1], d3, s); }
+            } else {
+                for (int a = 0; a < 2; ++a)
+                    for (int bb = 0; bb < 2; ++bb) {
+                        const int i = 2 * I + a, j = 2 * J + bb;
+                        if (i < n1 && j < n2) s += resid9<T>(n1, n2, i, j, a9[l], b[l], x[l]);
+                    }
+            }
             b[l + 1][K] = s;
             x[l + 1][K] = 0;
         }
         __syncthreads();
     }
-    dense_coarse_apply<T>(A.dn, A.dinv, b[L], x[L], A.singular);  // coarsest level
+    dense_coarse_apply<T>(A.dn, A.dinv, b[L], x[L]);  // coarsest level
     for (int l = L - 1; l >= 0; --l) {
         const int n1 = A.n1[l], n2 = A.n2[l], c1 = A.n1[l + 1], c2 = A.n2[l + 1];
+        const T* xc = x[l + 1];
         for (int k = threadIdx.x; k < n1 * n2; k += blockDim.x) {
             const int i = k / n2, j = k % n2;
-            int I = i >> 1, J = j >> 1;
-            int I2 = (i & 1) ? I + 1 : I - 1, J2 = (j & 1) ? J + 1 : J - 1;
-            if (I2 < 0 || I2 >= c1) I2 = I;
-            if (J2 < 0 || J2 >= c2) J2 = J;
-            const T* xc = x[l + 1];
-            T v = x[l][k];
-            v += T(0.5625) * xc[IX(I, J, c2)];
-            v += T(0.1875) * xc[IX(I2, J, c2)];
-            v += T(0.1875) * xc[IX(I, J2, c2)];
-            v += T(0.0625) * xc[IX(I2, J2, c2)];
-            x[l][k] = v;
+            x[l][k] = prolong_cell<T>(i, j, n2, x[l], c1, c2, xc, w4[l + 1]);
         }
         __syncthreads();
-        cv_smooth<T, KIND>(n1, n2, tx[l], ty[l], a9[l], id[l], b[l], x[l], true, A.post);
+        for (int s = 0; s < A.npost; ++s)
+            cv_colour<T, KIND>(n1, n2, tx[l], ty[l], a9[l], id[l], b[l], x[l],
+                               KIND == FACE5 ? (A.post_first + s) & 1 : 3 - (s & 3));
     }
     const int n0 = A.n1[0] * A.n2[0];
     for (int k = threadIdx.x; k < n0; k += blockDim.x) A.x0[k] = x[0][k];

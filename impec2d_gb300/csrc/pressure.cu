@@ -197,45 +197,103 @@ __global__ void k_exp9_fine(int n1, int n2, const double* __restrict__ lamx, con
 __constant__ int c_off[9][2] = {{0, 0}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}, {1, 0}, {1, 1}, {0, 1}, {-1, 1}};
 
 // ---------------------------------------------------------------- coarse operators
-// Coarse five-point faces (half the sum of the two fine faces they cover).  With diag != null
-// (no extra diagonal from a Dirichlet row) the kernel also writes the coarse diagonal and its
-// reciprocal from recomputed faces, in place of the level's k_idiag launch (same values).
-__global__ void k_face5_coarsen(int n1f, int n2f, const double* __restrict__ txf, const double* __restrict__ tyf,
-                                int n1c, int n2c, double* __restrict__ txc, double* __restrict__ tyc,
-                                float* __restrict__ txc32, float* __restrict__ tyc32, double* __restrict__ diag,
-                                double* __restrict__ idiag, float* __restrict__ diag32, float* __restrict__ idiag32) {
+// Five-point coarsening, 2 x 2 cells to one.  A coarse face carries the flux that two coarse cell
+// centres drive through what lies between them: the two fine faces on the interface (conductance
+// s, in parallel) in series with half of each cell's inside, h = 1 / (2 t_in), t_in the sum of
+// the two fine faces inside the cell in that direction:
+//   t = s / (1 + s (h_lo + h_hi)).
+// On a uniform grid that is the rediscretised face (s = 2, h = 1/4, t = 1); across a jump of the
+// mobility it keeps the harmonic mean that the sum of the fine faces loses.  The same quantities
+// give the transfer weights w = h t <= 1 of a coarse cell towards its four neighbours (planes E, W,
+// N, S): a child's value is the coarse one plus w times the difference to the neighbour on its
+// side, the pressure that the flux t (x_nb - x) loses over the child's half of the cell
+// (prolong5), and the restriction is that interpolation's transpose (k_restrict5).  With symmetric
+// smoothing the cycle is then symmetric, as CG wants it.  CG iterations to 1e-10 with these
+// coarse operators and transfers against half the sum of the fine faces with bilinear
+// interpolation: 24 -> 14 on a 1024^2 front (M = 41), 52 -> 17 on a 4096^2 lognormal field.
+//
+// plain (the stationary iteration, which diverges where a correction overshoots, as these can on
+// cell-to-cell jumps): half the sum of the fine faces, no weights.
+//
+// A block owns 32 x 8 coarse cells: h of the cells and a one-cell ring in shared memory, then
+// each face of the tile once, then weights, diagonal and 1/diagonal from those faces.  FP64-bound
+// (five divisions per coarse cell).
+constexpr int CO_C = 32, CO_R = 8;
+__global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, const double* __restrict__ txf,
+                                                          const double* __restrict__ tyf, int n1c, int n2c,
+                                                          double* __restrict__ txc, double* __restrict__ tyc,
+                                                          float* __restrict__ txc32, float* __restrict__ tyc32,
+                                                          double* __restrict__ w4, float* __restrict__ w432,
+                                                          double* __restrict__ diag, double* __restrict__ idiag,
+                                                          float* __restrict__ diag32, float* __restrict__ idiag32,
+                                                          int plain) {
     pdl_enter();
-    int J = blockIdx.x * BX + threadIdx.x, I = blockIdx.y * BY + threadIdx.y;
-    auto cx = [&](int a, int b) {  // coarse x-face (a, b)
-        int fi = 2 * a;
-        double s = 0.0;
-        if (fi <= n1f) {
-            s = txf[IX(fi, 2 * b, n2f)];
-            if (2 * b + 1 < n2f) s += txf[IX(fi, 2 * b + 1, n2f)];
-        }
-        return 0.5 * s;
+    __shared__ double hx[CO_R + 2][CO_C], hy[CO_R][CO_C + 2];      // cells (I0 - 1 + r, J0 + q), (I0 + r, J0 - 1 + q)
+    __shared__ double cx[CO_R + 1][CO_C], cy[CO_R][CO_C + 1];      // faces (I0 + r, J0 + q)
+    const int t = threadIdx.y * CO_C + threadIdx.x, I0 = blockIdx.y * CO_R, J0 = blockIdx.x * CO_C;
+    // fine faces in pairs (the second of a pair may lie outside an odd grid)
+    auto pair_x = [&](int fi, int J) {  // x-faces fi of the two columns of coarse column J
+        double v = txf[IX(fi, 2 * J, n2f)];
+        if (2 * J + 1 < n2f) v += txf[IX(fi, 2 * J + 1, n2f)];
+        return v;
     };
-    auto cy = [&](int a, int b) {  // coarse y-face (a, b)
-        int fj = 2 * b;
-        double s = 0.0;
-        if (fj <= n2f) {
-            s = tyf[IX(2 * a, fj, n2f + 1)];
-            if (2 * a + 1 < n1f) s += tyf[IX(2 * a + 1, fj, n2f + 1)];
-        }
-        return 0.5 * s;
+    auto pair_y = [&](int I, int fj) {
+        double v = tyf[IX(2 * I, fj, n2f + 1)];
+        if (2 * I + 1 < n1f) v += tyf[IX(2 * I + 1, fj, n2f + 1)];
+        return v;
     };
-    if (I <= n1c && J < n2c) {
-        const double t = cx(I, J);
-        txc[IX(I, J, n2c)] = t;
-        if (txc32) txc32[IX(I, J, n2c)] = (float)t;
+    auto half = [&](double in) { return in > 0.0 && !plain ? fmin(0.5 / in, 1e300) : 0.0; };
+    for (int k = t; k < (CO_R + 2) * CO_C; k += CO_C * CO_R) {
+        const int r = k / CO_C, q = k % CO_C, I = I0 - 1 + r, J = J0 + q;
+        hx[r][q] = I >= 0 && J < n2c && 2 * I + 1 < n1f ? half(pair_x(2 * I + 1, J)) : 0.0;
     }
-    if (I < n1c && J <= n2c) {
-        const double t = cy(I, J);
-        tyc[IX(I, J, n2c + 1)] = t;
-        if (tyc32) tyc32[IX(I, J, n2c + 1)] = (float)t;
+    for (int k = t; k < CO_R * (CO_C + 2); k += CO_C * CO_R) {
+        const int r = k / (CO_C + 2), q = k % (CO_C + 2), I = I0 + r, J = J0 - 1 + q;
+        hy[r][q] = J >= 0 && I < n1c && 2 * J + 1 < n2f ? half(pair_y(I, 2 * J + 1)) : 0.0;
     }
-    if (diag && I < n1c && J < n2c)
-        store_diag5(IX(I, J, n2c), cx(I, J), cx(I + 1, J), cy(I, J), cy(I, J + 1), diag, idiag, diag32, idiag32);
+    __syncthreads();
+    for (int k = t; k < (CO_R + 1) * CO_C; k += CO_C * CO_R) {
+        const int r = k / CO_C, q = k % CO_C, I = I0 + r, J = J0 + q;
+        double v = 0.0;
+        if (I <= n1c && J < n2c) {
+            if (I > 0 && I < n1c) {
+                const double a = pair_x(2 * I, J);
+                v = plain ? 0.5 * a : a / (1.0 + a * (hx[r][q] + hx[r + 1][q]));
+            }
+            if (r < CO_R || I == n1c) {  // the face below the tile belongs to the next tile, except the last one
+                txc[IX(I, J, n2c)] = v;
+                if (txc32) txc32[IX(I, J, n2c)] = (float)v;
+            }
+        }
+        cx[r][q] = v;
+    }
+    for (int k = t; k < CO_R * (CO_C + 1); k += CO_C * CO_R) {
+        const int r = k / (CO_C + 1), q = k % (CO_C + 1), I = I0 + r, J = J0 + q;
+        double v = 0.0;
+        if (I < n1c && J <= n2c) {
+            if (J > 0 && J < n2c) {
+                const double a = pair_y(I, 2 * J);
+                v = plain ? 0.5 * a : a / (1.0 + a * (hy[r][q] + hy[r][q + 1]));
+            }
+            if (q < CO_C || J == n2c) {
+                tyc[IX(I, J, n2c + 1)] = v;
+                if (tyc32) tyc32[IX(I, J, n2c + 1)] = (float)v;
+            }
+        }
+        cy[r][q] = v;
+    }
+    __syncthreads();
+    const int r = threadIdx.y, q = threadIdx.x, I = I0 + r, J = J0 + q;
+    if (I >= n1c || J >= n2c) return;
+    const size_t n = (size_t)n1c * n2c, k = IX(I, J, n2c);
+    const double w[4] = {hx[r + 1][q] * cx[r + 1][q], hx[r + 1][q] * cx[r][q], hy[r][q + 1] * cy[r][q + 1],
+                         hy[r][q + 1] * cy[r][q]};
+#pragma unroll
+    for (int e = 0; e < 4 && w4; ++e) {
+        w4[e * n + k] = w[e];
+        if (w432) w432[e * n + k] = (float)w[e];
+    }
+    if (diag) store_diag5(k, cx[r][q], cx[r + 1][q], cy[r][q], cy[r][q + 1], diag, idiag, diag32, idiag32);
 }
 
 __global__ void k_exp9_coarsen(int n1f, int n2f, const double* __restrict__ af, const unsigned char* __restrict__ maskf,
@@ -567,62 +625,146 @@ __global__ void k_gs4_exp9(int n1, int n2, const T* __restrict__ a9, const T* __
 }
 
 // ---------------------------------------------------------------- transfers
-// r = b - A x at (i, j) as one accumulation: s = b + sum t * x_nb (FACE5) or
-// b - sum a_e * x_nb (EXP9), then r = s - diag * x.
+// r = b - A x at (i, j) as one accumulation: s = b + sum t * x_nb (five-point) or
+// b - sum a_e * x_nb (nine-point), then r = s - diag * x.
 template <class T>
-__device__ __forceinline__ T resid(const Level& Lv, int i, int j, const T* __restrict__ tx, const T* __restrict__ ty,
-                                   const T* __restrict__ a9, const T* __restrict__ dg, const T* __restrict__ b,
-                                   const T* __restrict__ x) {
-    const int n1 = Lv.n1, n2 = Lv.n2;
+__device__ __forceinline__ T resid5(int n1, int n2, int i, int j, const T* __restrict__ tx, const T* __restrict__ ty,
+                                    const T* __restrict__ dg, const T* __restrict__ b, const T* __restrict__ x) {
     const size_t k = IX(i, j, n2);
     T s = b[k];
-    if (Lv.kind == FACE5) {
-        if (i > 0) s += tx[k] * x[k - n2];
-        if (i < n1 - 1) s += tx[k + n2] * x[k + n2];
-        if (j > 0) s += ty[IX(i, j, n2 + 1)] * x[k - 1];
-        if (j < n2 - 1) s += ty[IX(i, j + 1, n2 + 1)] * x[k + 1];
-    } else {
-        const size_t n = (size_t)n1 * n2;
-#pragma unroll
-        for (int e = 1; e < 9; ++e) {
-            const int ii = i + c_off[e][0], jj = j + c_off[e][1];
-            if (ii < 0 || ii >= n1 || jj < 0 || jj >= n2) continue;
-            s -= a9[e * n + k] * x[IX(ii, jj, n2)];
-        }
-    }
+    if (i > 0) s += tx[k] * x[k - n2];
+    if (i < n1 - 1) s += tx[k + n2] * x[k + n2];
+    if (j > 0) s += ty[IX(i, j, n2 + 1)] * x[k - 1];
+    if (j < n2 - 1) s += ty[IX(i, j + 1, n2 + 1)] * x[k + 1];
     return s - dg[k] * x[k];
 }
 
-// Residual of the fine level summed over each 2x2 aggregate -> coarse rhs; coarse x := 0.
 template <class T>
-__global__ void k_restrict(Level F, const T* __restrict__ tx, const T* __restrict__ ty, const T* __restrict__ a9,
-                           const T* __restrict__ dg, const T* __restrict__ b, const T* __restrict__ x, int n1c,
-                           int n2c, T* __restrict__ bc, T* __restrict__ xc, int zero_color, const T* __restrict__ idc) {
+__device__ __forceinline__ T resid9(int n1, int n2, int i, int j, const T* __restrict__ a9, const T* __restrict__ b,
+                                    const T* __restrict__ x) {
+    const size_t n = (size_t)n1 * n2, k = IX(i, j, n2);
+    T s = b[k];
+#pragma unroll
+    for (int e = 1; e < 9; ++e) {
+        const int ii = i + c_off[e][0], jj = j + c_off[e][1];
+        if (ii < 0 || ii >= n1 || jj < 0 || jj >= n2) continue;
+        s -= a9[e * n + k] * x[IX(ii, jj, n2)];
+    }
+    return s - a9[k] * x[k];
+}
+
+// Residual of the system's own operator on the finest level (nine-point when a9 is there, even if
+// a five-point hierarchy preconditions it).
+__device__ __forceinline__ double resid_op(const Level& F, int i, int j, const double* __restrict__ b,
+                                           const double* __restrict__ x) {
+    return F.a9 ? resid9<double>(F.n1, F.n2, i, j, F.a9, b, x)
+                : resid5<double>(F.n1, F.n2, i, j, F.tx, F.ty, F.diag, b, x);
+}
+
+// Nine-point levels: residual summed over each 2x2 aggregate -> coarse rhs; coarse x := 0.
+template <class T>
+__global__ void k_restrict9(int n1, int n2, const T* __restrict__ a9, const T* __restrict__ b, const T* __restrict__ x,
+                            int n1c, int n2c, T* __restrict__ bc, T* __restrict__ xc) {
     pdl_enter();
     int J = blockIdx.x * BX + threadIdx.x, I = blockIdx.y * BY + threadIdx.y;
     if (I >= n1c || J >= n2c) return;
     T s = 0;
     for (int a = 0; a < 2; ++a)
         for (int bb = 0; bb < 2; ++bb) {
-            int i = 2 * I + a, j = 2 * J + bb;
-            // zero_color >= 0: the red-black sweep just updated that colour, whose residual
-            // s - diag (s / diag) is zero up to one rounding (resid() recomputes the same s)
-            if (((i + j) & 1) == zero_color) continue;
-            if (i < F.n1 && j < F.n2) s += resid<T>(F, i, j, tx, ty, a9, dg, b, x);
+            const int i = 2 * I + a, j = 2 * J + bb;
+            if (i < n1 && j < n2) s += resid9<T>(n1, n2, i, j, a9, b, x);
         }
     bc[IX(I, J, n2c)] = s;
-    // The coarse cycle starts from x = 0.  Without idc that zero is written.  With idc (the
-    // coarse 1/diag), the coarse pre-smoothing's first colour (red, as k_rb_zero:
-    // x = b * idiag) is done here, and the black cells are left for its black pass to overwrite.
-    if (!idc) xc[IX(I, J, n2c)] = 0;
-    else if (((I + J) & 1) == 0) xc[IX(I, J, n2c)] = s * idc[IX(I, J, n2c)];
+    xc[IX(I, J, n2c)] = 0;
 }
 
-// Bilinear cell-centred prolongation (weights 9/16, 3/16, 3/16, 1/16; the outside
-// neighbour is replaced by the cell itself), added to the fine iterate.
+// Coarse right-hand side of a five-point cell from the residual sums of its children on the east,
+// west, north and south side (e, w, n, s) and those its neighbours' weights send here: the
+// transpose of prolong5.  Every V-cycle implementation sums in this order.
 template <class T>
-__device__ __forceinline__ T prolong_cell(int i, int j, int n2, const T* __restrict__ x, int n1c, int n2c,
-                                          const T* __restrict__ xc) {
+__device__ __forceinline__ T restrict_sum(T e, T w, T n, T s, T wE, T wW, T wN, T wS) {
+    T v = e + w;
+    v = fma(-wE, e, v);
+    v = fma(-wW, w, v);
+    v = fma(-wN, n, v);
+    return fma(-wS, s, v);
+}
+
+// Five-point restriction.  The sweep before it has just updated one colour, whose residual
+// s - diag (s / diag) is zero up to one rounding: ZC is that colour (its cells are skipped), or -1
+// (all four children count).  A block owns RS_C x RS_R coarse cells; the children's residuals of
+// the tile and of the ring of coarse cells around it (80 of 592 residuals for one colour) go to
+// shared memory, where the neighbours' weights pick them up.  FP64-bound: 12 operations for two
+// residuals, 9 for the weights.
+// w4 = null (plain transfers): the children's sum alone.
+// The coarse cycle starts from x = 0.  Without idc that zero is written.  With idc (the coarse
+// 1/diag), the coarse pre-smoothing's first colour (red, as k_rb_zero: x = b * idiag) is done
+// here, and the black cells are left for its black pass to overwrite.
+constexpr int RS_C = 32, RS_R = 8;
+template <class T, int ZC>
+__global__ void __launch_bounds__(RS_C * RS_R) k_restrict5(int n1, int n2, const T* __restrict__ tx,
+                                                           const T* __restrict__ ty, const T* __restrict__ dg,
+                                                           const T* __restrict__ b, const T* __restrict__ x, int n1c,
+                                                           int n2c, const T* __restrict__ w4, T* __restrict__ bc,
+                                                           T* __restrict__ xc, const T* __restrict__ idc) {
+    pdl_enter();
+    __shared__ T se[RS_R + 1][RS_C], sw[RS_R + 1][RS_C];  // rows I0 - 1 + r, I0 + r
+    __shared__ T sn[RS_R][RS_C + 1], ss[RS_R][RS_C + 1];  // columns J0 - 1 + q, J0 + q
+    const int r = threadIdx.y, q = threadIdx.x, I0 = blockIdx.y * RS_R, J0 = blockIdx.x * RS_C;
+    const int I = I0 + r, J = J0 + q;
+    auto child = [&](int a, int c, int di, int dj) -> T {  // residual of child (di, dj) of coarse cell (a, c)
+        if (((di + dj) & 1) == ZC) return T(0);
+        const int i = 2 * a + di, j = 2 * c + dj;
+        return i < n1 && j < n2 ? resid5<T>(n1, n2, i, j, tx, ty, dg, b, x) : T(0);
+    };
+    T e = 0, w = 0, n = 0, s = 0;
+    if (I < n1c && J < n2c) {
+        const T r00 = child(I, J, 0, 0), r01 = child(I, J, 0, 1), r10 = child(I, J, 1, 0), r11 = child(I, J, 1, 1);
+        if (ZC == 1) { e = n = r11; w = s = r00; }
+        else if (ZC == 0) { e = s = r10; w = n = r01; }
+        else { e = r10 + r11; w = r00 + r01; n = r01 + r11; s = r00 + r10; }
+    }
+    se[r + 1][q] = e;
+    sw[r][q] = w;
+    sn[r][q + 1] = n;
+    ss[r][q] = s;
+    // the ring: the east side of the row below, the west side of the row above, and so on
+    const int t = r * RS_C + q;
+    if (t < RS_C) {
+        const int c = J0 + t;
+        se[0][t] = I0 > 0 && c < n2c ? child(I0 - 1, c, 1, 0) + child(I0 - 1, c, 1, 1) : T(0);
+    } else if (t < 2 * RS_C) {
+        const int c = J0 + t - RS_C;
+        sw[RS_R][t - RS_C] = I0 + RS_R < n1c && c < n2c ? child(I0 + RS_R, c, 0, 0) + child(I0 + RS_R, c, 0, 1) : T(0);
+    } else if (t < 2 * RS_C + RS_R) {
+        const int a = I0 + t - 2 * RS_C;
+        sn[t - 2 * RS_C][0] = J0 > 0 && a < n1c ? child(a, J0 - 1, 0, 1) + child(a, J0 - 1, 1, 1) : T(0);
+    } else if (t < 2 * RS_C + 2 * RS_R) {
+        const int a = I0 + t - 2 * RS_C - RS_R;
+        ss[t - 2 * RS_C - RS_R][RS_C] =
+            J0 + RS_C < n2c && a < n1c ? child(a, J0 + RS_C, 0, 0) + child(a, J0 + RS_C, 1, 0) : T(0);
+    }
+    __syncthreads();
+    if (I >= n1c || J >= n2c) return;
+    const size_t nc = (size_t)n1c * n2c, k = IX(I, J, n2c);
+    T v = e + w;
+    if (w4) {
+        v = restrict_sum<T>(e, w, n, s, w4[k], w4[nc + k], w4[2 * nc + k], w4[3 * nc + k]);
+        if (I > 0) v = fma(w4[k - n2c], se[r][q], v);
+        if (I < n1c - 1) v = fma(w4[nc + k + n2c], sw[r + 1][q], v);
+        if (J > 0) v = fma(w4[2 * nc + k - 1], sn[r][q], v);
+        if (J < n2c - 1) v = fma(w4[3 * nc + k + 1], ss[r][q + 1], v);
+    }
+    bc[k] = v;
+    if (!idc) xc[k] = 0;
+    else if (((I + J) & 1) == 0) xc[k] = v * idc[k];
+}
+
+// Bilinear cell-centred prolongation (weights 9/16, 3/16, 3/16, 1/16; the outside neighbour is
+// replaced by the cell itself) of the nine-point levels and of plain transfers.
+template <class T>
+__device__ __forceinline__ T prolong_bilinear(int i, int j, int n2, const T* __restrict__ x, int n1c, int n2c,
+                                              const T* __restrict__ xc) {
     int I = i >> 1, J = j >> 1;
     int I2 = (i & 1) ? I + 1 : I - 1, J2 = (j & 1) ? J + 1 : J - 1;
     if (I2 < 0 || I2 >= n1c) I2 = I;
@@ -635,14 +777,33 @@ __device__ __forceinline__ T prolong_cell(int i, int j, int n2, const T* __restr
     return v;
 }
 
+// Five-point prolongation of one cell: x + xc + wx (xc_nb,x - xc) + wy (xc_nb,y - xc), the
+// neighbours being those on the cell's side of its aggregate (outside the grid w = 0).
+template <class T>
+__device__ __forceinline__ T prolong5(T x, T c, T cx, T cy, T wx, T wy) {
+    T v = fma(wx, cx - c, c);
+    v = fma(wy, cy - c, v);
+    return x + v;
+}
+template <class T>
+__device__ __forceinline__ T prolong_cell(int i, int j, int n2, const T* __restrict__ x, int n1c, int n2c,
+                                          const T* __restrict__ xc, const T* __restrict__ w4) {
+    if (!w4) return prolong_bilinear(i, j, n2, x, n1c, n2c, xc);
+    const int I = i >> 1, J = j >> 1;
+    const size_t nc = (size_t)n1c * n2c, k = IX(I, J, n2c);
+    const int I2 = (i & 1) ? min(I + 1, n1c - 1) : max(I - 1, 0), J2 = (j & 1) ? min(J + 1, n2c - 1) : max(J - 1, 0);
+    return prolong5<T>(x[IX(i, j, n2)], xc[k], xc[IX(I2, J, n2c)], xc[IX(I, J2, n2c)], w4[((i & 1) ? 0 : nc) + k],
+                       w4[((j & 1) ? 2 * nc : 3 * nc) + k]);
+}
+
 template <class T>
 __global__ void k_prolong(int n1, int n2, T* __restrict__ x, int n1c, int n2c, const T* __restrict__ xc,
-                          const unsigned char* __restrict__ mask) {
+                          const T* __restrict__ w4, const unsigned char* __restrict__ mask) {
     pdl_enter();
     int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
     if (i >= n1 || j >= n2) return;
     if (mask && mask[IX(i, j, n2)]) return;  // known cells take no correction
-    x[IX(i, j, n2)] = prolong_cell(i, j, n2, x, n1c, n2c, xc);
+    x[IX(i, j, n2)] = prolong_cell(i, j, n2, x, n1c, n2c, xc, w4);
 }
 
 // The same correction on the cells of one colour only (threads mapped as k_rb_face5).  When a
@@ -650,7 +811,7 @@ __global__ void k_prolong(int n1, int n2, T* __restrict__ x, int n1c, int n2c, c
 // colour's cells without reading them, so their correction would be dead work.
 template <class T>
 __global__ void k_prolong_rb(int n1, int n2, T* __restrict__ x, int n1c, int n2c, const T* __restrict__ xc,
-                             const unsigned char* __restrict__ mask, int color) {
+                             const T* __restrict__ w4, const unsigned char* __restrict__ mask, int color) {
     pdl_enter();
     const int jj = blockIdx.x * BX + threadIdx.x, i0 = blockIdx.y * (RB_ROWS * BY) + threadIdx.y;
 #pragma unroll
@@ -658,7 +819,7 @@ __global__ void k_prolong_rb(int n1, int n2, T* __restrict__ x, int n1c, int n2c
         const int i = i0 + r * BY, j = 2 * jj + ((i + color) & 1);
         if (i >= n1 || j >= n2) continue;
         if (mask && mask[IX(i, j, n2)]) continue;
-        x[IX(i, j, n2)] = prolong_cell(i, j, n2, x, n1c, n2c, xc);
+        x[IX(i, j, n2)] = prolong_cell(i, j, n2, x, n1c, n2c, xc, w4);
     }
 }
 
@@ -693,9 +854,11 @@ __global__ void k_dense_build(Level C, const double* __restrict__ tx, const doub
 }
 
 // Gauss-Jordan inversion of an n x n (n <= 64) diagonally dominant matrix in shared memory.
-// singular: D is the pinned singular system (row 0 = e_0), whose coarse solution has its mean
-// removed; the mean removal is linear, so it is folded into the stored matrix, which becomes
-// (I - 1 1^T / n) D^-1: every column less its mean.
+// singular: D is the pinned singular system (row 0 = e_0).  Its inverse is made the singular
+// operator's pseudo-inverse, P D^-1 P with P = I - 1 1^T / n (b(0) does not count: column 0 is
+// zeroed first): the solution has no mean, and a right-hand side whose sum is not quite zero loses
+// that excess evenly.  Left in, cell 0 would take it as a point source: the rounded rows of a
+// nine-point operator do not sum to zero, and CG then stopped at 1.8e-10 of ||f|| (1024^2, nu = 2/3).
 __global__ void k_dense_invert(int n, const double* __restrict__ D, double* __restrict__ Dinv, int singular) {
     pdl_enter();
     extern __shared__ double sm[];
@@ -731,7 +894,14 @@ __global__ void k_dense_invert(int n, const double* __restrict__ D, double* __re
             double m = 0;
             for (int r = 0; r < n; ++r) m += B[r * n + cc];
             m /= n;
-            for (int r = 0; r < n; ++r) B[r * n + cc] -= m;
+            for (int r = 0; r < n; ++r) B[r * n + cc] = cc == 0 ? 0.0 : B[r * n + cc] - m;
+        }
+        __syncthreads();
+        for (int r = threadIdx.x; r < n; r += blockDim.x) {
+            double m = 0;
+            for (int cc = 0; cc < n; ++cc) m += B[r * n + cc];
+            m /= n;
+            for (int cc = 0; cc < n; ++cc) B[r * n + cc] -= m;
         }
         __syncthreads();
     }
@@ -749,7 +919,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_fine_resid(Level F, const doubl
     pdl_enter();
     double acc[1] = {0.0};
     for_cells(F.n1, F.n2, [&](int i, int j, size_t k) {
-        double r = resid<double>(F, i, j, F.tx, F.ty, F.a9, F.diag, f, x);
+        double r = resid_op(F, i, j, f, x);
         if (r64) r64[k] = r;
         if (r32) r32[k] = (float)r;  // consistent rhs of the singular correction equation
         if ((int)k == pin) r = 0.0;  // the pinned row of the reference system has zero residual
@@ -809,7 +979,7 @@ __global__ void k_apply_ref(Level F, const double* __restrict__ x, int pin, int 
     size_t k = IX(i, j, F.n2);
     if ((int)k == pin || i == dir_row) { y[k] = kappa / dA * x[k]; return; }
     double v;
-    if (F.kind == FACE5) {
+    if (!F.a9) {
         double d, o;
         v = apply_face5<double>(i, j, F.n1, F.n2, F.tx, F.ty, x, d, o);
     } else {
@@ -826,7 +996,7 @@ constexpr size_t MG_CLUSTER_SMEM = 200 * 1024;
 
 // CTAs per cluster for k_cluster_vcycle: 16 where the device can co-schedule such a cluster
 // with the kernel's shared memory, else 8, else 0 (the per-level path is used).
-template <class T>
+template <class T, int KIND>
 static int cluster_size_for(int want) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(want);
@@ -840,7 +1010,7 @@ static int cluster_size_for(int want) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, k_cluster_vcycle<T>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&num, k_cluster_vcycle<T, KIND>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -853,6 +1023,16 @@ impec_status pressure_alloc(impec_ctx* ctx) {
     const impec_params& P = ctx->P;
     int n1 = P.N1, n2 = P.N2;
     const bool nine = P.nu < 1.0;
+    ctx->krylov = (int)env_long("IMPEC_MG_KRYLOV", 1) != 0;
+    // A nine-point system (nu < 1) is preconditioned with the hierarchy of its five-point part
+    // (nu = 1) where that is close to it: nu A5 <= A <= A5 for constant coefficients, whatever the
+    // cells' aspect ratio and the permeability's anisotropy, so CG pays for a condition number of
+    // at most 1 / nu and each cycle works on 2 coefficient planes instead of 9.  At nu = 1/2 and
+    // above that wins: 513 x 777, nu = 2/3, M = 41: 47 iterations of nine-point cycles against 15;
+    // towards nu = 0 the rotated stencil does not see a checkerboard and the bound is lost.  The
+    // stationary iteration smooths the system itself, and a Dirichlet row is eliminated from one
+    // operator only: both keep the nine-point levels.
+    const bool levels9 = nine && !(P.nu >= 0.5 && ctx->krylov && ctx->dir_row < 0);
     const size_t nc = (size_t)(n1 + 1) * (n2 + 1);
     if (nine) {
         IMPEC_CUDA_TRY(cudaMalloc((void**)&ctx->cm11, nc * 8));
@@ -864,13 +1044,19 @@ impec_status pressure_alloc(impec_ctx* ctx) {
         Level Lv;
         Lv.n1 = n1;
         Lv.n2 = n2;
-        Lv.kind = nine ? EXP9 : FACE5;
+        Lv.kind = levels9 ? EXP9 : FACE5;
         const size_t n = Lv.n();
         if (Lv.kind == FACE5) {
             IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.tx, (size_t)(n1 + 1) * n2 * 8));
             IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.ty, (size_t)n1 * (n2 + 1) * 8));
             IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.tx32, (size_t)(n1 + 1) * n2 * 4));
             IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.ty32, (size_t)n1 * (n2 + 1) * 4));
+            if (l > 0 && ctx->krylov) {
+                IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.w4, n * 4 * 8));
+                IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.w432, n * 4 * 4));
+            } else if (nine) {
+                IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.a9, n * 9 * 8));
+            }
         } else {
             IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.a9, n * 9 * 8));
             IMPEC_CUDA_TRY(cudaMalloc((void**)&Lv.a932, n * 9 * 4));
@@ -901,7 +1087,6 @@ impec_status pressure_alloc(impec_ctx* ctx) {
         IMPEC_CUDA_TRY(cudaMalloc((void**)&ctx->cg_p, nf * 8));
         IMPEC_CUDA_TRY(cudaMalloc((void**)&ctx->cg_q, nf * 8));
         IMPEC_CUDA_TRY(cudaMemset(ctx->cg_q, 0, nf * 8));
-        ctx->krylov = (int)env_long("IMPEC_MG_KRYLOV", 1) != 0;
         Tuning& T = ctx->tune;
         if (ctx->L[0].kind != FACE5) {
             // weighted nine-point operators (nu < 1): V(1,1) preconditions CG best (1024^2 step:
@@ -934,15 +1119,19 @@ impec_status pressure_alloc(impec_ctx* ctx) {
     IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_coarse_vcycle<float, FACE5>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
     IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_coarse_vcycle<float, EXP9>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
     const int cls = (int)MG_CLUSTER_SMEM;
-    IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_cluster_vcycle<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, cls));
-    IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_cluster_vcycle<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, cls));
     ctx->cl_size = 0;
-    if (cudaFuncSetAttribute(k_cluster_vcycle<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(k_cluster_vcycle<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-        const int want = (int)env_long("IMPEC_MG_CL_CTAS", CL_MAX_CTAS);
+    const int want = (int)env_long("IMPEC_MG_CL_CTAS", CL_MAX_CTAS);
+    const bool f5 = ctx->L[0].kind == FACE5;
+    auto allow = [&](auto* k) -> bool {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cls) == cudaSuccess &&
+               cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    };
+    if (f5 ? allow(k_cluster_vcycle<double, FACE5>) && allow(k_cluster_vcycle<float, FACE5>)
+           : allow(k_cluster_vcycle<double, EXP9>))
         for (int cs = want < CL_MAX_CTAS ? want : CL_MAX_CTAS; cs >= 2 && !ctx->cl_size; cs /= 2)
-            if (cluster_size_for<double>(cs) && cluster_size_for<float>(cs)) ctx->cl_size = cs;
-    }
+            if (f5 ? cluster_size_for<double, FACE5>(cs) && cluster_size_for<float, FACE5>(cs)
+                   : cluster_size_for<double, EXP9>(cs))
+                ctx->cl_size = cs;
     cudaGetLastError();
     return IMPEC_OK;
 }
@@ -950,7 +1139,7 @@ impec_status pressure_alloc(impec_ctx* ctx) {
 void pressure_free(impec_ctx* ctx) {
     for (Level& Lv : ctx->L) {
         void* ps[] = {Lv.tx,   Lv.ty,   Lv.a9,   Lv.idiag,   Lv.diag,   Lv.ed,  Lv.x,   Lv.b,
-                      Lv.tx32, Lv.ty32, Lv.a932, Lv.idiag32, Lv.diag32, Lv.x32, Lv.b32, Lv.xa, Lv.xa32};
+                      Lv.tx32, Lv.ty32, Lv.a932, Lv.idiag32, Lv.diag32, Lv.x32, Lv.b32, Lv.xa, Lv.xa32, Lv.w4, Lv.w432};
         for (void* p : ps)
             if (p) cudaFree(p);
     }
@@ -997,10 +1186,10 @@ impec_status pressure_setup(impec_ctx* ctx, const double* c) {
                                  sx, sy, F.tx, F.ty, f32 && !dir ? F.tx32 : nullptr, f32 && !dir ? F.ty32 : nullptr,
                                  dir ? nullptr : F.diag, dir ? nullptr : F.idiag,
                                  mixed && !dir ? F.diag32 : nullptr, mixed && !dir ? F.idiag32 : nullptr);
-    } else {
+    }
+    if (F.a9)
         ++ctx->nlaunch, launch_k(ctx->stream, k_exp9_fine, grid2(F.n1, F.n2), dim3(BX, BY), 0, F.n1, F.n2, ctx->lamx, ctx->lamy, ctx->cm11,
                                                                          ctx->cm22, ctx->cm12, P.nu, G, F.a9);
-    }
     IMPEC_LAUNCH_CHECK();
     const unsigned char* mask0 = dir ? ctx->dmask : nullptr;
     if (dir) {
@@ -1020,10 +1209,12 @@ impec_status pressure_setup(impec_ctx* ctx, const double* c) {
     for (size_t l = 0; l + 1 < ctx->L.size(); ++l) {
         Level &A = ctx->L[l], &B = ctx->L[l + 1];
         if (A.kind == FACE5) {
-            ++ctx->nlaunch, launch_k(ctx->stream, k_face5_coarsen, grid2(B.n1 + 1, B.n2 + 1), dim3(BX, BY), 0, A.n1, A.n2, A.tx, A.ty, B.n1,
-                                     B.n2, B.tx, B.ty, f32 ? B.tx32 : nullptr, f32 ? B.ty32 : nullptr,
+            ++ctx->nlaunch, launch_k(ctx->stream, k_coarsen5, dim3((B.n2 + CO_C - 1) / CO_C, (B.n1 + CO_R - 1) / CO_R),
+                                     dim3(CO_C, CO_R), 0, A.n1, A.n2, A.tx, A.ty, B.n1, B.n2, B.tx, B.ty,
+                                     f32 ? B.tx32 : nullptr, f32 ? B.ty32 : nullptr, B.w4, f32 ? B.w432 : nullptr,
                                      dir ? nullptr : B.diag, dir ? nullptr : B.idiag,
-                                     mixed && !dir ? B.diag32 : nullptr, mixed && !dir ? B.idiag32 : nullptr);
+                                     mixed && !dir ? B.diag32 : nullptr, mixed && !dir ? B.idiag32 : nullptr,
+                                     ctx->krylov ? 0 : 1);
             if (dir)
                 ++ctx->nlaunch, launch_k(ctx->stream, k_ed_coarsen, grid2(B.n1, B.n2), dim3(BX, BY), 0, A.n1, A.n2, A.ed,
                                          B.n1, B.n2, B.ed);
@@ -1087,6 +1278,13 @@ template <>
 const float* level_diag<float>(const Level& Lv) { return Lv.diag32; }
 
 template <class T>
+static const T* level_w4(const Level& Lv);
+template <>
+const double* level_w4<double>(const Level& Lv) { return Lv.w4; }
+template <>
+const float* level_w4<float>(const Level& Lv) { return Lv.w432; }
+
+template <class T>
 static T* level_alt(Level& Lv);
 template <>
 double* level_alt<double>(Level& Lv) { return Lv.xa; }
@@ -1121,22 +1319,39 @@ static dim3 rb_grid(const Level& Lv) {
     return dim3((Lv.n2 / 2 + 1 + BX - 1) / BX, (Lv.n1 + RB_ROWS * BY - 1) / (RB_ROWS * BY));
 }
 
-// zero: x holds no values yet and stands for x = 0 (five-point levels only, where the first
-// colour's update then needs no neighbour).  first_done: that first colour was already done
-// by the restriction that produced b (k_restrict with the coarse 1/diag).
+// The smoother's colours of a five-point V(pre, post) cycle, two to a sweep: npre of them before the
+// coarse correction (red, black, red, ...), npost after it, starting with the colour that came last
+// before.  With post = pre + 1 the odd sweep is split, one colour on either side: the colours
+// after the correction are then those before it in reverse, and with the transposed transfers the
+// cycle is symmetric for the same work (V(1,2): red black red | red black red).  CG iterations of
+// the 512^2 M = 100 field, V(1,2): 19 so split, 24 as two and four colours.
+struct Colours {
+    int npre, npost, post_first;
+};
+static Colours colours(const impec_ctx* ctx) {
+    const int pre = (int)ctx->tune.pre, post = (int)ctx->tune.post;
+    Colours c{2 * pre, 2 * post, 1};
+    if (ctx->krylov && pre >= 1 && post == pre + 1) c.npre = c.npost = 2 * pre + 1;
+    if (c.npre > 0) c.post_first = (c.npre - 1) & 1;
+    return c;
+}
+
+// ncol colours of red-black sweeps on a five-point level, starting with `first`.  zero: x holds no
+// values yet and stands for x = 0 (the first colour, red, then needs no neighbour).  first_done:
+// that first colour was already done by the restriction that produced b (k_restrict5 with the
+// coarse 1/diag).
 template <class T>
-static void smooth(impec_ctx* ctx, Level& Lv, int sweeps, bool reverse, bool zero = false, bool first_done = false) {
+static void smooth(impec_ctx* ctx, Level& Lv, int ncol, int first, bool zero = false, bool first_done = false) {
     const T *tx, *ty, *a9, *id;
     T *x, *b;
-    level_ptrs<T>(Lv, tx, ty, a9, id, x, b);
-    if (use_tile<T>(ctx, (size_t)(&Lv - ctx->L.data()))) {  // one launch per sweep, ping-pong
+    int c = 0;
+    if (use_tile<T>(ctx, (size_t)(&Lv - ctx->L.data()))) {  // two colours per launch, ping-pong
         const dim3 g((Lv.n2 + TILE_C - 1) / TILE_C, (Lv.n1 + TILE_R - 1) / TILE_R);
-        for (int s = 0; s < sweeps; ++s) {
+        for (; c + 2 <= ncol; c += 2) {
             level_ptrs<T>(Lv, tx, ty, a9, id, x, b);
             T* xo = level_alt<T>(Lv);
-            const int first = reverse ? 1 : 0;
             ++ctx->nlaunch;
-            if (zero && s == 0)  // x = 0: the first colour is b * idiag (first is red here)
+            if (zero && c == 0)  // x = 0: the first colour is b * idiag (first is red here)
                 launch_k(ctx->stream, k_rb_tile<T, true>, g, TILE_THREADS, 0, Lv.n1, Lv.n2, tx, ty, id, b, (const T*)x,
                          xo, first);
             else
@@ -1144,30 +1359,34 @@ static void smooth(impec_ctx* ctx, Level& Lv, int sweeps, bool reverse, bool zer
                          (const T*)x, xo, first);
             swap_iterate<T>(Lv);
         }
-        return;
     }
-    for (int s = 0; s < sweeps; ++s) {
-        if (Lv.kind == FACE5) {
-            const dim3 g = rb_grid(Lv);
-            for (int cc = 0; cc < 2; ++cc) {
-                const int col = reverse ? 1 - cc : cc;
-                if (zero && s == 0 && cc == 0) {
-                    if (first_done) continue;
-                    ++ctx->nlaunch;
-                    launch_k(ctx->stream, k_rb_zero<T>, g, dim3(BX, BY), 0, Lv.n1, Lv.n2, id, b, x, col);
-                } else {
-                    ++ctx->nlaunch;
-                    launch_k(ctx->stream, k_rb_face5<T>, g, dim3(BX, BY), 0, Lv.n1, Lv.n2, tx, ty, id, b, x, col);
-                }
-            }
+    level_ptrs<T>(Lv, tx, ty, a9, id, x, b);
+    const dim3 g = rb_grid(Lv);
+    for (; c < ncol; ++c) {
+        const int col = (first + c) & 1;
+        if (zero && c == 0) {
+            if (first_done) continue;
+            ++ctx->nlaunch;
+            launch_k(ctx->stream, k_rb_zero<T>, g, dim3(BX, BY), 0, Lv.n1, Lv.n2, id, b, x, col);
         } else {
-            dim3 g(((Lv.n2 + 1) / 2 + BX - 1) / BX, ((Lv.n1 + 1) / 2 + BY - 1) / BY);
-            for (int cc = 0; cc < 4; ++cc) {
-                int col = reverse ? 3 - cc : cc;
-                ++ctx->nlaunch, launch_k(ctx->stream, k_gs4_exp9<T>, g, dim3(BX, BY), 0, Lv.n1, Lv.n2, a9, id, b, x, col >> 1, col & 1);
-            }
+            ++ctx->nlaunch;
+            launch_k(ctx->stream, k_rb_face5<T>, g, dim3(BX, BY), 0, Lv.n1, Lv.n2, tx, ty, id, b, x, col);
         }
     }
+}
+
+// Four-colour sweeps of a nine-point level.
+template <class T>
+static void smooth9(impec_ctx* ctx, Level& Lv, int sweeps, bool reverse) {
+    const T *tx, *ty, *a9, *id;
+    T *x, *b;
+    level_ptrs<T>(Lv, tx, ty, a9, id, x, b);
+    dim3 g(((Lv.n2 + 1) / 2 + BX - 1) / BX, ((Lv.n1 + 1) / 2 + BY - 1) / BY);
+    for (int s = 0; s < sweeps; ++s)
+        for (int cc = 0; cc < 4; ++cc) {
+            int col = reverse ? 3 - cc : cc;
+            ++ctx->nlaunch, launch_k(ctx->stream, k_gs4_exp9<T>, g, dim3(BX, BY), 0, Lv.n1, Lv.n2, a9, id, b, x, col >> 1, col & 1);
+        }
 }
 
 // Shared-memory bytes the coarse CTA needs for levels l .. L-1.
@@ -1177,7 +1396,7 @@ static size_t coarse_bytes(const impec_ctx* ctx, size_t l) {
     for (size_t k = l; k < ctx->L.size(); ++k) {
         const Level& Lv = ctx->L[k];
         const size_t n = Lv.n();
-        b += Lv.kind == FACE5 ? (size_t)(Lv.n1 + 1) * Lv.n2 + (size_t)Lv.n1 * (Lv.n2 + 1) + 4 * n : 12 * n;
+        b += Lv.kind == FACE5 ? (size_t)(Lv.n1 + 1) * Lv.n2 + (size_t)Lv.n1 * (Lv.n2 + 1) + (k > l ? 8 : 4) * n : 12 * n;
     }
     return b * sizeof(T);
 }
@@ -1195,19 +1414,22 @@ static size_t coarse_start(const impec_ctx* ctx) {
 }
 
 // The colour whose residual the restriction skips: after a five-point pre-smoothing the colour
-// updated last (black, 1) has a residual of zero up to one rounding.  -1: none.  Every V-cycle
+// updated last has a residual of zero up to one rounding.  -1: none.  Every V-cycle
 // implementation (per-level, cluster, single-CTA) uses it, so they stay bit-identical.
 static int restrict_zero_color(const impec_ctx* ctx, const Level& Lv) {
-    return ctx->tune.rb_resid != 0 && Lv.kind == FACE5 && ctx->tune.pre >= 1 ? 1 : -1;
+    const int npre = colours(ctx).npre;
+    return ctx->tune.rb_resid != 0 && Lv.kind == FACE5 && npre > 0 ? (npre - 1) & 1 : -1;
 }
 
 template <class T>
 static void launch_coarse(impec_ctx* ctx, size_t lc) {
     CoarseArgs<T> A{};
     A.nl = (int)(ctx->L.size() - lc);
-    A.singular = ctx->singular;
-    A.pre = (int)ctx->tune.pre;
-    A.post = (int)ctx->tune.post;
+    const Colours col = colours(ctx);
+    const bool f5 = ctx->L[lc].kind == FACE5;
+    A.npre = f5 ? col.npre : 4 * (int)ctx->tune.pre;
+    A.npost = f5 ? col.npost : 4 * (int)ctx->tune.post;
+    A.post_first = col.post_first;
     A.zero_color = restrict_zero_color(ctx, ctx->L[lc]);
     A.dn = ctx->dense_n;
     A.dinv = ctx->dense_inv;
@@ -1218,7 +1440,7 @@ static void launch_coarse(impec_ctx* ctx, size_t lc) {
         level_ptrs<T>(Lv, tx, ty, a9, id, x, b);
         A.n1[k] = Lv.n1;
         A.n2[k] = Lv.n2;
-        A.tx[k] = tx; A.ty[k] = ty; A.a9[k] = a9; A.id[k] = id; A.dg[k] = level_diag<T>(Lv);
+        A.tx[k] = tx; A.ty[k] = ty; A.a9[k] = a9; A.id[k] = id; A.dg[k] = level_diag<T>(Lv); A.w4[k] = level_w4<T>(Lv);
         if (k == 0) { A.x0 = x; A.b0 = b; }
     }
     const size_t smem = coarse_bytes<T>(ctx, lc);
@@ -1240,20 +1462,23 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
     if (CS < 2 || nl < 2 || nl > (size_t)CL_MAXL || ctx->dense_n > CL_THREADS) return false;
     const long cta0 = ctx->tune.cl_cta0;
     A = ClusterArgs<T>{};
-    A.kind = ctx->L[ls].kind;
+    const Colours col = colours(ctx);
+    const int kind = ctx->L[ls].kind;
+    const bool f5 = kind == FACE5;
     A.nl = (int)nl;
-    A.singular = ctx->singular;
-    A.pre = (int)ctx->tune.pre;
-    A.post = (int)ctx->tune.post;
+    A.npre = f5 ? col.npre : 4 * (int)ctx->tune.pre;
+    A.npost = f5 ? col.npost : 4 * (int)ctx->tune.post;
+    A.post_first = col.post_first;
     A.zero_color = restrict_zero_color(ctx, ctx->L[ls]);
-    A.rb_skip = A.kind == FACE5 && ctx->tune.rb_skip != 0 && ctx->tune.pre >= 1 && ctx->tune.post >= 1 ? 1 : 0;
+    // five-point levels: its restriction knows one colour's residuals and weighted transfers only
+    if (f5 && (A.zero_color < 0 || !ctx->krylov)) return false;
     A.dn = ctx->dense_n;
     A.dinv = ctx->dense_inv;
     size_t off = 0;
     int nd = 0;
     for (size_t k = 0; k < nl; ++k) {
         Level& Lv = ctx->L[ls + k];
-        if (Lv.kind != A.kind) return false;
+        if (Lv.kind != kind || Lv.n() > 65536) return false;  // cl_div's range
         int R = Lv.n1;
         if (k + 1 < nl && nd == (int)k && (long)Lv.n() > cta0) {
             R = (Lv.n1 + CS - 1) / CS;
@@ -1264,13 +1489,16 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
         A.n2[k] = Lv.n2;
         A.rows[k] = R;
         const size_t n2 = (size_t)Lv.n2, r = (size_t)R;
-        const size_t ops = k + 1 < nl ? r * n2 : 0;  // nine-point: the dense level keeps x and b only
-        const size_t sz[6] = {A.kind == FACE5 ? (r + 1) * n2 : 9 * ops, A.kind == FACE5 ? r * (n2 + 1) : 0,
-                              A.kind == FACE5 ? r * n2 : ops, A.kind == FACE5 ? r * n2 : 0, r * n2, r * n2};
-        for (int a = 0; a < 6; ++a) {
+        const size_t ops = k + 1 < nl ? r * n2 : 0;  // the dense level keeps no operator
+        const size_t halo = f5 ? (r + 2) * n2 : r * n2, tr = f5 && k > 0 ? halo : 0;
+        const size_t sz[CL_ARRAYS] = {f5 ? (ops ? (r + 1) * n2 : 0) : 9 * ops, f5 && ops ? r * (n2 + 1) : 0, ops,
+                                      f5 ? ops : 0, halo, r * n2, 4 * tr, tr, tr};
+        for (int a = 0; a < CL_ARRAYS; ++a) {
             A.off[k][a] = (unsigned)off;
             off += sz[a];
         }
+        A.rhalf[k] = 1.0f / (float)((Lv.n2 + 1) / 2);
+        A.rn2[k] = 1.0f / (float)Lv.n2;
         const T *tx, *ty, *a9, *id;
         T *x, *b;
         level_ptrs<T>(Lv, tx, ty, a9, id, x, b);
@@ -1278,6 +1506,7 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
         A.ty[k] = ty;
         A.id[k] = id;
         A.dg[k] = level_diag<T>(Lv);
+        A.w4[k] = level_w4<T>(Lv);
         A.a9[k] = a9;
         if (k == 0) {
             A.x0 = x;
@@ -1295,10 +1524,9 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
 template <class T>
 static size_t cluster_start(impec_ctx* ctx) {
     if (ctx->cl_size < 2 || ctx->tune.cluster == 0) return SIZE_MAX;
-    // FP32 nine-point cycles keep their per-level and single-CTA kernels: each level's four
-    // colours are cheap launches there, and ten cluster-barrier phases per level cost more
-    // (mixed solve at 1024^2, nu = 2/3: 5.10 ms with the cluster against 4.76 ms without)
-    if (sizeof(T) == 4 && ctx->L[0].kind != FACE5) return SIZE_MAX;
+    // FP32 cycles of nine-point systems keep their per-level and single-CTA kernels (with nine-point
+    // levels the cluster costs more: mixed solve at 1024^2, nu = 2/3: 5.10 against 4.76 ms)
+    if (sizeof(T) == 4 && ctx->L[0].a9) return SIZE_MAX;
     const long cells = ctx->tune.cl_cells;
     ClusterArgs<T> A;
     size_t smem;
@@ -1309,10 +1537,11 @@ static size_t cluster_start(impec_ctx* ctx) {
 }
 
 template <class T>
-static void launch_cluster(impec_ctx* ctx, size_t ls) {
+static void launch_cluster(impec_ctx* ctx, size_t ls, bool zero) {
     ClusterArgs<T> A;
     size_t smem = 0;
     cluster_plan<T>(ctx, ls, A, smem);
+    A.zero0 = zero ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctx->cl_size);
     cfg.blockDim = dim3(CL_THREADS);
@@ -1328,16 +1557,17 @@ static void launch_cluster(impec_ctx* ctx, size_t ls) {
     cfg.attrs = at;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
     ++ctx->nlaunch;
-    cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T>, A);
+    if (ctx->L[ls].kind == FACE5) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5>, A);
+    else if constexpr (sizeof(T) == 8) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, EXP9>, A);
 }
 
-// Whether the V-cycle at level l runs per-level red-black kernels, so that a cycle started
-// from x = 0 needs no zero fill of the level's iterate (the first colour is k_rb_zero).
+// Whether a five-point V-cycle at level l started from x = 0 needs no zero fill of the level's
+// iterate: the per-level kernels start with k_rb_zero, the cluster with its own zero-start colour.
 template <class T>
 static bool zero_start_free(impec_ctx* ctx, size_t l) {
     const Level& F = ctx->L[l];
-    return ctx->tune.rb_skip != 0 && F.kind == FACE5 && ctx->tune.pre >= 1 && l != cluster_start<T>(ctx) &&
-           l != coarse_start<T>(ctx);
+    return ctx->tune.rb_skip != 0 && F.kind == FACE5 && ctx->tune.pre >= 1 &&
+           (l == cluster_start<T>(ctx) || l != coarse_start<T>(ctx));
 }
 
 // One V-cycle from level l down.  zero: the level's iterate stands for x = 0; unless
@@ -1349,8 +1579,9 @@ static void vcycle(impec_ctx* ctx, size_t l, bool zero, bool first_done = false)
     const T *tx, *ty, *a9, *id;
     T *x, *b;
     level_ptrs<T>(F, tx, ty, a9, id, x, b);
-    if (l == cluster_start<T>(ctx)) {
-        launch_cluster<T>(ctx, l);
+    const size_t cl = cluster_start<T>(ctx);
+    if (l == cl) {
+        launch_cluster<T>(ctx, l, zero && zero_start_free<T>(ctx, l));
         return;
     }
     const size_t lc = coarse_start<T>(ctx);
@@ -1362,25 +1593,42 @@ static void vcycle(impec_ctx* ctx, size_t l, bool zero, bool first_done = false)
     const T *ctx_, *cty, *ca9, *cid;
     T *cx, *cb;
     level_ptrs<T>(C, ctx_, cty, ca9, cid, cx, cb);
+    const unsigned char* mask = l == 0 && ctx->dir_row >= 0 ? ctx->dmask : nullptr;
+    if (F.kind != FACE5) {
+        smooth9<T>(ctx, F, (int)ctx->tune.pre, false);
+        ++ctx->nlaunch;
+        launch_k(ctx->stream, k_restrict9<T>, grid2(C.n1, C.n2), dim3(BX, BY), 0, F.n1, F.n2, a9, (const T*)b, (const T*)x,
+                 C.n1, C.n2, cb, cx);
+        vcycle<T>(ctx, l + 1, true);
+        ++ctx->nlaunch;
+        launch_k(ctx->stream, k_prolong<T>, grid2(F.n1, F.n2), dim3(BX, BY), 0, F.n1, F.n2, x, C.n1, C.n2, (const T*)cx,
+                 (const T*)nullptr, mask);
+        smooth9<T>(ctx, F, (int)ctx->tune.post, true);
+        return;
+    }
+    const Colours col = colours(ctx);
     const bool zs = zero && zero_start_free<T>(ctx, l);
-    smooth<T>(ctx, F, (int)ctx->tune.pre, false, zs, zs && first_done);
+    smooth<T>(ctx, F, col.npre, 0, zs, zs && first_done);
     level_ptrs<T>(F, tx, ty, a9, id, x, b);  // the sweep may have moved the iterate (ping-pong)
     ++ctx->nlaunch;
-    const int zero_color = restrict_zero_color(ctx, F);
-    // the coarse cycle's first colour is done here, unless that level sweeps in one launch
-    // (its zero-start sweep computes the first colour itself)
-    const bool cz = zero_start_free<T>(ctx, l + 1) && !use_tile<T>(ctx, l + 1);
-    launch_k(ctx->stream, k_restrict<T>, grid2(C.n1, C.n2), dim3(BX, BY), 0, F, tx, ty, a9, level_diag<T>(F), b, x,
-             C.n1, C.n2, cb, cx, zero_color, cz ? (const T*)cid : nullptr);
+    const int zc = restrict_zero_color(ctx, F);
+    // the coarse cycle's first colour is done here, unless that level's first launch does it (the
+    // one-launch sweep, the cluster)
+    const bool cz = zero_start_free<T>(ctx, l + 1) && !use_tile<T>(ctx, l + 1) && l + 1 != cl;
+    const auto k_restrict = zc == 1 ? k_restrict5<T, 1> : zc == 0 ? k_restrict5<T, 0> : k_restrict5<T, -1>;
+    launch_k(ctx->stream, k_restrict, dim3((C.n2 + RS_C - 1) / RS_C, (C.n1 + RS_R - 1) / RS_R), dim3(RS_C, RS_R), 0, F.n1,
+             F.n2, tx, ty, level_diag<T>(F), (const T*)b, (const T*)x, C.n1, C.n2, level_w4<T>(C), cb, cx,
+             cz ? (const T*)cid : nullptr);
     vcycle<T>(ctx, l + 1, true, cz);
     level_ptrs<T>(C, ctx_, cty, ca9, cid, cx, cb);  // the coarse iterate may have moved too
-    const unsigned char* mask = l == 0 && ctx->dir_row >= 0 ? ctx->dmask : nullptr;
     ++ctx->nlaunch;
-    if (ctx->tune.rb_skip != 0 && F.kind == FACE5 && ctx->tune.post >= 1)  // the black cells are overwritten next
-        launch_k(ctx->stream, k_prolong_rb<T>, rb_grid(F), dim3(BX, BY), 0, F.n1, F.n2, x, C.n1, C.n2, cx, mask, 0);
+    if (ctx->tune.rb_skip != 0 && col.npost > 0)  // cells of the post-smoothing's first colour are overwritten next
+        launch_k(ctx->stream, k_prolong_rb<T>, rb_grid(F), dim3(BX, BY), 0, F.n1, F.n2, x, C.n1, C.n2, (const T*)cx,
+                 level_w4<T>(C), mask, 1 - col.post_first);
     else
-        launch_k(ctx->stream, k_prolong<T>, grid2(F.n1, F.n2), dim3(BX, BY), 0, F.n1, F.n2, x, C.n1, C.n2, cx, mask);
-    smooth<T>(ctx, F, (int)ctx->tune.post, true);
+        launch_k(ctx->stream, k_prolong<T>, grid2(F.n1, F.n2), dim3(BX, BY), 0, F.n1, F.n2, x, C.n1, C.n2, (const T*)cx,
+                 level_w4<T>(C), mask);
+    smooth<T>(ctx, F, col.npost, col.post_first);
 }
 
 // Convergence check of the solve loop (one thread): relres = ||r||/||f||; decides whether
@@ -1433,18 +1681,32 @@ __device__ __forceinline__ double cg_z(const double* __restrict__ z, const float
 
 // (r, z) and (z, q) into out[0], out[1].  With S (CG, out = &S->pcg_rz), the last block also
 // stores the direction's beta = -alpha_old (z, q) / (z, r)_old (0 on the first iteration).
+// K = 4 (singular systems): also the sums of z and r, with which (r, z) is taken without either's
+// mean.  The rounded rows of the operator do not quite sum to zero, so r has a small mean that
+// no direction removes; the cycle answers it with a far larger mean of z (four times the
+// right-hand side per cell on each coarser level), and their product came to outweigh the rest of
+// (r, z): past its best iterate CG then diverged (1024^2, nu = 2/3: from 8e-11 of ||f|| to 1e-6 in
+// five iterations).
+template <int K>
 __global__ void __launch_bounds__(RED_THREADS) k_cg_dots(int n1, int n2, const double* __restrict__ r,
                                                          const double* __restrict__ z, const float* __restrict__ z32,
                                                          const double* __restrict__ q, double* partials, int mb,
                                                          unsigned* counter, double* out, DevScalars* S) {
     pdl_enter();
-    double acc[2] = {0.0, 0.0};
+    double acc[K];
+#pragma unroll
+    for (int e = 0; e < K; ++e) acc[e] = 0.0;
     for_cells(n1, n2, [&](int, int, size_t k) {
-        const double zz = cg_z(z, z32, k);
-        acc[0] += r[k] * zz;
+        const double zz = cg_z(z, z32, k), rr = r[k];
+        acc[0] += rr * zz;
         acc[1] += zz * q[k];
+        if (K == 4) {
+            acc[K - 2] += zz;
+            acc[K - 1] += rr;
+        }
     });
-    if (grid_reduce<2>(acc, 0u, partials, mb, counter, out) && threadIdx.x == 0 && S) {
+    if (grid_reduce<K>(acc, 0u, partials, mb, counter, out) && threadIdx.x == 0 && S) {
+        if (K == 4) S->pcg_rz -= S->pcg_zsum * S->pcg_rsum / ((double)n1 * n2);
         const bool first = S->mg_cycles == 0 || S->pcg_rz_old == 0.0;
         S->pcg_beta = first ? 0.0 : -S->pcg_alpha * S->pcg_zq / S->pcg_rz_old;
     }
@@ -1470,8 +1732,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_apply(Level F, const double*
     double acc[1] = {0.0};
     for_cells(F.n1, F.n2, [&](int i, int j, size_t k) {
         const int n1 = F.n1, n2 = F.n2;
-        double s = F.diag[k] * p[k];
-        if (F.kind == FACE5) {
+        double s = (F.a9 ? F.a9 : F.diag)[k] * p[k];
+        if (!F.a9) {
             if (i > 0) s -= F.tx[k] * p[k - n2];
             if (i < n1 - 1) s -= F.tx[k + n2] * p[k + n2];
             if (j > 0) s -= F.ty[IX(i, j, n2 + 1)] * p[k - 1];
@@ -1554,7 +1816,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_verify(Level F, const double
     }
     double acc[1] = {0.0};
     for_cells(F.n1, F.n2, [&](int i, int j, size_t k) {
-        double r = resid<double>(F, i, j, F.tx, F.ty, F.a9, F.diag, f, x);
+        double r = resid_op(F, i, j, f, x);
         r64[k] = r;
         if (r32) r32[k] = (float)r;
         if ((int)k == pin) r = 0.0;  // as k_fine_resid
@@ -1613,7 +1875,7 @@ static impec_status learned_guess(impec_ctx* ctx, double* x) {
     launch_k(ctx->stream, k_cg_apply, blocks, RED_THREADS, 0, F, (const double*)ctx->lrn_d, ctx->lrn_Ad, ctx->partials,
              ctx->max_blocks, ctx->counter, &S->pcg_pq, (DevScalars*)nullptr);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_dots, blocks, RED_THREADS, 0, F.n1, F.n2, (const double*)ctx->lrn_r0,
+    launch_k(ctx->stream, k_cg_dots<2>, blocks, RED_THREADS, 0, F.n1, F.n2, (const double*)ctx->lrn_r0,
              (const double*)ctx->lrn_d, (const float*)nullptr, (const double*)ctx->lrn_Ad, ctx->partials,
              ctx->max_blocks, ctx->counter, &S->pcg_rz, (DevScalars*)nullptr);
     ++ctx->nlaunch;
@@ -1712,8 +1974,8 @@ impec_status pressure_iteration(impec_ctx* ctx, double tol, cudaGraphConditional
     const float* z32 = mixed ? F.x32 : nullptr;
     const int cap = red_cap(ctx->num_sms, ctx->max_blocks), blocks = seg_blocks(F.n1, F.n2, cap);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_dots, blocks, RED_THREADS, 0, F.n1, F.n2, r, z, z32, ctx->cg_q, ctx->partials,
-             ctx->max_blocks, ctx->counter, &S->pcg_rz, S);
+    launch_k(ctx->stream, ctx->singular ? k_cg_dots<4> : k_cg_dots<2>, blocks, RED_THREADS, 0, F.n1, F.n2, (const double*)r, z, z32,
+             (const double*)ctx->cg_q, ctx->partials, ctx->max_blocks, ctx->counter, &S->pcg_rz, S);
     ++ctx->nlaunch;
     launch_k(ctx->stream, k_cg_direction, ctx->num_sms * 4, 256, 0, n, z, z32, ctx->cg_p, S);
     ++ctx->nlaunch;
@@ -1929,8 +2191,8 @@ extern "C" impec_status impec_time_kernel_cold(impec_ctx* ctx, int which, int re
     for (int r = 0; r < reps; ++r) {
         IMPEC_CUDA_TRY(cudaMemsetAsync(flush, r & 0xff, flush_bytes, ctx->stream));
         IMPEC_CUDA_TRY(cudaEventRecord(e0, ctx->stream));
-        if (which == 0) smooth<double>(ctx, F, 1, false);
-        else smooth<float>(ctx, F, 1, false);
+        if (which == 0) smooth<double>(ctx, F, 2, 0);
+        else smooth<float>(ctx, F, 2, 0);
         IMPEC_CUDA_TRY(cudaEventRecord(e1, ctx->stream));
         IMPEC_CUDA_TRY(cudaEventSynchronize(e1));
         float t = 0;
@@ -1972,8 +2234,8 @@ extern "C" impec_status impec_time_kernel(impec_ctx* ctx, int which, int reps, d
     IMPEC_CUDA_TRY(cudaEventRecord(e0, ctx->stream));
     for (int r = 0; r < reps; ++r) {
         switch (which) {
-            case 0: smooth<double>(ctx, F, 1, false); b = n * 8 * (4 + coef); break;  // x,b,idiag r + x w + operator
-            case 1: smooth<float>(ctx, F, 1, false); b = n * 4 * (4 + coef); break;
+            case 0: F.kind == FACE5 ? smooth<double>(ctx, F, 2, 0) : smooth9<double>(ctx, F, 1, false); b = n * 8 * (4 + coef); break;  // x,b,idiag r + x w + operator
+            case 1: F.kind == FACE5 ? smooth<float>(ctx, F, 2, 0) : smooth9<float>(ctx, F, 1, false); b = n * 4 * (4 + coef); break;
             case 2: IMPEC_TRY(pressure_residual(ctx)); b = n * 8 * (2 + coef) + (ctx->P.precision ? 4 * n : 0); break;
             case 3: IMPEC_TRY(advect_x_dev(ctx, ctx->c, ctx->t1, ctx->u, 1.0, &ctx->dscal->dt)); b = n * 24; break;
             case 4: IMPEC_TRY(advect_y_dev(ctx, ctx->c, ctx->t1, ctx->v, 1.0, &ctx->dscal->dt)); b = n * 24; break;
