@@ -135,7 +135,7 @@ _SIGS = {
 }
 
 KERNELS = {0: "k_rb_face5<double> (fine RB-GS sweep, FP64)", 1: "k_rb_face5<float> (fine RB-GS sweep, FP32)",
-           2: "k_fine_resid (FP64 residual + norm)", 3: "k_sweep_x (MUSCL x-sweep)", 4: "k_sweep_y (MUSCL y-sweep)"}
+           2: "k_fine_resid (FP64 residual + norm)", 3: "k_advect_tile (x-sweep)", 4: "k_advect_tile (y-sweep)"}
 
 
 def launch_count(ctx) -> int:

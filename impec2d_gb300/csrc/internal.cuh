@@ -258,10 +258,9 @@ impec_status max_stable_dt_dev(impec_ctx* ctx, const double* u, const double* v)
 // transport.cu
 impec_status tr_integrate_dev(impec_ctx* ctx, double* c, double dt_scale, const double* dt_dev, int slot);
 impec_status advect_x_dev(impec_ctx* ctx, const double* cin, double* cout, const double* u, double dt_scale,
-                          const double* dt_dev, const double* cghost = nullptr);
+                          const double* dt_dev);
 impec_status advect_y_dev(impec_ctx* ctx, const double* cin, double* cout, const double* v, double dt_scale, const double* dt_dev);
 impec_status advect_split_dev(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev, int* pfs);
-impec_status average_dev(impec_ctx* ctx, double* c, const double* a, const double* b);
 // dispersion.cu
 impec_status cn_setup(impec_ctx* ctx, const double* u, const double* v, double dt_scale, const double* dt_dev);
 impec_status cn_prepare(impec_ctx* ctx, double* c, double dt_scale, const double* dt_dev, bool residual = true);

@@ -53,40 +53,30 @@ impec_status tr_integrate_dev(impec_ctx* ctx, double* c, double dt_scale, const 
     return IMPEC_OK;
 }
 
-// ---------------------------------------------------------------- MUSCL-Hancock / upwind
-// Cell reconstruction and Hancock half step (src/MUSCLSplitSolver.cpp:54-93, :121-129).
-// The reference limiter xi(r) = min(2r/(1+r), 2/(1+r)) times (a+b)/2 equals, in exact
-// arithmetic, minmod(a, b) (r = a/b <= 1 gives a, r > 1 gives b, a*b <= 0 gives 0); the
-// selection below evaluates that value without the three divisions.
-// kap = 0.5 dt / (dx phi).  sl: state at the cell's left face, sr: at its right face.
+// ---------------------------------------------------------------- limiter and upwind selection
 // Comparisons on the integer pipe.  FP64 compares issue on the FP64 pipe, the bottleneck of
 // the transport kernels on GB300; for non-NaN doubles these are exact equivalents (a NaN
 // operand still yields a NaN result through the arithmetic around them).
 // x > 0: the bit pattern, read as a signed integer, is positive (+0 is 0, negatives are < 0).
 __device__ __forceinline__ bool pos(double x) { return __double_as_longlong(x) > 0LL; }
-// |a| <= |b|: IEEE magnitudes order like their bit patterns with the sign bit cleared.
-__device__ __forceinline__ bool abs_le(double a, double b) {
-    return (__double_as_longlong(a) & 0x7fffffffffffffffLL) <= (__double_as_longlong(b) & 0x7fffffffffffffffLL);
+// The reference limiter xi(r) = min(2r/(1+r), 2/(1+r)) times (a+b)/2 (src/MUSCLSplitSolver.cpp:54-93)
+// equals, in exact arithmetic, minmod(a, b): r = a/b <= 1 gives a, r > 1 gives b, opposite signs give 0.
+// IEEE magnitudes order like their bit patterns with the sign bit cleared.  The halves are masked
+// and compared as 32-bit words: a 64-bit mask of the sign bit is compiled to an FP64 absolute
+// value, one more FP64 instruction per slope (1024^2, X then Y: 29 instead of 26 per cell).
+__device__ __forceinline__ double minmod(double a, double b) {
+    const int ha = __double2hiint(a), hb = __double2hiint(b), la = __double2loint(a), lb = __double2loint(b);
+    const unsigned ua = ha & 0x7fffffff, ub = hb & 0x7fffffff;
+    const bool opposite = (ha ^ hb) < 0, le = ua < ub || (ua == ub && (unsigned)la <= (unsigned)lb);
+    return __hiloint2double(opposite ? 0 : le ? ha : hb, opposite ? 0 : le ? la : lb);
 }
 
-__device__ __forceinline__ void hancock(double cm, double c0, double cp, double ul, double ur, double kap,
-                                        double& sl, double& sr) {
-    double a = c0 - cm, b = cp - c0;
-    double d = pos(a * b) ? (abs_le(a, b) ? a : b) : 0.0;
-    double UR = fma(0.5, d, c0), UL = fma(-0.5, d, c0);
-    double df = kap * (ul * UL - ur * UR);
-    sl = UL + df;
-    sr = UR + df;
-}
-
-// WAF intercell flux (times phi) for the split sweeps (hyper_method "waf_split" / "waf"; the
-// reference parses these, src/SimParams.cpp:200-208, but ships no source for them).  Toro's
-// weighted average flux with the van Leer limiter (Riemann Solvers and Numerical Methods for
-// Fluid Dynamics, 3rd ed., ch. 13-14): cr = u dt / (dx phi) = u lam is the Courant number,
-// A = 1 - (1 - |cr|) * 2r / (1 + r) for r > 0 (else 1, the upwind flux), r = upwind jump /
-// local jump, and F = u ((1 + s A) cL + (1 - s A) cR) / 2 with s = sign(cr).
-__device__ __forceinline__ double waf_face(double u, double lam, double cLL, double cL, double cR, double cRR) {
-    const double cr = u * lam;
+// WAF intercell flux times dt / (dx phi) (hyper_method "waf_split" / "waf"; the reference parses
+// these, src/SimParams.cpp:200-208, but ships no source for them).  Toro's weighted average flux
+// with the van Leer limiter (Riemann Solvers and Numerical Methods for Fluid Dynamics, 3rd ed., ch.
+// 13-14): cr is the face's Courant number, A = 1 - (1 - |cr|) * 2r / (1 + r) for r > 0 (else 1, the
+// upwind flux), r = upwind jump / local jump, F = cr ((1 + s A) cL + (1 - s A) cR) / 2, s = sign(cr).
+__device__ __forceinline__ double waf_face(double cr, double cLL, double cL, double cR, double cRR) {
     const double dloc = cR - cL;
     double A = 1.0;
     if (dloc != 0.0) {
@@ -95,7 +85,7 @@ __device__ __forceinline__ double waf_face(double u, double lam, double cLL, dou
         if (r > 0.0) A = 1.0 - (1.0 - fabs(cr)) * (2.0 * r / (1.0 + r));
     }
     const double s = cr > 0.0 ? 1.0 : (cr < 0.0 ? -1.0 : 0.0);
-    return 0.5 * (1.0 + s * A) * (u * cL) + 0.5 * (1.0 - s * A) * (u * cR);
+    return 0.5 * (1.0 + s * A) * (cr * cL) + 0.5 * (1.0 - s * A) * (cr * cR);
 }
 
 // Reflected (or wrapped) cell index, clamped into [0, n): tile loads may reach further than
@@ -121,6 +111,21 @@ __device__ __forceinline__ double face_at(const double* __restrict__ u, int f, i
     return s * u[(size_t)ff * stride_f + off];
 }
 
+// ---------------------------------------------------------------- split sweeps cell by cell
+// For grids too small to fill the GPU with tiles (below): a thread per cell forms everything its
+// cell needs, more operations than a tile's strips but one short chain per launch.
+//
+// Cell reconstruction and Hancock half step (src/MUSCLSplitSolver.cpp:54-93, :121-129).
+// kap = 0.5 dt / (dx phi).  sl: state at the cell's left face, sr: at its right face.
+__device__ __forceinline__ void hancock(double cm, double c0, double cp, double ul, double ur, double kap,
+                                        double& sl, double& sr) {
+    const double d = minmod(c0 - cm, cp - c0);
+    const double UR = fma(0.5, d, c0), UL = fma(-0.5, d, c0);
+    const double df = kap * (ul * UL - ur * UR);
+    sl = UL + df;
+    sr = UR + df;
+}
+
 // One sweep along a line: cells k in [0,n) at positions base + k*cs of c, faces f in [0,n]
 // at base_f + f*fs of the face array.  Computes the update of cell k.
 // cg (may be null) supplies the cells outside [0,n) instead of the reflection of c.
@@ -143,9 +148,7 @@ __device__ __forceinline__ double sweep_cell(const double* __restrict__ c, const
     }
     if (SCHEME == IMPEC_WAFSPLIT) {
         double cmm = C(k - 2), cm = C(k - 1), c0 = C(k), cp = C(k + 1), cpp = C(k + 2);
-        Fw = waf_face(uw, lam, cmm, cm, c0, cp);
-        Fe = waf_face(ue, lam, cm, c0, cp, cpp);
-        return c0 + lam * (Fw - Fe);
+        return c0 + (waf_face(uw * lam, cmm, cm, c0, cp) - waf_face(ue * lam, cm, c0, cp, cpp));
     }
     double cmm = C(k - 2), cm = C(k - 1), c0 = C(k), cp = C(k + 1), cpp = C(k + 2);
     double uww = U(k - 1), uee = U(k + 2);
@@ -186,131 +189,274 @@ __global__ void k_sweep_y(int n1, int n2, const double* __restrict__ cin, double
     cout[IX(i, j, n2)] = sweep_cell<SCHEME, BC>(cin, nullptr, IX(i, 0, n2), 1, v, IX(i, 0, n2 + 1), 1, j, n2, kap, lam);
 }
 
-__global__ void k_average(size_t n, double* __restrict__ c, const double* __restrict__ a, const double* __restrict__ b) {
-    pdl_enter();
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        c[k] = 0.5 * (a[k] + b[k]);
-}
+// ---------------------------------------------------------------- split sweeps on a tile
+// The dimensionally split update (src/HyperbolicSplitSolver.cpp:51-159) of one TI x TJ tile: X, Y,
+// Y after X, X after Y, or (symmetric-parallel) the average of the last two.  All of them are
+// FP64-bound on GB300 (1.06 TFLOP/s), so the arithmetic is arranged for the fewest operations.
+//
+// With W = dt u / (dx phi) at the faces, the MUSCL-Hancock sweep (src/MUSCLSplitSolver.cpp:54-189)
+//   L, R = c -+ d/2 + (W_w (c - d/2) - W_e (c + d/2)) / 2,   c' = c + W_w s_w - W_e s_e,
+// s the upwind cell's state at the face (R of the cell before it where W > 0, else L of the cell
+// after it), is evaluated as
+//   base = E c,  E = 1 + (W_w - W_e) / 2;   s = base_up + d_up F,  F = (1/2 - S/4) or -(1/2 + S/4),
+// S = W_w + W_e of the upwind cell.  E (per cell) and F (per face) hold no c: the two sweeps that a
+// symmetric update makes in each direction share them.  A thread takes a strip of four cells along
+// the sweep, so that slopes, bases and face states are computed once (plus the strip's ends): 6.5
+// operations per cell and sweep, 43 per cell of a symmetric update with the halo, against 72
+// when every cell formed both of its states and both of its fluxes.  1024^2, symmetric MUSCL:
+// 152 us before, 95 now (84% of the FP64 pipe); a call with X then Y 160 -> 80 us, Strang 308 -> 118.
+//
+// The tile: an SM's FP64 units belong to its four sub-partitions (one warp instruction in 64
+// cycles each), so a block's warps should fill them evenly.  32 x 32 with strips of four gives 18
+// warps for the first sweeps and 16 for the second ones; strips of eight need fewer operations (39)
+// but come as 9 and 8 warps, which leaves sub-partitions idle (125 against 109 us a call), as do
+// 16 x 32 (118) and 28 x 28 with strips of seven (118).
+//
+// Shared memory (pitch 37: rows fall into different banks, so a warp can take one strip each of
+// 32 rows or of 32 columns): c with its two-cell halo, W, E and F of both directions, and the
+// results of the first sweeps (X(c) in the place of c); 85 KB, two blocks per SM.  The first
+// sweep covers the cells that the second one reads: 36 lines instead of 32.
+constexpr int TJ = 32, STRIP = 4, TP = (TJ + 4) | 1;
+enum { MODE_SYM = 0, MODE_XY = 1, MODE_YX = 2, MODE_X = 3, MODE_Y = 4 };  // XY: X, then Y on its result
+template <int TI, int MODE>
+struct Tile {
+    static constexpr int X1 = (TJ + 4) * (TI / STRIP), Y1 = (TI + 4) * (TJ / STRIP);  // strips of a first sweep
+    static constexpr int X2 = TJ * (TI / STRIP), Y2 = TI * (TJ / STRIP);              // strips of a second one
+    static constexpr int STRIPS = MODE == MODE_SYM  ? X1 + Y1
+                                  : MODE == MODE_XY ? (X1 > Y2 ? X1 : Y2)
+                                  : MODE == MODE_YX ? (Y1 > X2 ? Y1 : X2)
+                                  : MODE == MODE_X  ? X1
+                                                    : Y1;
+    static constexpr int THREADS = (STRIPS + 31) / 32 * 32;  // the strips of the largest phase, in whole warps
+    // planes of shared memory: c, three per direction, Y(c) beside X(c)
+    static constexpr int PLANE = (TI + 4) * TP;
+    static constexpr size_t SMEM = sizeof(double) * PLANE * (MODE == MODE_SYM ? 8 : MODE == MODE_X || MODE == MODE_Y ? 4 : 7);
+};
 
-// ---------------------------------------------------------------- fused symmetric-parallel update
-// One CTA owns a TI x TJ tile of the output.  It loads c (2-cell halo), the x-face velocities
-// u and the y-face velocities v it needs (ghost values by the reflections above), then
-// computes in shared memory  XY = Y(X(c)),  YX = X(Y(c))  and writes (XY + YX)/2, which is
-// AdvectSplit's SYMMETRIC_PARALLEL branch (src/HyperbolicSplitSolver.cpp:87-103).  Each
-// sweep first computes the two Hancock states of every cell it needs once, then the fluxes
-// and updates; the arithmetic per cell is that of sweep_cell, so results are identical.
-constexpr int TI = 16, TJ = 32, FUSED_THREADS = 256;
-constexpr int CW = TJ + 4;                // row width of c, c1 (j in [j0-2, j0+TJ+2))
-constexpr int VW = TJ + 3;                // row width of v faces (fj in [j0-1, j0+TJ+2))
-constexpr int HMAX = (TI + 4) * (TJ + 2) > (TI + 2) * (TJ + 4) ? (TI + 4) * (TJ + 2) : (TI + 2) * (TJ + 4);
+struct TileArgs {
+    int n1, n2;
+    const double* cin;
+    const double* cghost;  // cells beyond the x ends are taken from here (null: from cin)
+    double* cout;
+    const double* u;
+    const double* v;
+    const double* dt;      // device scalar
+    double fx, fy;         // scale / (dx phi), scale / (dy phi)
+    int row0;              // tile row of block row b: b == 0 ? 0 : row0 + b
+};
 
+// One strip: out[k] = new value of cell k (cells at c + k cs, faces at W + k ws, E at e + k cs', F as W).
+// c[-2 .. 9], W[0 .. 8], E[-1 .. 8], F[0 .. 8] are read.
 template <int SCHEME>
-__device__ __forceinline__ void states(double cm, double c0, double cp, double ul, double ur, double kap, double& sl,
-                                       double& sr) {
-    if (SCHEME == IMPEC_UPWINDSPLIT) { sl = sr = c0; return; }
-    hancock(cm, c0, cp, ul, ur, kap, sl, sr);
+__device__ __forceinline__ void sweep_strip(const double* c, int cs, const double* W, const double* E, const double* F,
+                                            int ws, double (&out)[STRIP]) {
+    if (SCHEME == IMPEC_WAFSPLIT) {
+        double cll = c[-2 * cs], cl = c[-cs], c0 = c[0], t = 0.0;
+#pragma unroll
+        for (int m = 0; m <= STRIP; ++m) {
+            const double cr = c[(m + 1) * cs], f = waf_face(W[m * ws], cll, cl, c0, cr);
+            if (m > 0) out[m - 1] = t - f;
+            t = c0 + f;
+            cll = cl; cl = c0; c0 = cr;
+        }
+        return;
+    }
+    if (SCHEME == IMPEC_UPWINDSPLIT) {  // src/UpwindSplitSolver.cpp:43-65
+        double cl = c[-cs], t = 0.0;
+#pragma unroll
+        for (int m = 0; m <= STRIP; ++m) {
+            const double c0 = c[m * cs], w = W[m * ws], s = pos(w) ? cl : c0;
+            if (m > 0) out[m - 1] = fma(-w, s, t);
+            t = fma(w, s, c0);
+            cl = c0;
+        }
+        return;
+    }
+    double c0 = c[-cs], a = c0 - c[-2 * cs], d1 = 0.0, b1 = 0.0, t = 0.0;
+#pragma unroll
+    for (int m = -1; m <= STRIP; ++m) {
+        const double cr = c[(m + 1) * cs], an = cr - c0;
+        const double d = minmod(a, an), b = E[m * ws] * c0;
+        if (m >= 0) {
+            const double w = W[m * ws];
+            const bool p = pos(w);
+            const double s = fma(p ? d1 : d, F[m * ws], p ? b1 : b);
+            if (m > 0) out[m - 1] = fma(-w, s, t);
+            t = fma(w, s, c0);
+        }
+        c0 = cr; a = an; d1 = d; b1 = b;
+    }
 }
 
-template <int SCHEME, int BC>
-__global__ void __launch_bounds__(FUSED_THREADS) k_advect_symmetric(int n1, int n2, const double* __restrict__ cin,
-                                                                     double* __restrict__ cout,
-                                                                     const double* __restrict__ u,
-                                                                     const double* __restrict__ v,
-                                                                     const double* __restrict__ dt_dev, double inv_dx_phi,
-                                                                     double inv_dy_phi) {
+template <int SCHEME, int BC, int MODE, int TI>
+__global__ void __launch_bounds__(Tile<TI, MODE>::THREADS) k_advect_tile(const TileArgs A) {
     pdl_enter();
-    __shared__ double sc[(TI + 4) * CW];   // c, rows i0-2 .. i0+TI+1
-    __shared__ double su[(TI + 3) * CW];   // u faces fi in [i0-1, i0+TI+1], cols j0-2 ..
-    __shared__ double sv[(TI + 4) * VW];   // v faces, rows i0-2 .., fj in [j0-1, j0+TJ+1]
-    __shared__ double s1[TI * CW];         // X(c) on rows i0..i0+TI-1, cols j0-2 ..
-    __shared__ double s2[(TI + 4) * TJ];   // Y(c) on rows i0-2 .., cols j0 ..
-    __shared__ double sxy[TI * TJ];        // Y(X(c))
-    __shared__ double hl[HMAX], hr[HMAX];  // Hancock states at the left / right face of a cell
-    const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ, t = threadIdx.x;
-    const double dt = dt_dev[0];
-    const double lx = dt * inv_dx_phi, kx = 0.5 * lx, ly = dt * inv_dy_phi, ky = 0.5 * ly;
-    // ---- loads (reflected ghosts) ----
-    for (int k = t; k < (TI + 4) * CW; k += FUSED_THREADS) {
-        int a = k / CW, b = k % CW;
-        sc[k] = cin[IX(cell_at<BC>(i0 - 2 + a, n1), cell_at<BC>(j0 - 2 + b, n2), n2)];
-    }
-    for (int k = t; k < (TI + 3) * CW; k += FUSED_THREADS) {
-        int a = k / CW, b = k % CW;
-        su[k] = face_at<BC>(u, i0 - 1 + a, n1, n2, cell_at<BC>(j0 - 2 + b, n2));
-    }
-    for (int k = t; k < (TI + 4) * VW; k += FUSED_THREADS) {
-        int a = k / VW, b = k % VW;
-        sv[k] = face_at<BC>(v + IX(cell_at<BC>(i0 - 2 + a, n1), 0, n2 + 1), j0 - 1 + b, n2, 1, 0);
-    }
-    __syncthreads();
-    // ---- XY path, X sweep: cells i in [i0-1, i0+TI], rows b in [0, CW) ----
-    for (int k = t; k < (TI + 2) * CW; k += FUSED_THREADS) {
-        int a = k / CW, b = k % CW;  // cell i = i0-1+a, c row index a+1
-        states<SCHEME>(sc[a * CW + b], sc[(a + 1) * CW + b], sc[(a + 2) * CW + b], su[a * CW + b], su[(a + 1) * CW + b],
-                       kx, hl[k], hr[k]);
-    }
-    __syncthreads();
-    for (int k = t; k < TI * CW; k += FUSED_THREADS) {
-        int a = k / CW, b = k % CW;  // cell i = i0+a: states at a+1, faces fi = i0+a (su row a+1), i0+a+1
-        double uw = su[(a + 1) * CW + b], ue = su[(a + 2) * CW + b];
-        double Fw = uw * (pos(uw) ? hr[a * CW + b] : hl[(a + 1) * CW + b]);
-        double Fe = ue * (pos(ue) ? hr[(a + 1) * CW + b] : hl[(a + 2) * CW + b]);
-        s1[k] = sc[(a + 2) * CW + b] + lx * (Fw - Fe);
+    using L = Tile<TI, MODE>;
+    constexpr int NT = L::THREADS, PL = L::PLANE, X1 = L::X1, Y1 = L::Y1, X2 = L::X2, Y2 = L::Y2;
+    constexpr bool XF = MODE == MODE_SYM || MODE == MODE_XY || MODE == MODE_X;  // a first sweep in x
+    constexpr bool YF = MODE == MODE_SYM || MODE == MODE_YX || MODE == MODE_Y;
+    constexpr bool HASX = MODE != MODE_Y, HASY = MODE != MODE_X;
+    extern __shared__ double adv_sm[];
+    double* sc = adv_sm;                  // c: rows i0-2 .., columns j0-2 ..; then X(c) over it
+    double* wx = sc + PL;                 // W of x-faces i0-1 .. (rows), columns as c
+    double* ex = wx + (HASX ? PL : 0);    // E of cells i0-1 .. (rows)
+    double* fx = ex + (HASX ? PL : 0);    // F of x-faces i0 .. at row f - i0 + 1 (as wx)
+    double* wy = fx + (HASX ? PL : 0);    // W of y-faces j0-1 .. (columns), rows as c
+    double* ey = wy + (HASY ? PL : 0);    // E of cells j0-1 .. (columns)
+    double* fy = ey + (HASY ? PL : 0);    // F of y-faces j0 .. at column f - j0 + 1 (as wy)
+    double* s1 = sc;                      // X(c): rows i0 .. at row i - i0 + 2, columns as c
+    double* s2 = MODE == MODE_SYM ? fy + PL : sc;  // Y(c): rows as c, columns j0 .. at column j - j0 + 2
+    const int n1 = A.n1, n2 = A.n2, t = threadIdx.x;
+    const int ti = blockIdx.y == 0 ? 0 : A.row0 + (int)blockIdx.y;
+    const int i0 = ti * TI, j0 = blockIdx.x * TJ;
+    const double dt = A.dt[0], lx = dt * A.fx, ly = dt * A.fy;
+    // ---- c and W (reflected or wrapped ghosts; tiles off the edges need none) ----
+    const bool inside = i0 >= 2 && j0 >= 2 && i0 + TI + 2 <= n1 && j0 + TJ + 2 <= n2;
+    for (int k = t; k < (TI + 4) * (TJ + 4); k += NT) {
+        const int a = k / (TJ + 4), b = k % (TJ + 4), i = i0 - 2 + a, j = j0 - 2 + b, o = a * TP + b;
+        if (inside) {
+            const size_t g = IX(i, j, n2);
+            sc[o] = A.cin[g];
+            if (HASX && a < TI + 3) wx[o] = lx * A.u[g + n2];                       // face i + 1
+            if (HASY && b < TJ + 3) wy[o] = ly * A.v[IX(i, j + 1, n2 + 1)];         // face j + 1
+        } else {
+            const int ic = cell_at<BC>(i, n1), jc = cell_at<BC>(j, n2);
+            const double* src = A.cghost && (i < 0 || i >= n1) ? A.cghost : A.cin;
+            sc[o] = src[IX(ic, jc, n2)];
+            if (HASX && a < TI + 3) wx[o] = lx * face_at<BC>(A.u, i + 1, n1, n2, jc);
+            if (HASY && b < TJ + 3) wy[o] = ly * face_at<BC>(A.v + IX(ic, 0, n2 + 1), j + 1, n2, 1, 0);
+        }
     }
     __syncthreads();
-    // ---- XY path, Y sweep on s1: cells j in [j0-1, j0+TJ], rows a in [0, TI) ----
-    for (int k = t; k < TI * (TJ + 2); k += FUSED_THREADS) {
-        int a = k / (TJ + 2), b = k % (TJ + 2);  // cell j = j0-1+b -> s1 col b+1; faces fj = j, j+1 -> sv col b, b+1
-        const double* row = s1 + a * CW;
-        const double* vr = sv + (a + 2) * VW;
-        states<SCHEME>(row[b], row[b + 1], row[b + 2], vr[b], vr[b + 1], ky, hl[k], hr[k]);
+    // ---- E and F ----
+    if (SCHEME == IMPEC_MUSCL) {
+        for (int k = t; k < (TI + 4) * (TJ + 4); k += NT) {
+            const int a = k / (TJ + 4), b = k % (TJ + 4), o = a * TP + b;
+            if (HASX && a < TI + 2) {  // cell i0-1+a between wx rows a, a+1; the face above it is wx row a+1
+                const double w = wx[o], e = wx[o + TP];
+                ex[o] = fma(0.5, w - e, 1.0);
+                if (a < TI + 1) {
+                    const bool p = pos(e);  // operands are selected, not results: one sum, one multiply-add
+                    fx[o + TP] = fma(-0.25, e + (p ? w : wx[o + 2 * TP]), p ? 0.5 : -0.5);
+                }
+            }
+            if (HASY && b < TJ + 2) {
+                const double w = wy[o], e = wy[o + 1];
+                ey[o] = fma(0.5, w - e, 1.0);
+                if (b < TJ + 1) {
+                    const bool p = pos(e);
+                    fy[o + 1] = fma(-0.25, e + (p ? w : wy[o + 2]), p ? 0.5 : -0.5);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    // ---- first sweeps: X(c) on all columns, Y(c) on all rows; the results wait in registers
+    // until every strip has read c, which X(c) then replaces ----
+    double r[STRIP];
+    const bool xs = XF && t < X1, ys = YF && t >= (XF ? X1 : 0) && t < (XF ? X1 : 0) + Y1;
+    const int q = XF ? t - X1 : t;
+    const int xb = t % (TJ + 4), xm = STRIP * (t / (TJ + 4)), ya = q % (TI + 4), ym = STRIP * (q / (TI + 4));
+    if (xs)
+        sweep_strip<SCHEME>(sc + (xm + 2) * TP + xb, TP, wx + (xm + 1) * TP + xb, ex + (xm + 1) * TP + xb,
+                            fx + (xm + 1) * TP + xb, TP, r);
+    if (ys)
+        sweep_strip<SCHEME>(sc + ya * TP + ym + 2, 1, wy + ya * TP + ym + 1, ey + ya * TP + ym + 1, fy + ya * TP + ym + 1, 1,
+                            r);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < STRIP; ++k) {
+        if (xs) s1[(xm + 2 + k) * TP + xb] = r[k];
+        if (ys) s2[ya * TP + ym + 2 + k] = r[k];
     }
     __syncthreads();
-    for (int k = t; k < TI * TJ; k += FUSED_THREADS) {
-        int a = k / TJ, b = k % TJ;  // cell j = j0+b: states index b+1
-        const double* vr = sv + (a + 2) * VW;
-        const int h = a * (TJ + 2);
-        double vs = vr[b + 1], vn = vr[b + 2];
-        double Fs = vs * (pos(vs) ? hr[h + b] : hl[h + b + 1]);
-        double Fn = vn * (pos(vn) ? hr[h + b + 1] : hl[h + b + 2]);
-        sxy[k] = s1[a * CW + b + 2] + ly * (Fs - Fn);
+    // ---- second sweeps: Y on X(c) and X on Y(c) ----
+    const int p = MODE == MODE_SYM ? t - Y2 : t;
+    const bool y2 = (MODE == MODE_SYM || MODE == MODE_XY) && t < Y2, x2 = (MODE == MODE_SYM || MODE == MODE_YX) && p >= 0 && p < X2;
+    const int ay = 2 + t % TI, my = STRIP * (t / TI), bx = 2 + p % TJ, mx = STRIP * (p / TJ);
+    if (y2)
+        sweep_strip<SCHEME>(s1 + ay * TP + my + 2, 1, wy + ay * TP + my + 1, ey + ay * TP + my + 1, fy + ay * TP + my + 1, 1,
+                            r);
+    if (x2)
+        sweep_strip<SCHEME>(s2 + (mx + 2) * TP + bx, TP, wx + (mx + 1) * TP + bx, ex + (mx + 1) * TP + bx,
+                            fx + (mx + 1) * TP + bx, TP, r);
+    if (MODE == MODE_SYM || MODE == MODE_XY || MODE == MODE_YX) __syncthreads();
+    if (MODE == MODE_SYM) {  // the threads that hold X(Y(c)) average and write: one column each
+        if (y2) {
+#pragma unroll
+            for (int k = 0; k < STRIP; ++k) s1[ay * TP + my + 2 + k] = r[k];
+        }
+        __syncthreads();
+        if (x2) {
+            const int j = j0 + bx - 2;
+#pragma unroll
+            for (int k = 0; k < STRIP; ++k) {
+                const int i = i0 + mx + k;
+                if (i < n1 && j < n2) A.cout[IX(i, j, n2)] = 0.5 * (s1[(mx + 2 + k) * TP + bx] + r[k]);
+            }
+        }
+        return;
     }
-    __syncthreads();
-    // ---- YX path, Y sweep on c: rows a in [0, TI+4) (i = i0-2+a), cells j in [j0-1, j0+TJ] ----
-    for (int k = t; k < (TI + 4) * (TJ + 2); k += FUSED_THREADS) {
-        int a = k / (TJ + 2), b = k % (TJ + 2);
-        const double* row = sc + a * CW;
-        const double* vr = sv + a * VW;
-        states<SCHEME>(row[b], row[b + 1], row[b + 2], vr[b], vr[b + 1], ky, hl[k], hr[k]);
+    if (MODE == MODE_XY || MODE == MODE_YX) {
+#pragma unroll
+        for (int k = 0; k < STRIP; ++k) {
+            if (y2) sc[ay * TP + my + 2 + k] = r[k];
+            if (x2) sc[(mx + 2 + k) * TP + bx] = r[k];
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    for (int k = t; k < (TI + 4) * TJ; k += FUSED_THREADS) {
-        int a = k / TJ, b = k % TJ;
-        const double* vr = sv + a * VW;
-        const int h = a * (TJ + 2);
-        double vs = vr[b + 1], vn = vr[b + 2];
-        double Fs = vs * (pos(vs) ? hr[h + b] : hl[h + b + 1]);
-        double Fn = vn * (pos(vn) ? hr[h + b + 1] : hl[h + b + 2]);
-        s2[k] = sc[a * CW + b + 2] + ly * (Fs - Fn);
+    for (int k = t; k < TI * TJ; k += NT) {
+        const int a = k / TJ, b = k % TJ, i = i0 + a, j = j0 + b;
+        if (i < n1 && j < n2) A.cout[IX(i, j, n2)] = sc[(a + 2) * TP + b + 2];
     }
-    __syncthreads();
-    // ---- YX path, X sweep on s2: cells i in [i0-1, i0+TI] (s2 rows a+1), cols b in [0, TJ) ----
-    for (int k = t; k < (TI + 2) * TJ; k += FUSED_THREADS) {
-        int a = k / TJ, b = k % TJ;
-        states<SCHEME>(s2[a * TJ + b], s2[(a + 1) * TJ + b], s2[(a + 2) * TJ + b], su[a * CW + b + 2],
-                       su[(a + 1) * CW + b + 2], kx, hl[k], hr[k]);
+}
+
+// Launches one tile kernel.  Its shared memory is above the default limit, which each device has
+// to be told once per kernel (a set attribute stays; setting it again does no harm).
+template <int SCHEME, int BC, int MODE, int TI>
+static cudaError_t launch_tile(cudaStream_t s, TileArgs A, bool edges) {
+    int rows = (A.n1 + TI - 1) / TI;
+    if (edges && rows > 3) {  // tile rows 0, rows - 2, rows - 1 (the last may hold one row only)
+        A.row0 = rows - 3;
+        rows = 3;
     }
-    __syncthreads();
-    for (int k = t; k < TI * TJ; k += FUSED_THREADS) {
-        int a = k / TJ, b = k % TJ;
-        const int gi = i0 + a, gj = j0 + b;
-        if (gi >= n1 || gj >= n2) continue;
-        double uw = su[(a + 1) * CW + b + 2], ue = su[(a + 2) * CW + b + 2];
-        double Fw = uw * (pos(uw) ? hr[a * TJ + b] : hl[(a + 1) * TJ + b]);
-        double Fe = ue * (pos(ue) ? hr[(a + 1) * TJ + b] : hl[(a + 2) * TJ + b]);
-        double yx = s2[(a + 2) * TJ + b] + lx * (Fw - Fe);
-        cout[IX(gi, gj, n2)] = 0.5 * (sxy[k] + yx);
+    static std::mutex mu;
+    static unsigned long long done = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev >= 64 || !(done >> dev & 1)) {
+            e = cudaFuncSetAttribute(k_advect_tile<SCHEME, BC, MODE, TI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)Tile<TI, MODE>::SMEM);
+            if (e != cudaSuccess) return e;
+            if (dev < 64) done |= 1ull << dev;
+        }
     }
+    const dim3 g((A.n2 + TJ - 1) / TJ, rows);
+    return launch_k(s, k_advect_tile<SCHEME, BC, MODE, TI>, g, Tile<TI, MODE>::THREADS, Tile<TI, MODE>::SMEM, A);
+}
+
+template <int SCHEME, int MODE>
+static cudaError_t launch_tile_bc(int bc, cudaStream_t s, const TileArgs& A, bool edges) {
+    // tiles of 8 rows where those of 32 would leave SMs without one (symmetric MUSCL, a call: 256^2 29
+    // against 33 us, 400 x 300 36 against 34: more of the first sweeps is halo)
+    const bool small = (size_t)A.n1 * A.n2 < 98304;
+    if (bc == IMPEC_BC_PERIODIC)
+        return small ? launch_tile<SCHEME, IMPEC_BC_PERIODIC, MODE, 8>(s, A, edges)
+                     : launch_tile<SCHEME, IMPEC_BC_PERIODIC, MODE, 32>(s, A, edges);
+    return small ? launch_tile<SCHEME, IMPEC_BC_NEUMANN, MODE, 8>(s, A, edges)
+                 : launch_tile<SCHEME, IMPEC_BC_NEUMANN, MODE, 32>(s, A, edges);
+}
+
+// hmtype: IMPEC_MUSCL, IMPEC_WAFSPLIT / IMPEC_WAF, else upwind.  edges: only the tile rows that
+// hold the two rows next to each x end.
+template <int MODE>
+static cudaError_t launch_tiles(int hmtype, int bc, cudaStream_t s, const TileArgs& A, bool edges = false) {
+    if (hmtype == IMPEC_MUSCL) return launch_tile_bc<IMPEC_MUSCL, MODE>(bc, s, A, edges);
+    if (hmtype == IMPEC_WAFSPLIT || hmtype == IMPEC_WAF) return launch_tile_bc<IMPEC_WAFSPLIT, MODE>(bc, s, A, edges);
+    return launch_tile_bc<IMPEC_UPWINDSPLIT, MODE>(bc, s, A, edges);
 }
 
 // ---------------------------------------------------------------- corner transport upwind
@@ -362,53 +508,63 @@ __global__ void k_ctu(int n1, int n2, const double* __restrict__ cin, double* __
 
 static dim3 tgrid(int n1, int n2) { return dim3((n2 + TBX - 1) / TBX, (n1 + TBY - 1) / TBY); }
 
-impec_status advect_x_dev(impec_ctx* ctx, const double* cin, double* cout, const double* u, double dt_scale,
-                          const double* dt_dev, const double* cghost) {
+// One launch of a tile mode on the context's grid; x and y sweeps over x_scale dt and y_scale dt.
+template <int MODE>
+static impec_status advect_tiles(impec_ctx* ctx, const double* cin, double* cout, const double* u, const double* v,
+                                 double x_scale, double y_scale, const double* dt_dev, const double* cghost = nullptr,
+                                 bool edges = false) {
     const impec_params& P = ctx->P;
-    const double f = 1.0 / (ctx->G.dx * P.porosity);
-    dim3 g = tgrid(P.N1, P.N2), b(TBX, TBY);
+    const TileArgs A{P.N1, P.N2, cin, cghost, cout, u, v, dt_dev, x_scale / (ctx->G.dx * P.porosity),
+                     y_scale / (ctx->G.dy * P.porosity), 0};
     ++ctx->nlaunch;
-    const bool per = P.bc == IMPEC_BC_PERIODIC;
-    if (P.hmtype == IMPEC_MUSCL) {
-        if (per) launch_k(ctx->stream, k_sweep_x<IMPEC_MUSCL, IMPEC_BC_PERIODIC>, g, b, 0, P.N1, P.N2, cin, cghost, cout, u, dt_dev, dt_scale, f);
-        else launch_k(ctx->stream, k_sweep_x<IMPEC_MUSCL, IMPEC_BC_NEUMANN>, g, b, 0, P.N1, P.N2, cin, cghost, cout, u, dt_dev, dt_scale, f);
-    } else if (P.hmtype == IMPEC_WAFSPLIT || P.hmtype == IMPEC_WAF) {
-        if (per) launch_k(ctx->stream, k_sweep_x<IMPEC_WAFSPLIT, IMPEC_BC_PERIODIC>, g, b, 0, P.N1, P.N2, cin, cghost, cout, u, dt_dev, dt_scale, f);
-        else launch_k(ctx->stream, k_sweep_x<IMPEC_WAFSPLIT, IMPEC_BC_NEUMANN>, g, b, 0, P.N1, P.N2, cin, cghost, cout, u, dt_dev, dt_scale, f);
-    } else {
-        if (per) launch_k(ctx->stream, k_sweep_x<IMPEC_UPWINDSPLIT, IMPEC_BC_PERIODIC>, g, b, 0, P.N1, P.N2, cin, cghost, cout, u, dt_dev, dt_scale, f);
-        else launch_k(ctx->stream, k_sweep_x<IMPEC_UPWINDSPLIT, IMPEC_BC_NEUMANN>, g, b, 0, P.N1, P.N2, cin, cghost, cout, u, dt_dev, dt_scale, f);
-    }
-    IMPEC_LAUNCH_CHECK();
+    IMPEC_CUDA_TRY(launch_tiles<MODE>(P.hmtype, P.bc, ctx->stream, A, edges));
     return IMPEC_OK;
+}
+
+// The cell-by-cell sweeps.
+static impec_status sweep_cells(impec_ctx* ctx, bool x, const double* cin, double* cout, const double* vel, double dt_scale,
+                                const double* dt_dev, const double* cghost = nullptr) {
+    const impec_params& P = ctx->P;
+    const dim3 g = tgrid(P.N1, P.N2), b(TBX, TBY);
+    const double f = 1.0 / ((x ? ctx->G.dx : ctx->G.dy) * P.porosity);
+    auto go = [&](auto kx, auto ky) {
+        return x ? launch_k(ctx->stream, kx, g, b, 0, P.N1, P.N2, cin, cghost, cout, vel, dt_dev, dt_scale, f)
+                 : launch_k(ctx->stream, ky, g, b, 0, P.N1, P.N2, cin, cout, vel, dt_dev, dt_scale, f);
+    };
+    const bool per = P.bc == IMPEC_BC_PERIODIC;
+    ++ctx->nlaunch;
+#define IMPEC_SWEEP(S)                                                                                       \
+    (per ? go(k_sweep_x<S, IMPEC_BC_PERIODIC>, k_sweep_y<S, IMPEC_BC_PERIODIC>)                              \
+         : go(k_sweep_x<S, IMPEC_BC_NEUMANN>, k_sweep_y<S, IMPEC_BC_NEUMANN>))
+    if (P.hmtype == IMPEC_MUSCL) IMPEC_CUDA_TRY(IMPEC_SWEEP(IMPEC_MUSCL));
+    else if (P.hmtype == IMPEC_WAFSPLIT || P.hmtype == IMPEC_WAF) IMPEC_CUDA_TRY(IMPEC_SWEEP(IMPEC_WAFSPLIT));
+    else IMPEC_CUDA_TRY(IMPEC_SWEEP(IMPEC_UPWINDSPLIT));
+#undef IMPEC_SWEEP
+    return IMPEC_OK;
+}
+
+// Whether sweeps in a row run cell by cell (microseconds a call, cells / tiles): below 2^16 cells
+// tiles do not fill the GPU and their phases take longer than two short launches (180^2, X then Y:
+// 22 / 27; Strang 35 / 41; 256^2: 27 / 27, 43 / 42; 512^2: 48 / 38, 82 / 58).  Upwind sweeps have so
+// little to compute that the tile's copy back costs more than the second launch up to 2^20 cells
+// (512^2: 24 / 26; 1024^2: 42 / 39), in Strang's three tile launches up to 2^18 (360^2: 33 / 34;
+// 512^2: 37 / 36).
+static bool by_cells(const impec_params& P) {
+    const size_t n = (size_t)P.N1 * P.N2;
+    const bool upwind = P.hmtype != IMPEC_MUSCL && P.hmtype != IMPEC_WAFSPLIT && P.hmtype != IMPEC_WAF;
+    return n < (size_t)1 << (!upwind ? 16 : P.dim_splitting == IMPEC_STRANG ? 18 : 20);
+}
+
+impec_status advect_x_dev(impec_ctx* ctx, const double* cin, double* cout, const double* u, double dt_scale,
+                          const double* dt_dev) {
+    if (by_cells(ctx->P)) return sweep_cells(ctx, true, cin, cout, u, dt_scale, dt_dev);
+    return advect_tiles<MODE_X>(ctx, cin, cout, u, nullptr, dt_scale, 0.0, dt_dev);
 }
 
 impec_status advect_y_dev(impec_ctx* ctx, const double* cin, double* cout, const double* v, double dt_scale,
                           const double* dt_dev) {
-    const impec_params& P = ctx->P;
-    const double f = 1.0 / (ctx->G.dy * P.porosity);
-    dim3 g = tgrid(P.N1, P.N2), b(TBX, TBY);
-    ++ctx->nlaunch;
-    const bool per = P.bc == IMPEC_BC_PERIODIC;
-    if (P.hmtype == IMPEC_MUSCL) {
-        if (per) launch_k(ctx->stream, k_sweep_y<IMPEC_MUSCL, IMPEC_BC_PERIODIC>, g, b, 0, P.N1, P.N2, cin, cout, v, dt_dev, dt_scale, f);
-        else launch_k(ctx->stream, k_sweep_y<IMPEC_MUSCL, IMPEC_BC_NEUMANN>, g, b, 0, P.N1, P.N2, cin, cout, v, dt_dev, dt_scale, f);
-    } else if (P.hmtype == IMPEC_WAFSPLIT || P.hmtype == IMPEC_WAF) {
-        if (per) launch_k(ctx->stream, k_sweep_y<IMPEC_WAFSPLIT, IMPEC_BC_PERIODIC>, g, b, 0, P.N1, P.N2, cin, cout, v, dt_dev, dt_scale, f);
-        else launch_k(ctx->stream, k_sweep_y<IMPEC_WAFSPLIT, IMPEC_BC_NEUMANN>, g, b, 0, P.N1, P.N2, cin, cout, v, dt_dev, dt_scale, f);
-    } else {
-        if (per) launch_k(ctx->stream, k_sweep_y<IMPEC_UPWINDSPLIT, IMPEC_BC_PERIODIC>, g, b, 0, P.N1, P.N2, cin, cout, v, dt_dev, dt_scale, f);
-        else launch_k(ctx->stream, k_sweep_y<IMPEC_UPWINDSPLIT, IMPEC_BC_NEUMANN>, g, b, 0, P.N1, P.N2, cin, cout, v, dt_dev, dt_scale, f);
-    }
-    IMPEC_LAUNCH_CHECK();
-    return IMPEC_OK;
-}
-
-impec_status average_dev(impec_ctx* ctx, double* c, const double* a, const double* b) {
-    const size_t n = (size_t)ctx->P.N1 * ctx->P.N2;
-    ++ctx->nlaunch, launch_k(ctx->stream, k_average, ctx->num_sms * 4, 256, 0, n, c, a, b);
-    IMPEC_LAUNCH_CHECK();
-    return IMPEC_OK;
+    if (by_cells(ctx->P)) return sweep_cells(ctx, false, cin, cout, v, dt_scale, dt_dev);
+    return advect_tiles<MODE_Y>(ctx, cin, cout, nullptr, v, 0.0, dt_scale, dt_dev);
 }
 
 // AdvectSplit (src/HyperbolicSplitSolver.cpp:51-106); pfs 0 = X_SWEEP, 1 = Y_SWEEP.
@@ -426,67 +582,45 @@ impec_status advect_split_dev(impec_ctx* ctx, double* c, const double* u, const 
         IMPEC_CUDA_TRY(cudaMemcpyAsync(c, t1, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
         return IMPEC_OK;  // unsplit: the alternating-sweep state stays as it was
     }
-    if (P.dim_splitting == IMPEC_SYMMETRIC_PARALLEL && (P.hmtype == IMPEC_WAFSPLIT || P.hmtype == IMPEC_WAF)) {
-        // the average of XY and YX through the per-sweep kernels (the fused tile kernel has
-        // MUSCL and upwind states only): t2 = Y(X(c)), t1 = X(Y(c)), c = (t2 + t1) / 2
-        IMPEC_TRY(advect_x_dev(ctx, c, t1, u, 1.0, dt_dev));
-        IMPEC_TRY(advect_y_dev(ctx, t1, t2, v, 1.0, dt_dev));
-        IMPEC_TRY(advect_y_dev(ctx, c, t3, v, 1.0, dt_dev));
-        IMPEC_TRY(advect_x_dev(ctx, t3, t1, u, 1.0, dt_dev));
-        IMPEC_TRY(average_dev(ctx, c, t2, t1));
-        *pfs = 0;
-        return IMPEC_OK;
-    }
+    // one tile launch per update, c -> t1 (neighbouring tiles read the old c), then back into c
+    bool x_first = true;
     switch (P.dim_splitting) {
-        case IMPEC_ALTERNATING:
-            if (*pfs == 1) {
-                IMPEC_TRY(advect_x_dev(ctx, c, t1, u, 1.0, dt_dev));
-                IMPEC_TRY(advect_y_dev(ctx, t1, c, v, 1.0, dt_dev));
-                *pfs = 0;
-            } else {
-                IMPEC_TRY(advect_y_dev(ctx, c, t1, v, 1.0, dt_dev));
-                IMPEC_TRY(advect_x_dev(ctx, t1, c, u, 1.0, dt_dev));
-                *pfs = 1;
-            }
-            break;
-        case IMPEC_X_FIRST:
-            IMPEC_TRY(advect_x_dev(ctx, c, t1, u, 1.0, dt_dev));
-            IMPEC_TRY(advect_y_dev(ctx, t1, c, v, 1.0, dt_dev));
-            *pfs = 0;
-            break;
-        case IMPEC_Y_FIRST:
-            IMPEC_TRY(advect_y_dev(ctx, c, t1, v, 1.0, dt_dev));
-            IMPEC_TRY(advect_x_dev(ctx, t1, c, u, 1.0, dt_dev));
-            *pfs = 1;
-            break;
+        case IMPEC_ALTERNATING: x_first = *pfs == 1; break;
+        case IMPEC_X_FIRST: break;
+        case IMPEC_Y_FIRST: x_first = false; break;
         case IMPEC_STRANG:
             // Advect_X leaves the ghost columns i < 0, i >= N1 untouched, so after X(dt/2), Y(dt)
             // they hold Y(dt) applied to the mirrored input, not mirrors of the new interior; the
             // last X(dt/2) reads them there (src/HyperbolicSplitSolver.cpp:80-85, :128-131, :152-155).
-            IMPEC_TRY(advect_y_dev(ctx, c, t3, v, 1.0, dt_dev));
-            IMPEC_TRY(advect_x_dev(ctx, c, t1, u, 0.5, dt_dev));
-            IMPEC_TRY(advect_y_dev(ctx, t1, t2, v, 1.0, dt_dev));
-            IMPEC_TRY(advect_x_dev(ctx, t2, c, u, 0.5, dt_dev, t3));
-            *pfs = 0;
-            break;
-        default: {  // SYMMETRIC_PARALLEL: one fused pass, c -> t1, then swap into c
-            const double fx = 1.0 / (ctx->G.dx * P.porosity), fy = 1.0 / (ctx->G.dy * P.porosity);
-            dim3 g((P.N2 + TJ - 1) / TJ, (P.N1 + TI - 1) / TI);
-            const bool per = P.bc == IMPEC_BC_PERIODIC;
-            ++ctx->nlaunch;
-            if (P.hmtype == IMPEC_MUSCL) {
-                if (per) launch_k(ctx->stream, k_advect_symmetric<IMPEC_MUSCL, IMPEC_BC_PERIODIC>, g, FUSED_THREADS, 0, P.N1, P.N2, c, t1, u, v, dt_dev, fx, fy);
-                else launch_k(ctx->stream, k_advect_symmetric<IMPEC_MUSCL, IMPEC_BC_NEUMANN>, g, FUSED_THREADS, 0, P.N1, P.N2, c, t1, u, v, dt_dev, fx, fy);
-            } else {
-                if (per) launch_k(ctx->stream, k_advect_symmetric<IMPEC_UPWINDSPLIT, IMPEC_BC_PERIODIC>, g, FUSED_THREADS, 0, P.N1, P.N2, c, t1, u, v, dt_dev, fx, fy);
-                else launch_k(ctx->stream, k_advect_symmetric<IMPEC_UPWINDSPLIT, IMPEC_BC_NEUMANN>, g, FUSED_THREADS, 0, P.N1, P.N2, c, t1, u, v, dt_dev, fx, fy);
+            // Only the two rows next to each end are ever read, so with tiles Y(dt) of the input runs
+            // there only.
+            if (by_cells(P)) {
+                IMPEC_TRY(sweep_cells(ctx, false, c, t3, v, 1.0, dt_dev));
+                IMPEC_TRY(sweep_cells(ctx, true, c, t1, u, 0.5, dt_dev));
+                IMPEC_TRY(sweep_cells(ctx, false, t1, t2, v, 1.0, dt_dev));
+                IMPEC_TRY(sweep_cells(ctx, true, t2, c, u, 0.5, dt_dev, t3));
+                *pfs = 0;
+                return IMPEC_OK;
             }
-            IMPEC_LAUNCH_CHECK();
+            IMPEC_TRY(advect_tiles<MODE_Y>(ctx, c, t3, nullptr, v, 0.0, 1.0, dt_dev, nullptr, true));
+            IMPEC_TRY(advect_tiles<MODE_XY>(ctx, c, t2, u, v, 0.5, 1.0, dt_dev));
+            IMPEC_TRY(advect_tiles<MODE_X>(ctx, t2, c, u, nullptr, 0.5, 0.0, dt_dev, t3));
+            *pfs = 0;
+            return IMPEC_OK;
+        default:
+            IMPEC_TRY(advect_tiles<MODE_SYM>(ctx, c, t1, u, v, 1.0, 1.0, dt_dev));
             IMPEC_CUDA_TRY(cudaMemcpyAsync(c, t1, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
             *pfs = 0;
-        }
+            return IMPEC_OK;
     }
-    (void)bytes;
+    *pfs = x_first ? 0 : 1;
+    if (by_cells(P)) {  // two launches through t1, no copy
+        IMPEC_TRY(sweep_cells(ctx, x_first, c, t1, x_first ? u : v, 1.0, dt_dev));
+        return sweep_cells(ctx, !x_first, t1, c, x_first ? v : u, 1.0, dt_dev);
+    }
+    IMPEC_TRY(x_first ? advect_tiles<MODE_XY>(ctx, c, t1, u, v, 1.0, 1.0, dt_dev)
+                      : advect_tiles<MODE_YX>(ctx, c, t1, u, v, 1.0, 1.0, dt_dev));
+    IMPEC_CUDA_TRY(cudaMemcpyAsync(c, t1, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     return IMPEC_OK;
 }
 
@@ -563,15 +697,8 @@ extern "C" impec_status impec_advect_symmetric_noalloc(const impec_params* P, do
     const double fx = 1.0 / (dx * P->porosity), fy = 1.0 / (dy * P->porosity);
     double* cnew = scratch + NOALLOC_FIELD_OFFSET;
     launch_k(s, k_noalloc_store_dt, 1, 1, 0, scratch, dt);
-    dim3 g((N2 + TJ - 1) / TJ, (N1 + TI - 1) / TI);
-    const bool per = P->bc == IMPEC_BC_PERIODIC;
-    if (P->hmtype == IMPEC_MUSCL) {
-        if (per) launch_k(s, k_advect_symmetric<IMPEC_MUSCL, IMPEC_BC_PERIODIC>, g, FUSED_THREADS, 0, N1, N2, c_dev, cnew, u_dev, v_dev, scratch, fx, fy);
-        else launch_k(s, k_advect_symmetric<IMPEC_MUSCL, IMPEC_BC_NEUMANN>, g, FUSED_THREADS, 0, N1, N2, c_dev, cnew, u_dev, v_dev, scratch, fx, fy);
-    } else {
-        if (per) launch_k(s, k_advect_symmetric<IMPEC_UPWINDSPLIT, IMPEC_BC_PERIODIC>, g, FUSED_THREADS, 0, N1, N2, c_dev, cnew, u_dev, v_dev, scratch, fx, fy);
-        else launch_k(s, k_advect_symmetric<IMPEC_UPWINDSPLIT, IMPEC_BC_NEUMANN>, g, FUSED_THREADS, 0, N1, N2, c_dev, cnew, u_dev, v_dev, scratch, fx, fy);
-    }
+    const TileArgs A{N1, N2, c_dev, nullptr, cnew, u_dev, v_dev, scratch, fx, fy, 0};
+    IMPEC_CUDA_TRY(launch_tiles<MODE_SYM>(P->hmtype, P->bc, s, A));
     IMPEC_LAUNCH_CHECK();
     IMPEC_CUDA_TRY(cudaMemcpyAsync(c_dev, cnew, (size_t)N1 * N2 * sizeof(double), cudaMemcpyDeviceToDevice, s));
     return IMPEC_OK;

@@ -84,3 +84,34 @@ def test_cg_settles_at_its_floor(engine, oracle_lib, N1, N2, nu, prec):
     oracle_lib.or_pressure_rhs(C.byref(OP), O.ptr(q), O.ptr(b))
     rr_or = oracle_lib.or_relres9(C.byref(OP), O.ptr(A), O.ptr(host(p).ravel().copy()), O.ptr(b))
     assert rr <= 1e-11 and rr_or <= 1e-11, (rr, rr_or)
+
+
+@pytest.mark.parametrize("N1,N2", [(2, 2), (3, 33), (32, 32), (33, 31), (64, 34), (35, 97), (130, 36), (97, 161)])
+@pytest.mark.parametrize("scheme", [4, 0, 1])  # MUSCL, upwind, WAF split
+@pytest.mark.parametrize("mode", [4, 0, 1, 2, 3])
+def test_sweep_tiles(engine, oracle_lib, N1, N2, scheme, mode):
+    """The split sweeps at the edges of their 32 x 32 tiles (one cell over, one short, a last tile of
+    one row, grids smaller than a halo) in every splitting, against the oracle.  A value is a
+    sum of about 20 rounded terms of size <= 1 in either formulation: 1e-13."""
+    import ctypes as C
+
+    import oracle as O
+    from helpers import cell_ghost, dev, host, rel_err, smooth_field, vel_split
+    E = engine
+    P = E.default_params(N1, N2, hmtype=scheme, dim_splitting=mode, porosity=0.7)
+    OP = oparams(P)
+    rng = np.random.default_rng(5)
+    p = smooth_field(N1, N2, 9, -1.0, 1.0) * 0.05
+    v = np.zeros(O.vel_shape(OP))
+    c = rng.uniform(0.0, 1.0, (N1, N2))
+    cg = cell_ghost(OP, c)
+    oracle_lib.or_calc_velocities(C.byref(OP), O.ptr(cell_ghost(OP, p)), O.ptr(v), O.ptr(cg))
+    u, vv = vel_split(OP, v)
+    dt = 0.8 * oracle_lib.or_max_stable_advection_dt(C.byref(OP), O.ptr(v)) * OP.porosity
+    pfs = C.c_int(1)
+    oracle_lib.or_advect_split(C.byref(OP), O.ptr(cg), O.ptr(v), dt, C.byref(pfs))
+    ctx = E.Context(P)
+    d = dev(c)
+    assert ctx.advect_split(d, dev(u), dev(vv), dt, 1) == pfs.value
+    assert rel_err(host(d), O.interior(OP, cg)) <= 1e-13
+    ctx.close()
