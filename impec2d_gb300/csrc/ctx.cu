@@ -183,7 +183,6 @@ impec_status impec_ctx_create(const impec_params* P, void* stream, impec_ctx** o
     ALLOC(ctx->muK11, n * 8);
     ALLOC(ctx->lamx, nu * 8); ALLOC(ctx->lamy, nv * 8);
     ALLOC(ctx->f, n * 8); ALLOC(ctx->r, n * 8);
-    ALLOC(ctx->dfx, nu * 2 * 8); ALLOC(ctx->dfy, nv * 2 * 8);
     ALLOC(ctx->cn_a9, n * 9 * 8); ALLOC(ctx->cn_b, n * 8); ALLOC(ctx->cn_idiag, n * 8);
     ctx->max_blocks = 4096;
     ALLOC(ctx->partials, (size_t)8 * ctx->max_blocks * 8);
@@ -229,7 +228,7 @@ impec_status impec_ctx_destroy(impec_ctx* ctx) {
     pressure_free(ctx);
     double* bufs[] = {ctx->c, ctx->p, ctx->q, ctx->u, ctx->v, ctx->t1, ctx->t2, ctx->t3, ctx->muK11,
                       ctx->muK22 == ctx->muK11 ? nullptr : ctx->muK22, ctx->lamx, ctx->lamy, ctx->f, ctx->r,
-                      ctx->dfx, ctx->dfy, ctx->cn_a9, ctx->cn_b, ctx->cn_idiag, ctx->partials, ctx->K11,
+                      ctx->cn_a9, ctx->cn_b, ctx->cn_idiag, ctx->partials, ctx->K11,
                       ctx->K22, ctx->well_q};
     for (double* b : bufs)
         if (b) cudaFree(b);

@@ -86,18 +86,18 @@ static impec_status capture_while(impec_ctx* ctx, Init init, Body body, long lon
     return IMPEC_OK;
 }
 
-static impec_status capture_cn_solve(impec_ctx* ctx, double* c) {
+impec_status capture_cn_solve(impec_ctx* ctx, const double* c, double* x) {
     const double tol = ctx->P.para_eps;
-    IMPEC_TRY(cn_prepare(ctx, c, 0.5, &ctx->dscal->dt, false));
+    IMPEC_TRY(cn_prepare(ctx, c, x));
     long long nb = 0;
     IMPEC_TRY(capture_while(
         ctx,
         [&](cudaGraphConditionalHandle h) {  // the first sweep runs before the first check (as dispersion_cn_dev)
-            IMPEC_TRY(cn_iteration(ctx, c));
+            IMPEC_TRY(cn_iteration(ctx, x));
             return cn_check(ctx, tol, 1, h, 1);
         },
         [&](cudaGraphConditionalHandle h) {
-            IMPEC_TRY(cn_iteration(ctx, c));
+            IMPEC_TRY(cn_iteration(ctx, x));
             return cn_check(ctx, tol, 1, h, 1);
         },
         nb));
@@ -131,15 +131,8 @@ static impec_status capture_step_into(impec_ctx* ctx, int pfs_in) {
         ++ctx->nlaunch;
         launch_k(ctx->stream, k_clip_dt, 1, 1, 0, S);
         // HyperbolicSplitSolver::Solve (src/HyperbolicSplitSolver.cpp:162-198)
-        IMPEC_TRY(tr_integrate_dev(ctx, ctx->c, 0.5, dt, 0));
-        if (P.diffusion) {
-            IMPEC_TRY(cn_setup(ctx, ctx->u, ctx->v, 0.5, dt));
-            IMPEC_TRY(capture_cn_solve(ctx, ctx->c));
-        }
         int pfs = pfs_in;
-        IMPEC_TRY(advect_split_dev(ctx, ctx->c, ctx->u, ctx->v, dt, &pfs));
-        IMPEC_TRY(tr_integrate_dev(ctx, ctx->c, 0.5, dt, 1));
-        if (P.diffusion) IMPEC_TRY(capture_cn_solve(ctx, ctx->c));
+        IMPEC_TRY(hyperbolic_capture(ctx, ctx->c, ctx->u, ctx->v, dt, &pfs));
         ++ctx->nlaunch;
         const long long loops = mg_body + (P.diffusion ? 2 * ctx->step_cn_body_launches : 0);
         launch_k(ctx->stream, k_advance, 1, 1, 0, S, ctx->nlaunch - n0 - loops, mg_body,

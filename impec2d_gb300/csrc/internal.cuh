@@ -207,7 +207,6 @@ struct impec_ctx {
     int* well_idx = nullptr;
     double* well_q = nullptr;
     // dispersion
-    double *dfx = nullptr, *dfy = nullptr;        // Peaceman tensors at x-faces (d11,d12) and y-faces (d22,d21)
     double *cn_a9 = nullptr, *cn_b = nullptr, *cn_idiag = nullptr;
     // reductions
     double* partials = nullptr;                   // [8][max_blocks]
@@ -260,12 +259,13 @@ impec_status tr_integrate_dev(impec_ctx* ctx, double* c, double dt_scale, const 
 impec_status advect_x_dev(impec_ctx* ctx, const double* cin, double* cout, const double* u, double dt_scale,
                           const double* dt_dev);
 impec_status advect_y_dev(impec_ctx* ctx, const double* cin, double* cout, const double* v, double dt_scale, const double* dt_dev);
-impec_status advect_split_dev(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev, int* pfs);
+impec_status advect_split_dev(impec_ctx* ctx, double* cin, double* cout, double* s1, double* s2, double* s3, const double* u,
+                              const double* v, const double* dt_dev, int* pfs);
 // dispersion.cu
 impec_status cn_setup(impec_ctx* ctx, const double* u, const double* v, double dt_scale, const double* dt_dev);
-impec_status cn_prepare(impec_ctx* ctx, double* c, double dt_scale, const double* dt_dev, bool residual = true);
+impec_status cn_prepare(impec_ctx* ctx, const double* c, double* x);
 impec_status cn_check(impec_ctx* ctx, double tol, int inc, cudaGraphConditionalHandle h, int use_h);
-impec_status cn_iteration(impec_ctx* ctx, double* c);
+impec_status cn_iteration(impec_ctx* ctx, double* x);
 impec_status dispersion_cn_dev(impec_ctx* ctx, double* c, const double* u, const double* v, double dt_scale,
                                const double* dt_dev, double tol, int* its, double* relres);
 // ctx.cu: false (and the error set) when ctx belongs to a live ensemble
@@ -278,9 +278,11 @@ void learned_release(impec_ctx* ctx);
 impec_status launch_step_graph(impec_ctx* ctx, double t_clip);
 impec_status launch_pressure_graph(impec_ctx* ctx);
 void invalidate_step_graph(impec_ctx* ctx);
+impec_status capture_cn_solve(impec_ctx* ctx, const double* c, double* x);  // c -> x, WHILE node in the active capture
 // step.cu
 impec_status hyperbolic_solve_dev(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev,
                                   int* pfs);
+impec_status hyperbolic_capture(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev, int* pfs);
 // reductions (common.cu)
 impec_status reduce_launch_sum(impec_ctx* ctx, const double* x, size_t n, double* out_dev);
 impec_status sync_scalars(impec_ctx* ctx);

@@ -18,14 +18,14 @@ static impec_status set_dt(impec_ctx* ctx, double dt) {
     return IMPEC_OK;
 }
 
-static impec_status cn_solve_host(impec_ctx* ctx, double* c, double tol) {
-    IMPEC_TRY(cn_prepare(ctx, c, 0.5, &ctx->dscal->dt, false));
-    IMPEC_TRY(cn_iteration(ctx, c));  // the first sweep before the first check, as in the step graph
+static impec_status cn_solve_host(impec_ctx* ctx, const double* c, double* x, double tol) {
+    IMPEC_TRY(cn_prepare(ctx, c, x));
+    IMPEC_TRY(cn_iteration(ctx, x));  // the first sweep before the first check, as in the step graph
     IMPEC_TRY(cn_check(ctx, tol, 1, 0, 0));
     for (;;) {
         IMPEC_TRY(sync_scalars(ctx));
         if (!ctx->hscal->go) break;
-        IMPEC_TRY(cn_iteration(ctx, c));
+        IMPEC_TRY(cn_iteration(ctx, x));
         IMPEC_TRY(cn_check(ctx, tol, 1, 0, 0));
     }
     if (ctx->hscal->flags & FLAG_CN_NAN) return IMPEC_ERR_NAN;
@@ -33,21 +33,36 @@ static impec_status cn_solve_host(impec_ctx* ctx, double* c, double tol) {
     return IMPEC_OK;
 }
 
-// HyperbolicSplitSolver::Solve with SPLIT2ND (src/HyperbolicSplitSolver.cpp:162-198), host
-// driven.  Both Crank-Nicolson half steps share v and dt/2, hence one matrix per call.
+// HyperbolicSplitSolver::Solve with SPLIT2ND (src/HyperbolicSplitSolver.cpp:162-198), its CN solves by
+// `solve(c, x)` (c -> x).  Both Crank-Nicolson half steps share v and dt/2, hence one matrix per
+// call.  With dispersion the field goes c -> t1 (CN) -> t2 (advection) -> c (CN): no step works in
+// place, so nothing is copied back.
+template <class Solve>
+static impec_status hyperbolic_parts(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev,
+                                     int* pfs, Solve solve) {
+    IMPEC_TRY(tr_integrate_dev(ctx, c, 0.5, dt_dev, 0));
+    if (!ctx->P.diffusion) {
+        IMPEC_TRY(advect_split_dev(ctx, c, c, ctx->t1, ctx->t2, ctx->t3, u, v, dt_dev, pfs));
+        return tr_integrate_dev(ctx, c, 0.5, dt_dev, 1);
+    }
+    IMPEC_TRY(cn_setup(ctx, u, v, 0.5, dt_dev));
+    IMPEC_TRY(solve((const double*)c, ctx->t1));
+    IMPEC_TRY(advect_split_dev(ctx, ctx->t1, ctx->t2, c, ctx->t3, nullptr, u, v, dt_dev, pfs));
+    IMPEC_TRY(tr_integrate_dev(ctx, ctx->t2, 0.5, dt_dev, 1));
+    return solve((const double*)ctx->t2, c);
+}
+
+// Launch only, for the step graph.
+impec_status hyperbolic_capture(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev, int* pfs) {
+    return hyperbolic_parts(ctx, c, u, v, dt_dev, pfs, [&](const double* a, double* x) { return capture_cn_solve(ctx, a, x); });
+}
+
+// Host driven.
 impec_status hyperbolic_solve_dev(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev,
                                   int* pfs) {
-    const impec_params& P = ctx->P;
     IMPEC_CUDA_TRY(cudaMemsetAsync(&ctx->dscal->flags, 0, sizeof(int), ctx->stream));
-    IMPEC_TRY(tr_integrate_dev(ctx, c, 0.5, dt_dev, 0));
-    if (P.diffusion) {
-        IMPEC_TRY(cn_setup(ctx, u, v, 0.5, dt_dev));
-        IMPEC_TRY(cn_solve_host(ctx, c, P.para_eps));
-    }
-    IMPEC_TRY(advect_split_dev(ctx, c, u, v, dt_dev, pfs));
-    IMPEC_TRY(tr_integrate_dev(ctx, c, 0.5, dt_dev, 1));
-    if (P.diffusion) IMPEC_TRY(cn_solve_host(ctx, c, P.para_eps));
-    return IMPEC_OK;
+    return hyperbolic_parts(ctx, c, u, v, dt_dev, pfs,
+                            [&](const double* a, double* x) { return cn_solve_host(ctx, a, x, ctx->P.para_eps); });
 }
 
 // GetTotalMass, CalculateDivergenceError, CalculateVelocityBoundaryError, max/min c
@@ -210,7 +225,7 @@ impec_status impec_advect_split(impec_ctx* ctx, double* c, const double* u, cons
     IMPEC_RANGE("impec_advect_split");
     if (!ctx || !c || !u || !v || !pfs) return IMPEC_ERR_ARG;
     IMPEC_TRY(set_dt(ctx, dt));
-    IMPEC_TRY(advect_split_dev(ctx, c, u, v, &ctx->dscal->dt, pfs));
+    IMPEC_TRY(advect_split_dev(ctx, c, c, ctx->t1, ctx->t2, ctx->t3, u, v, &ctx->dscal->dt, pfs));
     IMPEC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return IMPEC_OK;
 }

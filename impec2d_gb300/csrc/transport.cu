@@ -567,22 +567,26 @@ impec_status advect_y_dev(impec_ctx* ctx, const double* cin, double* cout, const
     return advect_tiles<MODE_Y>(ctx, cin, cout, nullptr, v, 0.0, dt_scale, dt_dev);
 }
 
-// AdvectSplit (src/HyperbolicSplitSolver.cpp:51-106); pfs 0 = X_SWEEP, 1 = Y_SWEEP.
-impec_status advect_split_dev(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev,
-                              int* pfs) {
+// AdvectSplit (src/HyperbolicSplitSolver.cpp:51-106), cin -> cout; pfs 0 = X_SWEEP, 1 = Y_SWEEP.  cout may
+// be cin; if not, cin's values are lost.  s1, s2, s3: scratch fields, none of them cin or cout.
+impec_status advect_split_dev(impec_ctx* ctx, double* cin, double* cout, double* s1, double* s2, double* s3, const double* u,
+                              const double* v, const double* dt_dev, int* pfs) {
     const impec_params& P = ctx->P;
     const size_t bytes = (size_t)P.N1 * P.N2 * 8;
-    double *t1 = ctx->t1, *t2 = ctx->t2, *t3 = ctx->t3;
-    if (P.hmtype == IMPEC_CTU) {  // unsplit: one CTU update, c -> t1, then back into c; pfs untouched
+    // one-launch updates read neighbouring tiles' old values: in place they go through s1
+    double* to = cout == cin ? s1 : cout;
+    auto back = [&]() -> impec_status {
+        if (to != cout) IMPEC_CUDA_TRY(cudaMemcpyAsync(cout, to, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        return IMPEC_OK;
+    };
+    if (P.hmtype == IMPEC_CTU) {  // unsplit: one CTU update; the alternating-sweep state stays as it was
         const double fx = 1.0 / (ctx->G.dx * P.porosity), fy = 1.0 / (ctx->G.dy * P.porosity);
+        const auto k = P.bc == IMPEC_BC_PERIODIC ? k_ctu<IMPEC_BC_PERIODIC> : k_ctu<IMPEC_BC_NEUMANN>;
         ++ctx->nlaunch;
-        if (P.bc == IMPEC_BC_PERIODIC) launch_k(ctx->stream, k_ctu<IMPEC_BC_PERIODIC>, tgrid(P.N1, P.N2), dim3(TBX, TBY), 0, P.N1, P.N2, c, t1, u, v, dt_dev, fx, fy);
-        else launch_k(ctx->stream, k_ctu<IMPEC_BC_NEUMANN>, tgrid(P.N1, P.N2), dim3(TBX, TBY), 0, P.N1, P.N2, c, t1, u, v, dt_dev, fx, fy);
+        launch_k(ctx->stream, k, tgrid(P.N1, P.N2), dim3(TBX, TBY), 0, P.N1, P.N2, (const double*)cin, to, u, v, dt_dev, fx, fy);
         IMPEC_LAUNCH_CHECK();
-        IMPEC_CUDA_TRY(cudaMemcpyAsync(c, t1, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-        return IMPEC_OK;  // unsplit: the alternating-sweep state stays as it was
+        return back();
     }
-    // one tile launch per update, c -> t1 (neighbouring tiles read the old c), then back into c
     bool x_first = true;
     switch (P.dim_splitting) {
         case IMPEC_ALTERNATING: x_first = *pfs == 1; break;
@@ -594,34 +598,30 @@ impec_status advect_split_dev(impec_ctx* ctx, double* c, const double* u, const 
             // last X(dt/2) reads them there (src/HyperbolicSplitSolver.cpp:80-85, :128-131, :152-155).
             // Only the two rows next to each end are ever read, so with tiles Y(dt) of the input runs
             // there only.
+            *pfs = 0;
             if (by_cells(P)) {
-                IMPEC_TRY(sweep_cells(ctx, false, c, t3, v, 1.0, dt_dev));
-                IMPEC_TRY(sweep_cells(ctx, true, c, t1, u, 0.5, dt_dev));
-                IMPEC_TRY(sweep_cells(ctx, false, t1, t2, v, 1.0, dt_dev));
-                IMPEC_TRY(sweep_cells(ctx, true, t2, c, u, 0.5, dt_dev, t3));
-                *pfs = 0;
-                return IMPEC_OK;
+                double* mid = cout == cin ? s3 : cin;  // the input is done with after two sweeps
+                IMPEC_TRY(sweep_cells(ctx, false, cin, s2, v, 1.0, dt_dev));
+                IMPEC_TRY(sweep_cells(ctx, true, cin, s1, u, 0.5, dt_dev));
+                IMPEC_TRY(sweep_cells(ctx, false, s1, mid, v, 1.0, dt_dev));
+                return sweep_cells(ctx, true, mid, cout, u, 0.5, dt_dev, s2);
             }
-            IMPEC_TRY(advect_tiles<MODE_Y>(ctx, c, t3, nullptr, v, 0.0, 1.0, dt_dev, nullptr, true));
-            IMPEC_TRY(advect_tiles<MODE_XY>(ctx, c, t2, u, v, 0.5, 1.0, dt_dev));
-            IMPEC_TRY(advect_tiles<MODE_X>(ctx, t2, c, u, nullptr, 0.5, 0.0, dt_dev, t3));
-            *pfs = 0;
-            return IMPEC_OK;
+            IMPEC_TRY(advect_tiles<MODE_Y>(ctx, cin, s2, nullptr, v, 0.0, 1.0, dt_dev, nullptr, true));
+            IMPEC_TRY(advect_tiles<MODE_XY>(ctx, cin, s1, u, v, 0.5, 1.0, dt_dev));
+            return advect_tiles<MODE_X>(ctx, s1, cout, u, nullptr, 0.5, 0.0, dt_dev, s2);
         default:
-            IMPEC_TRY(advect_tiles<MODE_SYM>(ctx, c, t1, u, v, 1.0, 1.0, dt_dev));
-            IMPEC_CUDA_TRY(cudaMemcpyAsync(c, t1, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
             *pfs = 0;
-            return IMPEC_OK;
+            IMPEC_TRY(advect_tiles<MODE_SYM>(ctx, cin, to, u, v, 1.0, 1.0, dt_dev));
+            return back();
     }
     *pfs = x_first ? 0 : 1;
-    if (by_cells(P)) {  // two launches through t1, no copy
-        IMPEC_TRY(sweep_cells(ctx, x_first, c, t1, x_first ? u : v, 1.0, dt_dev));
-        return sweep_cells(ctx, !x_first, t1, c, x_first ? v : u, 1.0, dt_dev);
+    if (by_cells(P)) {  // two launches through s1, no copy
+        IMPEC_TRY(sweep_cells(ctx, x_first, cin, s1, x_first ? u : v, 1.0, dt_dev));
+        return sweep_cells(ctx, !x_first, s1, cout, x_first ? v : u, 1.0, dt_dev);
     }
-    IMPEC_TRY(x_first ? advect_tiles<MODE_XY>(ctx, c, t1, u, v, 1.0, 1.0, dt_dev)
-                      : advect_tiles<MODE_YX>(ctx, c, t1, u, v, 1.0, 1.0, dt_dev));
-    IMPEC_CUDA_TRY(cudaMemcpyAsync(c, t1, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    return IMPEC_OK;
+    IMPEC_TRY(x_first ? advect_tiles<MODE_XY>(ctx, cin, to, u, v, 1.0, 1.0, dt_dev)
+                      : advect_tiles<MODE_YX>(ctx, cin, to, u, v, 1.0, 1.0, dt_dev));
+    return back();
 }
 
 }  // namespace impec

@@ -115,3 +115,36 @@ def test_sweep_tiles(engine, oracle_lib, N1, N2, scheme, mode):
     assert ctx.advect_split(d, dev(u), dev(vv), dt, 1) == pfs.value
     assert rel_err(host(d), O.interior(OP, cg)) <= 1e-13
     ctx.close()
+
+
+@pytest.mark.parametrize("N1,N2", [(2, 2), (3, 5), (16, 32), (17, 33), (15, 31), (33, 257), (48, 513), (130, 70)])
+@pytest.mark.parametrize("stype", [0, 2])  # wells; a Dirichlet row in the CN system (N1 >= 4)
+def test_cn_half_step_at_tile_edges(engine, oracle_lib, N1, N2, stype):
+    """The dispersion kernels at the edges of their 16 x 32 tiles, row segments (256 and 512
+    columns) and odd row counts, against the oracle's CN solve.  Both stop at 1e-13 of ||b|| and
+    the matrix is within a factor 3 of the identity here: 1e-12, in the norm that the residual has."""
+    import ctypes as C
+
+    import oracle as O
+    from helpers import cell_ghost, dev, host, smooth_field, vel_split
+    if stype == 2 and N1 < 4:
+        return
+    E = engine
+    P = E.default_params(N1, N2, stype=stype, diffusion=1, alpha_l=0.5, alpha_t=0.05, Dm=1e-3, para_eps=1e-13, max_cycles=400)
+    OP = oparams(P)
+    v = np.zeros(O.vel_shape(OP))
+    c = np.random.default_rng(6).uniform(0.0, 1.0, (N1, N2))
+    cg = cell_ghost(OP, c)
+    p = smooth_field(N1, N2, 9, -1.0, 1.0) * 0.05
+    oracle_lib.or_calc_velocities(C.byref(OP), O.ptr(cell_ghost(OP, p)), O.ptr(v), O.ptr(cg))
+    u, vv = vel_split(OP, v)
+    dt = 0.5 * oracle_lib.or_max_stable_dt(C.byref(OP), O.ptr(v))
+    its, rr = C.c_int(), C.c_double()
+    assert oracle_lib.or_cn_solve(C.byref(OP), O.ptr(cg), O.ptr(v), dt, 0, 1e-14, C.byref(its), C.byref(rr)) == 0
+    ctx = E.Context(P)
+    d = dev(c)
+    _, rr_d = ctx.dispersion_cn(d, dev(u), dev(vv), dt, 1e-13)
+    assert rr_d <= 1e-13
+    ref = O.interior(OP, cg)
+    assert np.linalg.norm(host(d) - ref) <= 1e-12 * np.linalg.norm(ref)
+    ctx.close()
