@@ -24,7 +24,16 @@
 // found without an integer division.
 //
 // Staging: every CTA copies its bands (and CTA 0 the coarsest inverse) with asynchronous
-// element copies (cp.async), all in flight at once, and waits for them once.
+// element copies (cp.async), all in flight at once, and waits for them once.  That takes 11,000 of
+// the launch's 100,000 cycles, so the kernel is launched with programmatic serialisation: it stages
+// its operators while the kernel before it, the restriction that produces its right-hand side,
+// still runs (300 x 130 solve 1.80 -> 1.71 ms, 1024^2 step 4.20 -> 4.16, alternating runs).  A solve
+// whose finest level is the cluster's has no such kernel in front inside its loop.
+//
+// Measured without gain (100,000 instead of 101,000 cycles): each thread's cell and its
+// coefficients held in registers over a level's colours.  A colour of a small level then takes 650
+// cycles instead of 1,000, but fetching them takes as long, and the rest is the barrier (1,000 to
+// 1,400 cycles, 26 of them), the gathers and the prolongations.
 //
 // Every barrier is reached by all threads of all CTAs the same number of times (the counts
 // depend only on the arguments), and no CTA touches another's shared memory after the last one.
@@ -361,14 +370,13 @@ __device__ void cl_prolong9(const cooperative_groups::cluster_group& cl, T* sm, 
 // KIND: FACE5 or EXP9 (every level of the cycle).
 template <class T, int KIND>
 __global__ void __launch_bounds__(CL_THREADS) k_cluster_vcycle(const __grid_constant__ ClusterArgs<T> A) {
-    pdl_enter();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char cl_raw[];
     T* sm = reinterpret_cast<T*>(cl_raw);
     const int rank = (int)cl.block_rank();
 
-    // stage this CTA's bands (operators of every level; iterate and rhs of level 0)
+    // stage this CTA's bands: operators of every level
     for (int l = 0; l < A.nl; ++l) {
         int lo, cnt;
         cl_band(A, l, rank, lo, cnt);
@@ -402,21 +410,28 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_vcycle(const __grid_cons
                 for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) stage_async(tx + e * ps + k, A.a9[l] + e * n + at + k);
             for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) stage_async(id + k, A.id[l] + at + k);
         }
-        if (l == 0) {
-            T* x = sm + A.off[0][CL_X];
-            T* b = sm + A.off[0][CL_B];
-            for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) stage_async(b + k, A.b0 + at + k);
-            if (KIND != FACE5) {
-                for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) stage_async(x + k, A.x0 + at + k);
-            } else if (!A.zero0) {  // with the neighbours' edge rows
-                const int first = lo > 0 ? 0 : 1, last = lo + cnt < A.n1[0] ? cnt + 2 : cnt + 1;
-                for (int k = first * n2 + threadIdx.x; k < last * n2; k += CL_THREADS) stage_async(x + k, A.x0 + at + k - n2);
-            }
-        }
     }
     if (rank == 0) {  // the dense inverse of the coarsest level
         double* dinv = reinterpret_cast<double*>(cl_raw + A.dinv_off);
         for (int k = threadIdx.x; k < A.dn * A.dn; k += CL_THREADS) stage_async(dinv + k, A.dinv + k);
+    }
+    // The operators were complete before the kernel in front of this one began (it does not write
+    // them); its output, level 0's right-hand side and iterate, only counts from here on.
+    pdl_enter();
+    {
+        int lo, cnt;
+        cl_band(A, 0, rank, lo, cnt);
+        const int n2 = A.n2[0];
+        const size_t at = (size_t)lo * n2;
+        T* x = sm + A.off[0][CL_X];
+        T* b = sm + A.off[0][CL_B];
+        for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) stage_async(b + k, A.b0 + at + k);
+        if (KIND != FACE5) {
+            for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) stage_async(x + k, A.x0 + at + k);
+        } else if (!A.zero0 && cnt > 0) {  // with the neighbours' edge rows
+            const int first = lo > 0 ? 0 : 1, last = lo + cnt < A.n1[0] ? cnt + 2 : cnt + 1;
+            for (int k = first * n2 + threadIdx.x; k < last * n2; k += CL_THREADS) stage_async(x + k, A.x0 + at + k - n2);
+        }
     }
     stage_wait();
     cl.sync();

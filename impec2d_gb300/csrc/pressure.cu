@@ -1555,7 +1555,7 @@ static void launch_cluster(impec_ctx* ctx, size_t ls, bool zero) {
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cfg.numAttrs = 2;  // always with programmatic serialisation (mgcluster.cuh: staging)
     ++ctx->nlaunch;
     if (ctx->L[ls].kind == FACE5) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5>, A);
     else if constexpr (sizeof(T) == 8) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, EXP9>, A);
