@@ -990,6 +990,7 @@ __global__ void k_apply_ref(Level F, const double* __restrict__ x, int pin, int 
 
 #include "mgfused.cuh"
 #include "mgcluster.cuh"
+#include "mglevel.cuh"
 
 constexpr size_t MG_COARSE_SMEM = 160 * 1024;
 constexpr size_t MG_CLUSTER_SMEM = 200 * 1024;
@@ -1018,6 +1019,19 @@ static int cluster_size_for(int want) {
 }
 
 // ---------------------------------------------------------------- host orchestration
+
+template <class T, int TR, int TC>
+static cudaError_t level_attribute() {
+    const int smem = (int)LvTile<T, TR, TC>::SMEM;
+    const cudaError_t e = cudaFuncSetAttribute(k_down5<T, TR, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_up5<T, TR, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}
+static impec_status level_kernel_attributes() {
+    IMPEC_CUDA_TRY((level_attribute<double, 16, 32>()));
+    IMPEC_CUDA_TRY((level_attribute<double, 16, 16>()));
+    IMPEC_CUDA_TRY((level_attribute<float, 32, 32>()));
+    return IMPEC_OK;
+}
 
 impec_status pressure_alloc(impec_ctx* ctx) {
     const impec_params& P = ctx->P;
@@ -1119,6 +1133,7 @@ impec_status pressure_alloc(impec_ctx* ctx) {
     IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_coarse_vcycle<float, FACE5>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
     IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_coarse_vcycle<float, EXP9>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
     const int cls = (int)MG_CLUSTER_SMEM;
+    IMPEC_TRY(level_kernel_attributes());
     ctx->cl_size = 0;
     const int want = (int)env_long("IMPEC_MG_CL_CTAS", CL_MAX_CTAS);
     const bool f5 = ctx->L[0].kind == FACE5;
@@ -1570,6 +1585,43 @@ static bool zero_start_free(impec_ctx* ctx, size_t l) {
            (l == cluster_start<T>(ctx) || l != coarse_start<T>(ctx));
 }
 
+// Whether a half cycle of level l is one launch (mglevel.cuh): per-level five-point kernels with the
+// default three colours on either side, starting from x = 0 (CG), with both red-black shortcuts.
+template <class T>
+static bool fused_level(impec_ctx* ctx, size_t l) {
+    const Colours c = colours(ctx);
+    return ctx->krylov && ctx->L[l].kind == FACE5 && c.npre == LV_N && c.npost == LV_N && ctx->tune.rb_skip != 0 &&
+           ctx->tune.rb_resid != 0;
+}
+
+template <class T, int TR, int TC>
+static void launch_down_up(impec_ctx* ctx, Level& F, Level& C, bool down, T* xc, const unsigned char* mask) {
+    const T *tx, *ty, *a9, *id, *tx_, *ty_, *a9_, *id_;
+    T *x, *b, *cx, *cb;
+    level_ptrs<T>(F, tx, ty, a9, id, x, b);
+    level_ptrs<T>(C, tx_, ty_, a9_, id_, cx, cb);
+    const dim3 g((F.n2 + TC - 1) / TC, (F.n1 + TR - 1) / TR);
+    const int vec = F.n2 % (int)(16 / sizeof(T)) == 0;  // rows of 16-byte pieces (the arrays are cudaMalloc's)
+    ++ctx->nlaunch;
+    if (down)
+        launch_k(ctx->stream, k_down5<T, TR, TC>, g, LV_T, LvTile<T, TR, TC>::SMEM, F.n1, F.n2, tx, ty, id, level_diag<T>(F),
+                 (const T*)b, level_alt<T>(F), C.n1, C.n2, level_w4<T>(C), cb, xc, vec);
+    else
+        launch_k(ctx->stream, k_up5<T, TR, TC>, g, LV_T, LvTile<T, TR, TC>::SMEM, F.n1, F.n2, tx, ty, id, (const T*)b,
+                 (const T*)level_alt<T>(F), x, C.n1, C.n2, (const T*)cx, level_w4<T>(C), mask, vec);
+}
+// Tiles (ms): FP64 16 x 32 on large levels, 16 x 16 where those leave SMs idle (1024^2 step 4.05 / 4.11
+// and 4.20 with 32 x 32; 513 x 777 nine-point step 3.07 / 2.96); FP32 32 x 32, whose halo costs less than
+// 16 x 32's (2048^2 step 7.95 / 8.14, 4096^2 solve 25.6 / 26.9) and which leaves more blocks per SM
+// than 32 x 64 (8.92, 29.1).  One launch per colour and transfer: 4.13, 3.22, 8.41, 29.0; 300 x 130
+// solve 1.80 against 1.53, 256^2 step 1.03 against 0.95.
+template <class T>
+static void launch_half(impec_ctx* ctx, Level& F, Level& C, bool down, T* xc, const unsigned char* mask) {
+    if constexpr (sizeof(T) == 4) launch_down_up<T, 32, 32>(ctx, F, C, down, xc, mask);
+    else if (F.n() >= (size_t)1 << 19) launch_down_up<T, 16, 32>(ctx, F, C, down, xc, mask);
+    else launch_down_up<T, 16, 16>(ctx, F, C, down, xc, mask);
+}
+
 // One V-cycle from level l down.  zero: the level's iterate stands for x = 0; unless
 // zero_start_free<T>(ctx, l), the caller has filled it with zeros.  first_done: the caller
 // (the restriction from level l - 1) also did the pre-smoothing's first colour.
@@ -1604,6 +1656,12 @@ static void vcycle(impec_ctx* ctx, size_t l, bool zero, bool first_done = false)
         launch_k(ctx->stream, k_prolong<T>, grid2(F.n1, F.n2), dim3(BX, BY), 0, F.n1, F.n2, x, C.n1, C.n2, (const T*)cx,
                  (const T*)nullptr, mask);
         smooth9<T>(ctx, F, (int)ctx->tune.post, true);
+        return;
+    }
+    if (zero && fused_level<T>(ctx, l)) {
+        launch_half<T>(ctx, F, C, true, l + 1 == lc && l + 1 != cl ? cx : nullptr, mask);
+        vcycle<T>(ctx, l + 1, true);
+        launch_half<T>(ctx, F, C, false, nullptr, mask);
         return;
     }
     const Colours col = colours(ctx);

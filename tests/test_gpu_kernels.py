@@ -148,3 +148,29 @@ def test_cn_half_step_at_tile_edges(engine, oracle_lib, N1, N2, stype):
     ref = O.interior(OP, cg)
     assert np.linalg.norm(host(d) - ref) <= 1e-12 * np.linalg.norm(ref)
     ctx.close()
+
+
+@pytest.mark.parametrize("N1,N2", [(130, 132), (131, 257), (260, 130), (514, 515), (1030, 770)])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_half_cycle_kernels_match_separate_launches(engine, monkeypatch, N1, N2, prec):
+    """A half cycle per launch (tiles with a recomputed halo; 16-byte and element staging, last tiles
+    of a few rows and columns) gives the bits of one launch per colour and transfer: the same
+    cycles, residual and pressure.  A context without the red-black shortcuts runs the latter."""
+    import torch
+
+    from helpers import dev, host
+    E = engine
+    c = np.random.default_rng(4).uniform(0.0, 1.0, (N1, N2))
+    out = []
+    for skip in ("1", "0"):
+        monkeypatch.setenv("IMPEC_MG_RB_SKIP", skip)
+        P = E.default_params(N1, N2, stype=1, nu=1.0, precision=prec, max_cycles=200)
+        ctx = E.Context(P)
+        ctx.set_source(dev(source(oparams(P))))
+        p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+        n0 = E.launch_count(ctx)
+        cyc, rr, _ = ctx.pressure_solve(dev(c), p, 1e-10)
+        out.append((cyc, rr, host(p), E.launch_count(ctx) - n0))
+        ctx.close()
+    assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
+    assert out[0][3] < out[1][3]
