@@ -1424,7 +1424,8 @@ static size_t coarse_start(const impec_ctx* ctx) {
     // with a Dirichlet row the finest level keeps its own kernels (its prolongation is masked)
     const size_t l0 = ctx->dir_row >= 0 && ctx->L.size() > 1 ? 1 : 0;
     for (size_t l = l0; l < ctx->L.size(); ++l)
-        if (ctx->L[l].n() <= cells && coarse_bytes<T>(ctx, l) <= MG_COARSE_SMEM) return l;
+        if (ctx->L[l].n() <= cells && ctx->L.size() - l <= (size_t)MGC_MAXL && coarse_bytes<T>(ctx, l) <= MG_COARSE_SMEM)
+            return l;
     return ctx->L.size() - 1;
 }
 
