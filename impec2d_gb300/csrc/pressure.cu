@@ -1733,10 +1733,40 @@ __global__ void k_mg_check(DevScalars* S, double tol, int max_cycles, int inc, c
 //   beta = (z_k, r_k - r_{k-1}) / (z_{k-1}, r_{k-1}) = -alpha_{k-1} (z_k, A p_{k-1}) / (z_{k-1}, r_{k-1}),
 // which needs only (z, r) and (z, q) with q = A p still holding the previous direction.
 
-// z: the V-cycle's finest iterate, FP64 or FP32.
-__device__ __forceinline__ double cg_z(const double* __restrict__ z, const float* __restrict__ z32, size_t k) {
-    return z32 ? (double)z32[k] : z[k];
+// The vector kernels walk the flat arrays in pairs of values (16-byte accesses, every array being
+// an allocation of its own), CG_U pairs per thread with all their loads in flight; the remainder goes pair by
+// pair (a batch under a predicate would occupy the FP64 pipe for its absent pairs too).  Their limits are
+// HBM and that pipe, of which a float-to-double conversion takes as much as an addition: widen()
+// converts with integer operations.  Measured against one value per step and plain conversions, 4096^2
+// with an FP32 cycle: dots 181 -> 114 us, update 178 -> 145, direction 77 -> 44; 1024^2 FP64: 21.3 ->
+// 17.6, 15.7, 7.1 -> 6.2.
+constexpr int CG_U = 2;
+
+// f(std::integral_constant<int, U>, k, step): the U pairs k, k + step, ..
+template <class F>
+__device__ __forceinline__ void walk_pairs(size_t n, F&& f) {
+    const size_t pairs = n / 2, step = (size_t)gridDim.x * blockDim.x;
+    size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (; k + (CG_U - 1) * step < pairs; k += CG_U * step) f(std::integral_constant<int, CG_U>(), k, step);
+    for (; k < pairs; k += step) f(std::integral_constant<int, 1>(), k, step);
 }
+
+// (double)v by moving the fields; subnormal values are scaled into the normal range first (exact).
+// Without a branch: a conversion under a predicate would occupy the FP64 pipe all the same.
+__device__ __forceinline__ double widen(float v) {
+    const bool small = (__float_as_uint(v) & 0x7fffffffu) < 0x00800000u;
+    const unsigned u = __float_as_uint(small ? v * 0x1p64f : v), m = u & 0x7fffffffu;
+    unsigned hi = (m >> 3) + (small ? 0x34000000u : 0x38000000u);  // exponent bias + 896 (- 64)
+    if (m >= 0x7f800000u) hi |= 0x7ff00000u;  // infinite, NaN
+    if (m == 0u) hi = 0u;
+    return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)(u << 29));
+}
+
+// z: the V-cycle's finest iterate, FP64 or FP32.
+__device__ __forceinline__ double2 load_pair(const double* p, size_t k) { return reinterpret_cast<const double2*>(p)[k]; }
+__device__ __forceinline__ float2 load_pair(const float* p, size_t k) { return reinterpret_cast<const float2*>(p)[k]; }
+__device__ __forceinline__ double wide(double v) { return v; }
+__device__ __forceinline__ double wide(float v) { return widen(v); }
 
 // (r, z) and (z, q) into out[0], out[1].  With S (CG, out = &S->pcg_rz), the last block also
 // stores the direction's beta = -alpha_old (z, q) / (z, r)_old (0 on the first iteration).
@@ -1745,40 +1775,87 @@ __device__ __forceinline__ double cg_z(const double* __restrict__ z, const float
 // no direction removes; the cycle answers it with a far larger mean of z (four times the
 // right-hand side per cell on each coarser level), and their product came to outweigh the rest of
 // (r, z): past its best iterate CG then diverged (1024^2, nu = 2/3: from 8e-11 of ||f|| to 1e-6 in
-// five iterations).
-template <int K>
-__global__ void __launch_bounds__(RED_THREADS) k_cg_dots(int n1, int n2, const double* __restrict__ r,
-                                                         const double* __restrict__ z, const float* __restrict__ z32,
-                                                         const double* __restrict__ q, double* partials, int mb,
-                                                         unsigned* counter, double* out, DevScalars* S) {
+// five iterations).  An FP32 z is summed in FP32 over a thread's 2 CG_U values at a time, whose
+// rounding is that of the values themselves.
+template <int K, class Z>
+__global__ void __launch_bounds__(RED_THREADS) k_cg_dots(size_t n, const double* __restrict__ r,
+                                                            const Z* __restrict__ z, const double* __restrict__ q,
+                                                            double* partials, int mb, unsigned* counter, double* out,
+                                                            DevScalars* S) {
     pdl_enter();
     double acc[K];
 #pragma unroll
     for (int e = 0; e < K; ++e) acc[e] = 0.0;
-    for_cells(n1, n2, [&](int, int, size_t k) {
-        const double zz = cg_z(z, z32, k), rr = r[k];
-        acc[0] += rr * zz;
-        acc[1] += zz * q[k];
-        if (K == 4) {
-            acc[K - 2] += zz;
-            acc[K - 1] += rr;
+    walk_pairs(n, [&](auto u, size_t k0, size_t step) {
+        constexpr int U = u.value;
+        double2 rr[U], qq[U];
+        decltype(load_pair(z, 0)) zz[U];
+#pragma unroll
+        for (int e = 0; e < U; ++e) {
+            rr[e] = load_pair(r, k0 + e * step);
+            zz[e] = load_pair(z, k0 + e * step);
+            qq[e] = load_pair(q, k0 + e * step);
         }
+        Z zs = 0;
+#pragma unroll
+        for (int e = 0; e < U; ++e) {
+            const double z0 = wide(zz[e].x), z1 = wide(zz[e].y);
+            acc[0] += rr[e].x * z0;
+            acc[1] += z0 * qq[e].x;
+            acc[0] += rr[e].y * z1;
+            acc[1] += z1 * qq[e].y;
+            if (K == 4) {
+                zs = e == 0 ? zz[e].x + zz[e].y : zs + (zz[e].x + zz[e].y);
+                acc[K - 1] += rr[e].x;
+                acc[K - 1] += rr[e].y;
+            }
+        }
+        if (K == 4) acc[K - 2] += wide(zs);
     });
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        const double z0 = wide(z[n - 1]), r0 = r[n - 1];
+        acc[0] += r0 * z0;
+        acc[1] += z0 * q[n - 1];
+        if (K == 4) {
+            acc[K - 2] += z0;
+            acc[K - 1] += r0;
+        }
+    }
     if (grid_reduce<K>(acc, 0u, partials, mb, counter, out) && threadIdx.x == 0 && S) {
-        if (K == 4) S->pcg_rz -= S->pcg_zsum * S->pcg_rsum / ((double)n1 * n2);
+        if (K == 4) S->pcg_rz -= S->pcg_zsum * S->pcg_rsum / (double)n;
         const bool first = S->mg_cycles == 0 || S->pcg_rz_old == 0.0;
         S->pcg_beta = first ? 0.0 : -S->pcg_alpha * S->pcg_zq / S->pcg_rz_old;
     }
 }
 
 // p = z + beta p (p = z on the first iteration, whatever p held).
-__global__ void k_cg_direction(size_t n, const double* __restrict__ z, const float* __restrict__ z32,
-                               double* __restrict__ p, const DevScalars* __restrict__ S) {
+template <class Z>
+__global__ void __launch_bounds__(256) k_cg_direction(size_t n, const Z* __restrict__ z, double* __restrict__ p,
+                                                      const DevScalars* __restrict__ S) {
     pdl_enter();
     const bool first = S->mg_cycles == 0 || S->pcg_rz_old == 0.0;
     const double beta = S->pcg_beta;  // from k_cg_dots
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        p[k] = first ? cg_z(z, z32, k) : cg_z(z, z32, k) + beta * p[k];
+    double2* p2 = reinterpret_cast<double2*>(p);
+    walk_pairs(n, [&](auto u, size_t k0, size_t step) {
+        constexpr int U = u.value;
+        double2 pp[U];
+        decltype(load_pair(z, 0)) zz[U];
+#pragma unroll
+        for (int e = 0; e < U; ++e) {
+            zz[e] = load_pair(z, k0 + e * step);
+            if (!first) pp[e] = p2[k0 + e * step];
+        }
+#pragma unroll
+        for (int e = 0; e < U; ++e) {
+            double2 v = make_double2(wide(zz[e].x), wide(zz[e].y));
+            if (!first) {
+                v.x += beta * pp[e].x;
+                v.y += beta * pp[e].y;
+            }
+            p2[k0 + e * step] = v;
+        }
+    });
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) p[n - 1] = first ? wide(z[n - 1]) : wide(z[n - 1]) + beta * p[n - 1];
 }
 
 // q = A p with the integrated operator (diag p - sum t p_nb) and (p, q) into out[0].  With S
@@ -1817,22 +1894,48 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_apply(Level F, const double*
 // alpha = (r, z) / (p, Ap); x += alpha p; r -= alpha Ap (and its FP32 copy); ||r||^2 over the
 // cells other than the pinned one.  The last block of the reduction then runs the iteration's
 // convergence check (k_mg_check's work, one launch fewer per iteration).
-__global__ void __launch_bounds__(RED_THREADS) k_cg_update(int n1, int n2, double* __restrict__ x,
+__global__ void __launch_bounds__(RED_THREADS) k_cg_update(size_t n, double* __restrict__ x,
                                                            double* __restrict__ r, float* __restrict__ r32,
                                                            const double* __restrict__ p, const double* __restrict__ q,
-                                                           int pin, DevScalars* S, double* partials, int mb,
+                                                           size_t pin, DevScalars* S, double* partials, int mb,
                                                            unsigned* counter, double* out, double tol, int max_cycles,
                                                            cudaGraphConditionalHandle h, int use_h) {
     pdl_enter();
     const double alpha = S->pcg_step;  // from k_cg_apply
     double acc[1] = {0.0};
-    for_cells(n1, n2, [&](int, int, size_t k) {
-        x[k] += alpha * p[k];
-        const double rr = r[k] - alpha * q[k];
-        r[k] = rr;
-        if (r32) r32[k] = (float)rr;
-        if ((int)k != pin) acc[0] += rr * rr;
-    });
+    double2 *x2 = reinterpret_cast<double2*>(x), *r2 = reinterpret_cast<double2*>(r);
+    const size_t pairs = n / 2, step = (size_t)gridDim.x * RED_THREADS;
+    for (size_t k0 = blockIdx.x * (size_t)RED_THREADS + threadIdx.x; k0 < pairs; k0 += CG_U * step) {
+        double2 xx[CG_U], rr[CG_U], pp[CG_U], qq[CG_U];
+#pragma unroll
+        for (int e = 0; e < CG_U; ++e)
+            if (k0 + e * step < pairs) {
+                xx[e] = x2[k0 + e * step];
+                rr[e] = r2[k0 + e * step];
+                pp[e] = load_pair(p, k0 + e * step);
+                qq[e] = load_pair(q, k0 + e * step);
+            }
+#pragma unroll
+        for (int e = 0; e < CG_U; ++e) {
+            const size_t k = k0 + e * step;
+            if (k >= pairs) continue;
+            xx[e].x += alpha * pp[e].x;
+            xx[e].y += alpha * pp[e].y;
+            x2[k] = xx[e];
+            const double ra = rr[e].x - alpha * qq[e].x, rb = rr[e].y - alpha * qq[e].y;
+            r2[k] = make_double2(ra, rb);
+            if (r32) reinterpret_cast<float2*>(r32)[k] = make_float2((float)ra, (float)rb);
+            if (2 * k != pin) acc[0] += ra * ra;
+            if (2 * k + 1 != pin) acc[0] += rb * rb;
+        }
+    }
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        x[n - 1] += alpha * p[n - 1];
+        const double ra = r[n - 1] - alpha * q[n - 1];
+        r[n - 1] = ra;
+        if (r32) r32[n - 1] = (float)ra;
+        if (n - 1 != pin) acc[0] += ra * ra;
+    }
     if (grid_reduce<1>(acc, 0u, partials, mb, counter, out) && threadIdx.x == 0) {
         __threadfence();
         mg_check(S, tol, max_cycles, 1, h, use_h, 1);
@@ -1934,9 +2037,8 @@ static impec_status learned_guess(impec_ctx* ctx, double* x) {
     launch_k(ctx->stream, k_cg_apply, blocks, RED_THREADS, 0, F, (const double*)ctx->lrn_d, ctx->lrn_Ad, ctx->partials,
              ctx->max_blocks, ctx->counter, &S->pcg_pq, (DevScalars*)nullptr);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_dots<2>, blocks, RED_THREADS, 0, F.n1, F.n2, (const double*)ctx->lrn_r0,
-             (const double*)ctx->lrn_d, (const float*)nullptr, (const double*)ctx->lrn_Ad, ctx->partials,
-             ctx->max_blocks, ctx->counter, &S->pcg_rz, (DevScalars*)nullptr);
+    launch_k(ctx->stream, k_cg_dots<2, double>, flat_blocks((F.n() + 1) / 2, cap), RED_THREADS, 0, F.n(),
+             (const double*)ctx->lrn_r0, (const double*)ctx->lrn_d, (const double*)ctx->lrn_Ad, ctx->partials, ctx->max_blocks, ctx->counter, &S->pcg_rz, (DevScalars*)nullptr);
     ++ctx->nlaunch;
     launch_k(ctx->stream, k_learn_step, ctx->num_sms * 4, 256, 0, F.n(), x, (const double*)ctx->lrn_d,
              (const DevScalars*)S, ctx->lrn_alpha);
@@ -2032,17 +2134,26 @@ impec_status pressure_iteration(impec_ctx* ctx, double tol, cudaGraphConditional
     const double* z = mixed ? nullptr : F.x;
     const float* z32 = mixed ? F.x32 : nullptr;
     const int cap = red_cap(ctx->num_sms, ctx->max_blocks), blocks = seg_blocks(F.n1, F.n2, cap);
+    // Blocks per SM of the vector kernels.  The dots are bound by the FP64 pipe, which two blocks fill and
+    // whose block sums are overhead (1024^2: 17.6 us with 2, 19.6 with 4, 23.6 with 8); the update by
+    // HBM (15.8 us with 4, 18.6 with 8), the direction by it too (4096^2 FP32: 53 us with 4, 44 with 8).
+    const auto vblocks = [&](int per_sm) { return flat_blocks((n + 1) / 2, min(ctx->num_sms * per_sm, ctx->max_blocks)); };
+    const auto dots = [&](auto kernel, auto* zz) {
+        ++ctx->nlaunch;
+        launch_k(ctx->stream, kernel, vblocks(2), RED_THREADS, 0, n, (const double*)r, zz, (const double*)ctx->cg_q, ctx->partials,
+                 ctx->max_blocks, ctx->counter, &S->pcg_rz, S);
+    };
+    if (mixed) dots(ctx->singular ? k_cg_dots<4, float> : k_cg_dots<2, float>, z32);
+    else dots(ctx->singular ? k_cg_dots<4, double> : k_cg_dots<2, double>, z);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, ctx->singular ? k_cg_dots<4> : k_cg_dots<2>, blocks, RED_THREADS, 0, F.n1, F.n2, (const double*)r, z, z32,
-             (const double*)ctx->cg_q, ctx->partials, ctx->max_blocks, ctx->counter, &S->pcg_rz, S);
-    ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_direction, ctx->num_sms * 4, 256, 0, n, z, z32, ctx->cg_p, S);
+    if (mixed) launch_k(ctx->stream, k_cg_direction<float>, vblocks(8), 256, 0, n, z32, ctx->cg_p, (const DevScalars*)S);
+    else launch_k(ctx->stream, k_cg_direction<double>, vblocks(8), 256, 0, n, z, ctx->cg_p, (const DevScalars*)S);
     ++ctx->nlaunch;
     launch_k(ctx->stream, k_cg_apply, blocks, RED_THREADS, 0, F, ctx->cg_p, ctx->cg_q, ctx->partials,
              ctx->max_blocks, ctx->counter, &S->pcg_pq, S);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_update, blocks, RED_THREADS, 0, F.n1, F.n2, ctx->cg_x, r, mixed ? F.b32 : nullptr,
-             (const double*)ctx->cg_p, (const double*)ctx->cg_q, pin_index(ctx), S, ctx->partials, ctx->max_blocks,
+    launch_k(ctx->stream, k_cg_update, vblocks(4), RED_THREADS, 0, n, ctx->cg_x, r, mixed ? F.b32 : nullptr,
+             (const double*)ctx->cg_p, (const double*)ctx->cg_q, (size_t)pin_index(ctx), S, ctx->partials, ctx->max_blocks,
              ctx->counter, &S->rnorm2, tol, ctx->P.max_cycles, h, 0);
     ++ctx->nlaunch;
     launch_k(ctx->stream, k_cg_verify, blocks, RED_THREADS, 0, F, (const double*)ctx->f, (const double*)ctx->cg_x,

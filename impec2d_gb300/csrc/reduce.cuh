@@ -17,30 +17,41 @@ __device__ __forceinline__ double warp_max(double v) {
     return v;
 }
 
-// Reduce K values across the block; result valid in thread 0.  maxmask bit k selects max.
-// A shared-memory tree (128, 64, 32 pairs) and then one warp's shuffle tree: 12 FP64 warp
-// instructions per value instead of 45 for a shuffle tree in every warp.  An FP64 instruction
-// costs the same whether all lanes or some take part, so the pairing count is what matters.
+// Reduce K values across the block; the results are valid in thread 0.  maxmask bit k selects max.
+// An FP64 instruction occupies a quarter of an SM for 64 cycles whether all lanes or some take part, so the
+// instruction count on the busiest quarter is what matters.  One value: a shared-memory tree (128, 64,
+// 32 pairs) and then one warp's shuffle tree, 8 in a row.  Several values: one warp each, on different
+// quarters, 12 in a row (the tree for all of them: 8 K, most in one warp).
 // Requires blockDim.x == RED_THREADS.
 template <int K>
 __device__ __forceinline__ void block_reduce(double (&v)[K], unsigned maxmask) {
+    static_assert(K <= RED_THREADS / 32, "one warp per value");
     __shared__ double sh[K][RED_THREADS];
     const int t = threadIdx.x;
 #pragma unroll
     for (int k = 0; k < K; ++k) sh[k][t] = v[k];
     __syncthreads();
+    if (K == 1) {
 #pragma unroll
-    for (int s = RED_THREADS / 2; s >= 32; s >>= 1) {
-        if (t < s)
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                sh[k][t] = ((maxmask >> k) & 1) ? fmax(sh[k][t], sh[k][t + s]) : sh[k][t] + sh[k][t + s];
-        __syncthreads();
+        for (int s = RED_THREADS / 2; s >= 32; s >>= 1) {
+            if (t < s) sh[0][t] = (maxmask & 1) ? fmax(sh[0][t], sh[0][t + s]) : sh[0][t] + sh[0][t + s];
+            __syncthreads();
+        }
+        if (t < 32) v[0] = (maxmask & 1) ? warp_max(sh[0][t]) : warp_sum(sh[0][t]);
+        return;
     }
-    if (t < 32) {
+    const int w = t / 32, lane = t & 31;
+    if (w < K) {
+        const bool mx = (maxmask >> w) & 1;
+        double a = sh[w][lane];
 #pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = ((maxmask >> k) & 1) ? warp_max(sh[k][t]) : warp_sum(sh[k][t]);
+        for (int s = 32; s < RED_THREADS; s += 32) a = mx ? fmax(a, sh[w][lane + s]) : a + sh[w][lane + s];
+        a = mx ? warp_max(a) : warp_sum(a);
+        if (lane == 0) sh[w][0] = a;
     }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = sh[k][0];
 }
 
 // Blocks for a row-segment walk over an n1 x n2 grid: one block per segment of RED_THREADS
