@@ -8,8 +8,8 @@
 // computed again in the halo, one ring less for every colour (their values equal what the
 // neighbouring tiles compute: same inputs, same arithmetic): 30% more operations on a 16 x 32 tile.
 // FP64 is bound by its pipe (1024^2: down 39 us, up 31, at 74 and 85% of it; 43 and 41 us as
-// separate launches), FP32 by instruction issue (4096^2: 169 and 153 us; HBM alone would take 50), small
-// levels by the number of launches, two instead of eight.
+// separate launches), FP32 by instruction issue (its large levels take mgmarch.cuh), small levels by the
+// number of launches, two instead of eight.
 // Per-cell arithmetic and its order are those of k_rb_zero, k_rb_face5, k_restrict5 and
 // k_prolong_rb, so the cycle gives the same bits.
 //

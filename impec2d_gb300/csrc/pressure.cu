@@ -991,6 +991,7 @@ __global__ void k_apply_ref(Level F, const double* __restrict__ x, int pin, int 
 #include "mgfused.cuh"
 #include "mgcluster.cuh"
 #include "mglevel.cuh"
+#include "mgmarch.cuh"
 
 constexpr size_t MG_COARSE_SMEM = 160 * 1024;
 constexpr size_t MG_CLUSTER_SMEM = 200 * 1024;
@@ -1030,6 +1031,11 @@ static impec_status level_kernel_attributes() {
     IMPEC_CUDA_TRY((level_attribute<double, 16, 32>()));
     IMPEC_CUDA_TRY((level_attribute<double, 16, 16>()));
     IMPEC_CUDA_TRY((level_attribute<float, 32, 32>()));
+    const auto march = [](auto* k) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM); };
+    IMPEC_CUDA_TRY(march(k_down5_march<4>));
+    IMPEC_CUDA_TRY(march(k_down5_march<1>));
+    IMPEC_CUDA_TRY(march(k_up5_march<4>));
+    IMPEC_CUDA_TRY(march(k_up5_march<1>));
     return IMPEC_OK;
 }
 
@@ -1611,14 +1617,43 @@ static void launch_down_up(impec_ctx* ctx, Level& F, Level& C, bool down, T* xc,
         launch_k(ctx->stream, k_up5<T, TR, TC>, g, LV_T, LvTile<T, TR, TC>::SMEM, F.n1, F.n2, tx, ty, id, (const T*)b,
                  (const T*)level_alt<T>(F), x, C.n1, C.n2, (const T*)cx, level_w4<T>(C), mask, vec);
 }
+// The marching form.  Segments: as many warps as two blocks per SM hold, of at least MM_MINROWS rows (a segment
+// reads eight more than it writes).
+template <int P>
+static void launch_march(impec_ctx* ctx, Level& F, Level& C, bool down, float* xc) {
+    using T = float;
+    const T *tx, *ty, *a9, *id, *tx_, *ty_, *a9_, *id_;
+    T *x, *b, *cx, *cb;
+    level_ptrs<T>(F, tx, ty, a9, id, x, b);
+    level_ptrs<T>(C, tx_, ty_, a9_, id_, cx, cb);
+    const long strips = (F.n2 + MM_COLS - 1) / MM_COLS, warps = 2L * MM_WARPS * ctx->num_sms;
+    const long segs = max(1L, warps / strips), rows = (F.n1 + segs - 1) / segs;
+    const int H = (int)max((long)MM_MINROWS, rows + (rows & 1));
+    const long units = strips * ((F.n1 + H - 1) / H);
+    const int g = (int)((units + MM_WARPS - 1) / MM_WARPS);
+    ++ctx->nlaunch;
+    if (down)
+        launch_k(ctx->stream, k_down5_march<P>, g, 32 * MM_WARPS, MM_SMEM, F.n1, F.n2, H, tx, ty, id, level_diag<T>(F), (const T*)b,
+                 level_alt<T>(F), C.n1, C.n2, level_w4<T>(C), cb, xc);
+    else
+        launch_k(ctx->stream, k_up5_march<P>, g, 32 * MM_WARPS, MM_SMEM, F.n1, F.n2, H, tx, ty, id, (const T*)b,
+                 (const T*)level_alt<T>(F), x, C.n1, C.n2, (const T*)cx, level_w4<T>(C));
+}
+
 // Tiles (ms): FP64 16 x 32 on large levels, 16 x 16 where those leave SMs idle (1024^2 step 4.05 / 4.11
 // and 4.20 with 32 x 32; 513 x 777 nine-point step 3.07 / 2.96); FP32 32 x 32, whose halo costs less than
 // 16 x 32's (2048^2 step 7.95 / 8.14, 4096^2 solve 25.6 / 26.9) and which leaves more blocks per SM
-// than 32 x 64 (8.92, 29.1).  One launch per colour and transfer: 4.13, 3.22, 8.41, 29.0; 300 x 130
+// than 32 x 64 (8.92, 29.1).  Large FP32 levels march (mgmarch.cuh) unless cells are masked: solve of 1024^2 2.70 / 2.78,
+// 1023 x 1021 2.92 / 3.10, 2048^2 5.28 / 5.90, 4093 x 4095 16.1 / 19.9, but 722 x 721 2.46 / 2.34 and
+// 512^2 1.92 / 1.86 (segments of 16 rows read 24).  One launch per colour and transfer: 4.13, 3.22, 8.41, 29.0; 300 x 130
 // solve 1.80 against 1.53, 256^2 step 1.03 against 0.95.
 template <class T>
 static void launch_half(impec_ctx* ctx, Level& F, Level& C, bool down, T* xc, const unsigned char* mask) {
-    if constexpr (sizeof(T) == 4) launch_down_up<T, 32, 32>(ctx, F, C, down, xc, mask);
+    if constexpr (sizeof(T) == 4) {
+        if (mask || F.n() < MM_MINCELLS) launch_down_up<T, 32, 32>(ctx, F, C, down, xc, mask);
+        else if (F.n2 % 4 == 0) launch_march<4>(ctx, F, C, down, xc);
+        else launch_march<1>(ctx, F, C, down, xc);
+    }
     else if (F.n() >= (size_t)1 << 19) launch_down_up<T, 16, 32>(ctx, F, C, down, xc, mask);
     else launch_down_up<T, 16, 16>(ctx, F, C, down, xc, mask);
 }

@@ -176,6 +176,29 @@ def test_half_cycle_kernels_match_separate_launches(engine, monkeypatch, N1, N2,
     assert out[0][3] < out[1][3]
 
 
+@pytest.mark.parametrize("N1,N2", [(1001, 900), (900, 1001), (100, 8004), (101, 8001), (8001, 100), (1500, 560), (887, 1122)])
+def test_marching_half_cycles(engine, monkeypatch, N1, N2):
+    """Large FP32 levels, a warp per strip and segment (16-byte and element copies, strips and segments of
+    all remainders): the bits of one launch per colour and transfer."""
+    import torch
+
+    from helpers import dev, host
+    E = engine
+    c = np.random.default_rng(4).uniform(0.0, 1.0, (N1, N2))
+    out = []
+    for skip in ("1", "0"):
+        monkeypatch.setenv("IMPEC_MG_RB_SKIP", skip)
+        P = E.default_params(N1, N2, stype=1, nu=1.0, precision=1, max_cycles=200, x_lb=0.0, x_ub=float(N1), y_lb=0.0,
+                             y_ub=float(N2))
+        ctx = E.Context(P)
+        ctx.set_source(dev(source(oparams(P))))
+        p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+        cyc, rr, _ = ctx.pressure_solve(dev(c), p, 1e-10)
+        out.append((cyc, rr, host(p)))
+        ctx.close()
+    assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
+
+
 @pytest.mark.parametrize("N1,N2", [(2, 1025), (2, 2000), (2000, 2), (3, 1300)])
 @pytest.mark.parametrize("nu", [1.0, 0.25])
 def test_thin_grids(engine, monkeypatch, N1, N2, nu):
