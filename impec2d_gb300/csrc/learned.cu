@@ -11,6 +11,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <string>
@@ -849,6 +850,199 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv_wgrad_tma(const __grid_cons
     if (warp == 0) umma::tmem_free(tmem, 128);
 }
 
+// Weight gradient by image rows.  The unit of work is a row segment of 64 pixels; units are ordered by image, panel
+// (up to WgRows::PANEL segments side by side), row, segment, and a CTA takes a slice of them.  Each unit is
+// loaded once into a slot of a ring in shared memory: CB channels of the input's 66 pixels (the segment with one
+// pixel on either side) and CA channels of the 64 of dZ.  Slots stay until the rows above and below have
+// met them: unit u multiplies its dZ with the inputs of the units one panel row before, at and after it (the
+// vertical taps).  GEMM rows: (dx, ci) of one dy, 128 at a time, as blocks of CB channels whose starts lie one
+// pixel apart (the horizontal taps; CB = 32: three blocks and one whose results are not used; CB = 64: two, and
+// one with one unused), columns: CA output channels, K: the 64 pixels; 3 or 6 accumulators in TMEM.
+// Pixels outside the image load as zeros, which also covers segments that end beyond it; rows above and
+// below it are left out.
+//
+// Against (tap, ci) x channel tiles over a slice of the pixels (k_conv_wgrad_tma), which fetch every input row for
+// each tap and pad 32 output channels to 128: a twelfth of the loads.  What bounds it now is the MMAs, 80 to
+// 95 cycles for each 128 x CA x 16 (both operands transposed): with one thread's time, 134 while the four on one
+// accumulator followed each other, 107 with the accumulators innermost, less with descriptors moved by
+// one addition; a dozen runtime divisions per unit had cost 1,000 cycles.  Three boxes instead of one with shifted
+// starts: the same time, a third of the ring.
+//
+// Order of summation: over long slices the tensor core's truncated FP32 sums lose about 2^-24 of a sum per
+// step (4e-5 after 642 units).  CB = 32 (the widest images, so the longest slices): panels of four segments and the
+// slices of k_conv_wgrad_tma, so that the gradients stay those of its sums over images of up to 256 columns;
+// CB = 64: single segments and one wave of shorter slices (a third of the error, and every SM at work).
+//
+// 64 images of 256^2, us before / now: 32 to 32 channels 1555 / 397, 64 to 32 1961 / 396; of 128^2: 64 to 64
+// 340 / 117, 128 to 64 430 / 215; of 64^2: 256 to 128 442 / 214; 52 of 200^2, 32 to 32, whose rows
+// did not tile boxes: 1869 / 286.
+constexpr int WR_MAXSLOTS = 23, WR_XPIX = WG_PIX + 2;
+
+template <int CA, int CB>
+struct WgRows {
+    static constexpr int XLOAD = WR_XPIX * CB * 2, XB = (XLOAD + 1023) / 1024 * 1024, ZB = WG_PIX * CA * 2, SLOT = XB + ZB;  // bytes
+    static constexpr int PANEL = CB == 32 ? 4 : 1;
+    static constexpr int MT = CB / 32, ACC = 3 * MT;  // 128-row tiles per dy, accumulators
+    static constexpr uint32_t COLS = ACC * CA <= 128 ? 128 : ACC * CA <= 256 ? 256 : 512;
+    static constexpr int PAD = 8192 + 1024;  // the last tile of the last slot reads up to 8 KB past it; alignment
+};
+
+// Position of a unit (image b, panel p, row y, segment s), stepped without divisions: one thread issues all
+// copies of a CTA and one all MMAs, and a dozen runtime divisions per unit took 2,000 cycles of its time.
+struct WrUnit {
+    int b, p, y, s;
+    __device__ __forceinline__ WrUnit(int u, int H, int ps, int panels) {
+        const int row = u / ps, bp = row / H;
+        s = u - row * ps;
+        y = row - bp * H;
+        b = bp / panels;
+        p = bp - b * panels;
+    }
+    __device__ __forceinline__ void next(int H, int ps, int panels) {
+        if (++s < ps) return;
+        s = 0;
+        if (++y < H) return;
+        y = 0;
+        if (++p < panels) return;
+        p = 0;
+        ++b;
+    }
+};
+// A position in the ring.
+struct WrSlot {
+    int slot, use;
+    __device__ __forceinline__ void next(int slots) {
+        if (++slot == slots) slot = 0, ++use;
+    }
+};
+
+template <int CA, int CB>
+__global__ void __launch_bounds__(WG_THREADS) k_conv_wgrad_rows(const __grid_constant__ CUtensorMap tz,
+                                                                const __grid_constant__ CUtensorMap tx, int H, int ps,
+                                                                int panels, int cin, int cout, int Kp, int units, int per,
+                                                                int slots, float* __restrict__ dW, int* __restrict__ err) {
+    using G = WgRows<CA, CB>;
+    extern __shared__ __align__(1024) unsigned char wr_smem[];
+    __shared__ uint64_t full[WR_MAXSLOTS], empty[WR_MAXSLOTS], done;
+    __shared__ uint32_t tslot;
+    __shared__ volatile int fail, tma_issued, used;  // used: the dy whose accumulators were written
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c0 = blockIdx.x * CB, n0 = blockIdx.y * CA;
+    const int ua = blockIdx.z * per, ub = min(ua + per, units);
+    const int va = max(ua - ps, 0), vb = min(ub + ps, units);  // units whose slots the slice reads
+    unsigned char* base = wr_smem + ((1024 - (umma::smem_u32(wr_smem) & 1023)) & 1023);
+    if (warp == 0) umma::tmem_alloc(&tslot, G::COLS);
+    if (tid == 0) {
+        for (int st = 0; st < slots; ++st) {
+            umma::mbar_init(&full[st], 1);
+            umma::mbar_init(&empty[st], 1);
+        }
+        umma::mbar_init(&done, 1);
+        fail = 0;
+        tma_issued = 0;
+        used = 0;
+    }
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const uint32_t tmem = tslot;
+    if (warp == 4) {
+        if (lane == 0) {  // TMA producer
+            WrUnit w(va, H, ps, panels);
+            WrSlot q{0, 0};
+            for (int v = va; v < vb; ++v, w.next(H, ps, panels), q.next(slots)) {
+                if (q.use > 0 && !umma::mbar_wait(&empty[q.slot], (uint32_t)((q.use - 1) & 1), GB_WAIT_TRIES)) {
+                    fail = 1;
+                    break;
+                }
+                unsigned char* sp = base + q.slot * G::SLOT;
+                const int x0 = (w.p * ps + w.s) * WG_PIX;
+                umma::mbar_expect_tx(&full[q.slot], (uint32_t)(G::XLOAD + G::ZB));
+                umma::tma_load_4d(sp, &tx, c0, x0 - 1, w.y, w.b, &full[q.slot]);
+                umma::tma_load_4d(sp + G::XB, &tz, n0, x0, w.y, w.b, &full[q.slot]);
+                tma_issued = v - va + 1;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        if (lane == 0) {  // MMA issuer
+            constexpr uint32_t idesc = umma::idesc_bf16_f32_mn(128, CA);
+            // descriptors: the halves that stay, and the first slot's start addresses, to which offsets / 16 are added
+            const uint64_t ad0 = umma::smem_desc_mn(umma::smem_u32(base), CB * 2, 8 * CB * 2, CB * 2);
+            const uint64_t bd0 = umma::smem_desc_mn(umma::smem_u32(base) + G::XB, G::ZB, 8 * CA * 2, CA * 2);
+            const uint32_t a0 = (uint32_t)ad0, ahi = (uint32_t)(ad0 >> 32), b0 = (uint32_t)bd0, bhi = (uint32_t)(bd0 >> 32);
+            WrUnit w(ua, H, ps, panels);
+            WrSlot land{0, 0};            // the next slot to land
+            int ready = 0, mask = 0;      // slots that have landed; dy whose accumulators hold a sum
+            int at = ua - va, above = 0, below = ua - va + ps;  // slots of units u, u - ps (from u = va + ps on), u + ps
+            bool ok = true;
+            for (int u = ua; u < ub; ++u, w.next(H, ps, panels)) {
+                const int need = min(u + ps, vb - 1) - va;
+                for (; ready <= need && ok; ++ready, land.next(slots))
+                    ok = umma::mbar_wait(&full[land.slot], (uint32_t)(land.use & 1), GB_WAIT_TRIES);
+                if (!ok) break;
+                umma::fence_after();
+                const uint32_t sx[3] = {a0 + (uint32_t)above * (G::SLOT / 16), a0 + (uint32_t)at * (G::SLOT / 16),
+                                        a0 + (uint32_t)below * (G::SLOT / 16)};
+                const uint32_t sz = b0 + (uint32_t)at * (G::SLOT / 16);
+                const int on = (w.y > 0 ? 1 : 0) | 2 | (w.y + 1 < H ? 4 : 0);
+                // accumulators innermost: an MMA waits for the one before it on the same accumulator
+#pragma unroll
+                for (int ks = 0; ks < WG_PIX / 16; ++ks)  // 16 pixels = two 8-row K groups
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy) {
+                        if (!((on >> dy) & 1)) continue;
+                        const uint32_t acc = ks > 0 ? 1u : (uint32_t)(mask >> dy) & 1u;
+#pragma unroll
+                        for (int t = 0; t < G::MT; ++t)
+                            umma::mma_bf16(tmem + (uint32_t)((dy * G::MT + t) * CA), umma::desc(sx[dy] + (t * 2 + ks * 16) * CB * 2 / 16, ahi),
+                                           umma::desc(sz + ks * 16 * CA * 2 / 16, bhi), idesc, acc);
+                    }
+                mask |= on;
+                if (u - ps >= va) {
+                    umma::commit(&empty[above]);
+                    above = above + 1 == slots ? 0 : above + 1;
+                }
+                at = at + 1 == slots ? 0 : at + 1;
+                below = below + 1 == slots ? 0 : below + 1;
+            }
+            if (!ok) fail = 1;
+            // no load of this CTA outlives it (bounded)
+            for (; ready < tma_issued; ++ready, land.next(slots)) umma::mbar_wait(&full[land.slot], (uint32_t)(land.use & 1), GB_WAIT_TRIES >> 4);
+            used = mask;
+            umma::commit(&done);
+        }
+        __syncwarp();
+    }
+    const bool fin = warp < 4 && ub > ua ? umma::mbar_wait(&done, 0u, GB_WAIT_TRIES) : true;
+    const bool ok = __syncthreads_and(fin) != 0 && fail == 0;
+    if (ok && ub > ua && warp < 4) {
+        umma::fence_after();
+        const int m = warp * 32 + lane;
+#pragma unroll 1
+        for (int g = 0; g < G::ACC; ++g) {
+            const int dy = g / G::MT, dx = g % G::MT * 2 + m / CB, ci = c0 + m % CB, k = (dy * 3 + dx) * cin + ci;
+            if (!((used >> dy) & 1)) continue;
+#pragma unroll 1
+            for (int h = 0; h < CA / 32; ++h) {
+                float v[32];
+                umma::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(g * CA + h * 32), v);
+                if (dx > 2 || ci >= cin) continue;
+#pragma unroll
+                for (int n = 0; n < 32; ++n) {
+                    const int co = n0 + h * 32 + n;
+                    if (co < cout) atomicAdd(dW + (size_t)co * Kp + k, v[n]);
+                }
+            }
+        }
+    }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    if (warp == 0) umma::tmem_free(tmem, G::COLS);
+}
+
 void launch_wt_transpose(const __nv_bfloat16* W, int cin, int cout, __nv_bfloat16* Wd, cudaStream_t s) {
     k_conv_wt_transpose<<<128, 256, 0, s>>>(W, cin, cout, conv_kp(cin), Wd, conv_kp(cout));
 }
@@ -1073,22 +1267,20 @@ impec_status launch_conv(const ConvArgs& a, cudaStream_t s) {
     return launch_conv_any<32>(a, s);
 }
 
-// Boxes of 64 pixels: whole rows (W a multiple of 64) or whole-row groups of one image, as in
-// conv_tma_plan; cin and cout multiples of 32; P a multiple of 64.
-static bool wgrad_tma_plan(int B, int H, int W, int cin, int cout, int* wb, int* hb, int* bb) {
+// Whether TMA boxes fit the operands of a weight gradient.
+static bool wgrad_boxes_ok(int cin, int cout) {
     static const bool off = [] {
         const char* e = getenv("IMPEC_CONV_TMA");
         return e && e[0] == '0';
     }();
-    if (off || (cin % 32 && cin != 8) || (cout % 32 && cout != 8) || ((long long)B * H * W) % WG_PIX ||
-        !tmap_encoder())
-        return false;
-    if (W >= WG_PIX) {
-        if (W % WG_PIX) return false;
-        *wb = WG_PIX, *hb = 1, *bb = 1;
-        return true;
-    }
-    if (WG_PIX % W) return false;
+    return !off && (cin % 32 == 0 || cin == 8) && (cout % 32 == 0 || cout == 8) && tmap_encoder();
+}
+
+// Boxes of 64 pixels of several rows or images (k_conv_wgrad_tma), for images of at most 16 columns that
+// tile them; all other images go by rows, whose segments of 64 columns are mostly empty there.  64 images,
+// us by boxes / by rows: 32^2, 32 to 32 channels 63 / 50, 256 to 256 256 / 247; 16^2: 44 / 37 and 110 / 161.
+static bool wgrad_tma_plan(int B, int H, int W, int cin, int cout, int* wb, int* hb, int* bb) {
+    if (!wgrad_boxes_ok(cin, cout) || W > 16 || WG_PIX % W || ((long long)B * H * W) % WG_PIX) return false;
     const int r = WG_PIX / W;
     *wb = W;
     if (r >= H) {
@@ -1145,11 +1337,60 @@ static impec_status launch_wgrad_tma(const __nv_bfloat16* dZ, const __nv_bfloat1
     return IMPEC_OK;
 }
 
+template <int CA, int CB>
+static impec_status launch_wgrad_rows(const __nv_bfloat16* dZ, const __nv_bfloat16* X, int B, int H, int W_, int cin,
+                                      int cout, float* dW, int* err, int num_sms, cudaStream_t s) {
+    using G = WgRows<CA, CB>;
+    constexpr int SMEM = 216 * 1024;
+    static bool attr = false;
+    if (!attr) {
+        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv_wgrad_rows<CA, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        attr = true;
+    }
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    auto encode = [&](CUtensorMap* m, const void* p, int c, int box, int pix) {
+        const cuuint64_t d[4] = {(cuuint64_t)c, (cuuint64_t)W_, (cuuint64_t)H, (cuuint64_t)B};
+        const cuuint64_t st[3] = {(cuuint64_t)c * 2, (cuuint64_t)W_ * c * 2, (cuuint64_t)H * W_ * c * 2};
+        const cuuint32_t bx[4] = {(cuuint32_t)box, (cuuint32_t)pix, 1, 1};
+        return tmap_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)p, d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              box == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    CUtensorMap tz, tx;
+    if (!encode(&tz, dZ, cout, CA, WG_PIX) || !encode(&tx, X, cin, CB, WR_XPIX)) {
+        set_error("wgrad: cuTensorMapEncodeTiled failed");
+        return IMPEC_ERR_CUDA;
+    }
+    const int gx = (cin + CB - 1) / CB, gy = (cout + CA - 1) / CA, strips = (W_ + WG_PIX - 1) / WG_PIX;
+    const int panels = (strips + G::PANEL - 1) / G::PANEL, ps = (strips + panels - 1) / panels;
+    const int units = B * panels * H * ps;
+    int splits = std::max(1, num_sms / (gx * gy));
+    if (CB == 32) {  // as launch_wgrad_tma's
+        const int tiles = (cin >= CB ? (9 * cin + 127) / 128 : (9 + 128 / CB - 1) / (128 / CB)) * ((cout + 127) / 128);
+        splits = (2 * num_sms + tiles - 1) / tiles;
+    }
+    const int per = (units + splits - 1) / splits;
+    const dim3 g(gx, gy, (units + per - 1) / per);
+    const int slots = std::min(WR_MAXSLOTS, (SMEM - G::PAD) / G::SLOT);  // at least 2 ps + 2
+    static_assert((SMEM - G::PAD) / G::SLOT >= 2 * G::PANEL + 2, "a unit's window and one slot more");
+    k_conv_wgrad_rows<CA, CB><<<g, WG_THREADS, slots * G::SLOT + G::PAD, s>>>(tz, tx, H, ps, panels, cin, cout, conv_kp(cin),
+                                                                            units, per, slots, dW, err);
+    IMPEC_CUDA_TRY(cudaGetLastError());
+    return IMPEC_OK;
+}
+
 impec_status launch_wgrad(const __nv_bfloat16* dZ, const __nv_bfloat16* X, int B, int H, int W_, int cin, int cout,
                           float* dW, int* err, int num_sms, cudaStream_t s) {
     int wb, hb, bb;
-    if (wgrad_tma_plan(B, H, W_, cin, cout, &wb, &hb, &bb)) {
-        const bool a64 = cout % 64 == 0, b64 = cin % 64 == 0;  // 8-channel operands take 32-channel boxes
+    const bool a64 = cout % 64 == 0, b64 = cin % 64 == 0;  // 8-channel operands take 32-channel boxes
+    const bool boxes = wgrad_tma_plan(B, H, W_, cin, cout, &wb, &hb, &bb);
+    if (wgrad_boxes_ok(cin, cout) && !boxes) {
+        if (a64 && b64) return launch_wgrad_rows<64, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);
+        if (a64) return launch_wgrad_rows<64, 32>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);
+        if (b64) return launch_wgrad_rows<32, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);
+        return launch_wgrad_rows<32, 32>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);
+    }
+    if (boxes) {
         if (a64 && b64) return launch_wgrad_tma<64, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, wb, hb, bb, s);
         if (a64) return launch_wgrad_tma<64, 32>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, wb, hb, bb, s);
         if (b64) return launch_wgrad_tma<32, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, wb, hb, bb, s);

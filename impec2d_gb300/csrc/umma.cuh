@@ -60,6 +60,9 @@ __device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t lbo, u
     return d;
 }
 
+// A descriptor from its halves; the low one may be moved by (byte offset / 16).
+__device__ __forceinline__ uint64_t desc(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
+
 // Instruction descriptor of kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9 and
 // 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
