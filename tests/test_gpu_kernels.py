@@ -271,3 +271,32 @@ def test_weight_gradient_by_rows(engine, B, H, W, cin, cout):
         y, x = divmod(tap, 3)
         ref[:, tap * cin:(tap + 1) * cin] = dz.T @ xp[:, y:y + H, x:x + W].reshape(-1, cin)
     assert (dW.double() - ref).abs().max().item() <= 2e-5 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("B,H,W", [(3, 8, 8), (2, 8, 72), (2, 40, 24)])
+def test_net_gradients_of_batches(engine, B, H, W):
+    """Pooling, upsampling and their gradients over batches and images that are not square: the gradients
+    of a batch are the mean of its images' from the CPU restatement, with that comparison's tolerance
+    (bf16 rounding of every stored activation)."""
+    import torch
+
+    from oracle import learned_ref as R
+    E = engine
+    net = E.Net(seed=3)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    X = torch.zeros((B, H, W, 8), device="cuda")
+    X[..., :4] = torch.randn((B, H, W, 4), generator=g, device="cuda")
+    X = X.to(torch.bfloat16)
+    T = torch.randn((B, H, W), generator=g, device="cuda")
+    loss = net.backprop(X, T)
+    grads, params = net.parameters(which=1), net.parameters(which=0)
+    refs = [R.forward_backward(params, X[b].float().cpu().numpy(), T[b].cpu().numpy()) for b in range(B)]
+    loss_ref, grads_ref = np.mean([r[0] for r in refs]), np.mean([r[1] for r in refs], axis=0)
+    assert abs(loss - loss_ref) <= 1e-3 * abs(loss_ref)
+    off = 0
+    for cin, cout, *_ in R.LAYERS:
+        n = cout * R.kp(cin) + cout
+        a, b = grads[off:off + n], grads_ref[off:off + n]
+        assert np.linalg.norm(a - b) <= 3e-2 * np.linalg.norm(b) + 1e-12
+        off += n
+    net.close()
