@@ -300,3 +300,25 @@ def test_net_gradients_of_batches(engine, B, H, W):
         assert np.linalg.norm(a - b) <= 3e-2 * np.linalg.norm(b) + 1e-12
         off += n
     net.close()
+
+
+@pytest.mark.parametrize("N1,N2", [(2, 2), (3, 257), (129, 65), (700, 513)])
+def test_diagnostics_on_the_edges(engine, N1, N2):
+    """Mass, flux through the boundary faces, extremes of both signs and a NaN that the extremes pass over:
+    sums of at most 4e5 terms of the order of one, 1e-12 relative."""
+    from helpers import dev
+    E = engine
+    ctx = E.Context(E.default_params(N1, N2, stype=1))
+    rng = np.random.default_rng(N1)
+    c, u, v = rng.normal(size=(N1, N2)), rng.normal(size=(N1 + 1, N2)), rng.normal(size=(N1, N2 + 1))
+    be = np.abs(u[0]).sum() + np.abs(u[-1]).sum() + np.abs(v[:, 0]).sum() + np.abs(v[:, -1]).sum()
+    d = ctx.diagnostics(dev(c), dev(u), dev(v))
+    assert d[3] == c.max() and d[4] == c.min()
+    assert abs(d[2] - be) <= 1e-12 * be
+    for s in (1.0, -1.0):  # one sign only
+        d = ctx.diagnostics(dev(s * np.abs(c)), dev(u), dev(v))
+        assert d[3] == (s * np.abs(c)).max() and d[4] == (s * np.abs(c)).min()
+    c[0, 0] = np.nan
+    d = ctx.diagnostics(dev(c), dev(u), dev(v))
+    assert d[3] == np.nanmax(c) and d[4] == np.nanmin(c)
+    ctx.close()
