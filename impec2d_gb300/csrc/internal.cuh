@@ -102,11 +102,11 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-bool pdl_enabled();  // programmatic launches only with IMPEC_PDL=1
+bool pdl_enabled();  // programmatic launches throughout with IMPEC_PDL=1, else where the code asks for them
 
-// kernel<<<g, b, smem, s>>>(args...) with the programmatic-serialisation attribute.
+// kernel<<<g, b, smem, s>>>(args...), with pdl with the programmatic-serialisation attribute.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(cudaStream_t s, void (*k)(KArgs...), dim3 g, dim3 b, size_t smem, Args&&... args) {
+inline cudaError_t launch_ks(bool pdl, cudaStream_t s, void (*k)(KArgs...), dim3 g, dim3 b, size_t smem, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
     cfg.blockDim = b;
@@ -116,8 +116,12 @@ inline cudaError_t launch_k(cudaStream_t s, void (*k)(KArgs...), dim3 g, dim3 b,
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k(cudaStream_t s, void (*k)(KArgs...), dim3 g, dim3 b, size_t smem, Args&&... args) {
+    return launch_ks(pdl_enabled(), s, k, g, b, smem, std::forward<Args>(args)...);
 }
 
 // Device-resident scalars of a step (so a step needs no host round trip).

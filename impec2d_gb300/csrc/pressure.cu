@@ -2173,25 +2173,29 @@ impec_status pressure_iteration(impec_ctx* ctx, double tol, cudaGraphConditional
     // whose block sums are overhead (1024^2: 17.6 us with 2, 19.6 with 4, 23.6 with 8); the update by
     // HBM (15.8 us with 4, 18.6 with 8), the direction by it too (4096^2 FP32: 53 us with 4, 44 with 8).
     const auto vblocks = [&](int per_sm) { return flat_blocks((n + 1) / 2, min(ctx->num_sms * per_sm, ctx->max_blocks)); };
+    // On small grids an iteration's vector kernels are short beside the launches between them, which programmatic
+    // serialisation overlaps; on larger ones the waiting blocks take the running kernel's places (us without / with:
+    // 128^2 step 1007 / 990, 300 x 130 solve 1520 / 1415, 256^2 step 918 / 929, 513 x 777 step 2820 / 2970).
+    const bool pdl = pdl_enabled() || n < (size_t)3 << 14;
     const auto dots = [&](auto kernel, auto* zz) {
         ++ctx->nlaunch;
-        launch_k(ctx->stream, kernel, vblocks(2), RED_THREADS, 0, n, (const double*)r, zz, (const double*)ctx->cg_q, ctx->partials,
+        launch_ks(pdl, ctx->stream, kernel, vblocks(2), RED_THREADS, 0, n, (const double*)r, zz, (const double*)ctx->cg_q, ctx->partials,
                  ctx->max_blocks, ctx->counter, &S->pcg_rz, S);
     };
     if (mixed) dots(ctx->singular ? k_cg_dots<4, float> : k_cg_dots<2, float>, z32);
     else dots(ctx->singular ? k_cg_dots<4, double> : k_cg_dots<2, double>, z);
     ++ctx->nlaunch;
-    if (mixed) launch_k(ctx->stream, k_cg_direction<float>, vblocks(8), 256, 0, n, z32, ctx->cg_p, (const DevScalars*)S);
-    else launch_k(ctx->stream, k_cg_direction<double>, vblocks(8), 256, 0, n, z, ctx->cg_p, (const DevScalars*)S);
+    if (mixed) launch_ks(pdl, ctx->stream, k_cg_direction<float>, vblocks(8), 256, 0, n, z32, ctx->cg_p, (const DevScalars*)S);
+    else launch_ks(pdl, ctx->stream, k_cg_direction<double>, vblocks(8), 256, 0, n, z, ctx->cg_p, (const DevScalars*)S);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_apply, blocks, RED_THREADS, 0, F, ctx->cg_p, ctx->cg_q, ctx->partials,
+    launch_ks(pdl, ctx->stream, k_cg_apply, blocks, RED_THREADS, 0, F, ctx->cg_p, ctx->cg_q, ctx->partials,
              ctx->max_blocks, ctx->counter, &S->pcg_pq, S);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_update, vblocks(4), RED_THREADS, 0, n, ctx->cg_x, r, mixed ? F.b32 : nullptr,
+    launch_ks(pdl, ctx->stream, k_cg_update, vblocks(4), RED_THREADS, 0, n, ctx->cg_x, r, mixed ? F.b32 : nullptr,
              (const double*)ctx->cg_p, (const double*)ctx->cg_q, (size_t)pin_index(ctx), S, ctx->partials, ctx->max_blocks,
              ctx->counter, &S->rnorm2, tol, ctx->P.max_cycles, h, 0);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_verify, blocks, RED_THREADS, 0, F, (const double*)ctx->f, (const double*)ctx->cg_x,
+    launch_ks(pdl, ctx->stream, k_cg_verify, blocks, RED_THREADS, 0, F, (const double*)ctx->f, (const double*)ctx->cg_x,
              pin_index(ctx), mixed ? F.b32 : nullptr, r, S, ctx->partials, ctx->max_blocks, ctx->counter, tol,
              ctx->P.max_cycles, h, use_h);
     IMPEC_LAUNCH_CHECK();
