@@ -159,8 +159,8 @@ def time_kernel(ctx, which: int, reps: int = 20):
 
 def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = None, traffic_path: str | None = None,
                    reps: int = 20):
-    """Achieved bandwidth of the dominant kernel, the fine-level red-black sweep, against the
-    measured HBM copy bandwidth, and its FP64 operation rate against the measured DFMA rate.
+    """Achieved bandwidth of a red-black sweep of the finest level (two colours by the per-level sweep
+    kernels; inside a CG solve the half-cycle kernels do the same arithmetic) against the measured HBM copy bandwidth, and its FP64 operation rate against the measured DFMA rate.
     Each repetition is timed cold: L2 is overwritten first (``flush``, a CUDA tensor larger
     than L2), then CUDA events on the engine's stream bracket the sweep.  Algorithmic bytes
     follow the five-point model: x read and written, b, and the two face planes (40 B per cell in
@@ -168,10 +168,12 @@ def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = 
     profiles/traffic.json when that file names the kernel and grid."""
     import json
     which = 1 if precision == "mixed" else 0
-    if P.nu != 1.0:  # nine-point operator: four-colour sweeps, timed back to back
+    if P.nu != 1.0:  # nine-point operator, timed back to back: its own levels or the five-point hierarchy's
         ms, b = time_kernel(ctx, which)
         t = "double" if which == 0 else "float"
-        return {"bound": "hbm", "kernel": f"k_gs4_exp9<{t}> (fine four-colour GS sweep, nine-point)",
+        planes9 = round(b / (P.N1 * P.N2 * (8 if which == 0 else 4))) == 13
+        return {"bound": "hbm", "kernel": f"k_gs4_exp9<{t}> (fine four-colour GS sweep, nine-point)" if planes9
+                else f"k_rb_face5<{t}> (fine red-black sweep of the five-point hierarchy)",
                 "grid": f"{P.N1}x{P.N2}", "achieved": b / (ms * 1e-3) / 1e9, "peak": 6800.0, "unit": "GB/s",
                 "frac": b / (ms * 1e-3) / 1e9 / 6800.0, "peak_source": "fallback", "bytes_per_launch": b,
                 "ms_per_launch": ms, "timing": "back-to-back launches", "traffic": None}

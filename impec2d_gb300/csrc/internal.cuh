@@ -148,9 +148,9 @@ namespace impec {
 struct LearnedHook;  // learned_net.cu
 
 struct Tuning {
-    // Smoother sweeps before / after the coarse correction: V(1,2) for five-point operators
-    // (1024^2 IMPES step 3.19 ms against 3.32 ms with V(2,2), 10 instead of 9 iterations;
-    // at 4096^2 on heterogeneous fields the FP64 solve ties), V(1,1) for nine-point ones.
+    // Smoother sweeps before / after the coarse correction, V(1,2) for five-point operators (as three
+    // colours on either side: pressure.cu, Colours), V(1,1) for nine-point ones.  Measured with
+    // separate launches: 1024^2 step 3.19 ms against 3.32 with V(2,2), 10 instead of 9 iterations.
     long pre = 1, post = 2;
     long cluster = 1;              // coarse levels in one thread-block-cluster launch
     long cl_cells = 16384;         // largest level of the cluster V-cycle
@@ -159,15 +159,13 @@ struct Tuning {
     long coarse_cells32 = 1024;    // the same, FP32
     long rb_skip = 1;  // five-point levels: no zero fill before pre-smoothing, red-only prolongation
     long rb_resid = 1;  // five-point levels: restriction sums the red residuals only (black ones are ~0)
-    // FP64 five-point levels of at least this many cells sweep both colours in one launch
-    // (k_rb_tile, ping-pong iterate): every coefficient is read once per sweep instead of once
-    // per colour, which pays where the level streams from HBM (4096^2 sweep 185 against 240 us
-    // cold; 4096^2 solve 17.9 ms with 2048^2 and 4096^2 levels so swept, 18.0 with 4096^2
-    // alone, 19.7 with none) and costs where it sits in L2 (1024^2 solve 2.23 against 2.08 ms
-    // with every level so swept: the recomputed ring and one more dependent phase); 0 disables
+    // FP64 five-point levels of at least this many cells sweep both colours in one launch (k_rb_tile,
+    // ping-pong iterate) where a half cycle is not one launch anyway (pressure.cu, fused_level: CG with
+    // the default schedule): every coefficient is read once per sweep instead of once per colour, which
+    // pays where the level streams from HBM (4096^2 sweep 185 against 240 us cold) and costs where it sits
+    // in L2 (1024^2 solve 2.23 against 2.08 ms with every level so swept); 0 disables
     long tile_cells = 1L << 22;
-    // the same for FP32 levels (mixed precision): 4096^2 cold sweep 110 against 130 us, mixed
-    // solve 14.35 against 14.44 ms; with every level so swept the 1024^2 solve is 12% slower
+    // the same for FP32 levels (mixed precision): 4096^2 cold sweep 110 against 130 us
     long tile_cells32 = 1L << 22;
 };
 }  // namespace impec

@@ -1324,8 +1324,6 @@ void swap_iterate<float>(Level& Lv) { std::swap(Lv.x32, Lv.xa32); }
 // if each V-cycle starts the level from a write that reads no old iterate: true for the coarse
 // levels and, with CG, for the finest level (its cycles start from x = 0); the stationary
 // iteration's finest level, which corrects the solution in place, keeps the two-launch sweep.
-// FP64 only: the FP32 sweeps of the mixed-precision cycle measured no faster in one launch
-// (4096^2: 133 against 131 us cold).
 template <class T>
 static bool use_tile(impec_ctx* ctx, size_t l) {
     Level& Lv = ctx->L[l];
@@ -1761,10 +1759,10 @@ __global__ void k_mg_check(DevScalars* S, double tol, int max_cycles, int inc, c
 // ---------------------------------------------------------------- V-cycle preconditioned CG
 // The reference solves the pressure system with CG preconditioned by HYPRE's SMG
 // (src/MGSolver.cpp:594-629); here the preconditioner is one V-cycle of the engine's own
-// multigrid (V(1,2) for five-point, V(1,1) for nine-point operators by default), z = M^-1 r, in
+// multigrid (three colours on either side for five-point, V(1,1) for nine-point levels by default), z = M^-1 r, in
 // FP64 or (mixed precision) in FP32 on the FP32 copy of r.  CG runs in FP64 on the consistent
-// singular system.  Because neither a cycle with unequal pre- and post-smoothing nor the FP32
-// cycle is a symmetric operator, the direction uses the flexible (Polak-Ribiere) coefficient
+// singular system.  Because the FP32 cycle is not quite a symmetric operator (nor is a cycle of
+// another schedule), the direction uses the flexible (Polak-Ribiere) coefficient
 //   beta = (z_k, r_k - r_{k-1}) / (z_{k-1}, r_{k-1}) = -alpha_{k-1} (z_k, A p_{k-1}) / (z_{k-1}, r_{k-1}),
 // which needs only (z, r) and (z, q) with q = A p still holding the previous direction.
 
@@ -2445,7 +2443,7 @@ extern "C" impec_status impec_time_kernel(impec_ctx* ctx, int which, int reps, d
         switch (which) {
             case 0: F.kind == FACE5 ? smooth<double>(ctx, F, 2, 0) : smooth9<double>(ctx, F, 1, false); b = n * 8 * (4 + coef); break;  // x,b,idiag r + x w + operator
             case 1: F.kind == FACE5 ? smooth<float>(ctx, F, 2, 0) : smooth9<float>(ctx, F, 1, false); b = n * 4 * (4 + coef); break;
-            case 2: IMPEC_TRY(pressure_residual(ctx)); b = n * 8 * (2 + coef) + (ctx->P.precision ? 4 * n : 0); break;
+            case 2: IMPEC_TRY(pressure_residual(ctx)); b = n * 8 * (F.a9 ? 11 : 4) + (ctx->P.precision ? 4 * n : 0); break;
             case 3: IMPEC_TRY(advect_x_dev(ctx, ctx->c, ctx->t1, ctx->u, 1.0, &ctx->dscal->dt)); b = n * 24; break;
             case 4: IMPEC_TRY(advect_y_dev(ctx, ctx->c, ctx->t1, ctx->v, 1.0, &ctx->dscal->dt)); b = n * 24; break;
         }

@@ -195,7 +195,8 @@ impec_status impec_project_diagonal(impec_ctx* ctx, int field, double* out_dev, 
 impec_status impec_project_diagonal_download(impec_ctx* ctx, int field, double* out_host, int d_N1, int d_N2);
 
 /* Engine tunables of a context (no counterpart in the reference): "mg_pre", "mg_post" (smoother
- * sweeps before / after the coarse correction, 0..8, sum >= 1), "cluster" (0/1: coarse levels in
+ * sweeps before / after the coarse correction, 0..8, sum >= 1; five-point levels with
+ * mg_post = mg_pre + 1 split their colours evenly between the two sides), "cluster" (0/1: coarse levels in
  * one thread-block-cluster launch), "cluster_cells", "cluster_cta0", "coarse_cells64",
  * "coarse_cells32" (level-size thresholds).  Defaults come from the IMPEC_MG_* environment at
  * context creation.  Changing a value drops the captured graphs. */
