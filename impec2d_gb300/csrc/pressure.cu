@@ -1762,7 +1762,7 @@ __global__ void k_mg_check(DevScalars* S, double tol, int max_cycles, int inc, c
 // multigrid (three colours on either side for five-point, V(1,1) for nine-point levels by default), z = M^-1 r, in
 // FP64 or (mixed precision) in FP32 on the FP32 copy of r.  CG runs in FP64 on the consistent
 // singular system.  Because the FP32 cycle is not quite a symmetric operator (nor is a cycle of
-// another schedule), the direction uses the flexible (Polak-Ribiere) coefficient
+// another schedule), the direction uses the flexible (Polak-Ribiere) coefficient there
 //   beta = (z_k, r_k - r_{k-1}) / (z_{k-1}, r_{k-1}) = -alpha_{k-1} (z_k, A p_{k-1}) / (z_{k-1}, r_{k-1}),
 // which needs only (z, r) and (z, q) with q = A p still holding the previous direction.
 
@@ -1801,21 +1801,24 @@ __device__ __forceinline__ float2 load_pair(const float* p, size_t k) { return r
 __device__ __forceinline__ double wide(double v) { return v; }
 __device__ __forceinline__ double wide(float v) { return widen(v); }
 
-// (r, z) and (z, q) into out[0], out[1].  With S (CG, out = &S->pcg_rz), the last block also
+// (r, z) and, unless SYM, (z, q) into out[0], out[1].  With S (CG, out = &S->pcg_rz), the last block also
 // stores the direction's beta = -alpha_old (z, q) / (z, r)_old (0 on the first iteration).
-// K = 4 (singular systems): also the sums of z and r, with which (r, z) is taken without either's
+// SING (singular systems): also the sums of z and r, with which (r, z) is taken without either's
 // mean.  The rounded rows of the operator do not quite sum to zero, so r has a small mean that
 // no direction removes; the cycle answers it with a far larger mean of z (four times the
 // right-hand side per cell on each coarser level), and their product came to outweigh the rest of
 // (r, z): past its best iterate CG then diverged (1024^2, nu = 2/3: from 8e-11 of ||f|| to 1e-6 in
 // five iterations).  An FP32 z is summed in FP32 over a thread's 2 CG_U values at a time, whose
 // rounding is that of the values themselves.
-template <int K, class Z>
+// SYM (a symmetric cycle: FP64 five-point levels with as many colours on either side, no masked cells): beta =
+// (r, z) / (r, z)_old, to which the flexible coefficient then reduces, without q (1024^2: 17.1 -> 14.7 us).
+template <bool SING, bool SYM, class Z>
 __global__ void __launch_bounds__(RED_THREADS) k_cg_dots(size_t n, const double* __restrict__ r,
-                                                            const Z* __restrict__ z, const double* __restrict__ q,
-                                                            double* partials, int mb, unsigned* counter, double* out,
-                                                            DevScalars* S) {
+                                                         const Z* __restrict__ z, const double* __restrict__ q,
+                                                         double* partials, int mb, unsigned* counter, double* out,
+                                                         DevScalars* S) {
     pdl_enter();
+    constexpr int ZS = SYM ? 1 : 2, K = ZS + (SING ? 2 : 0);  // (r, z), (z, q) unless SYM, sums of z and r
     double acc[K];
 #pragma unroll
     for (int e = 0; e < K; ++e) acc[e] = 0.0;
@@ -1827,37 +1830,38 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_dots(size_t n, const double*
         for (int e = 0; e < U; ++e) {
             rr[e] = load_pair(r, k0 + e * step);
             zz[e] = load_pair(z, k0 + e * step);
-            qq[e] = load_pair(q, k0 + e * step);
+            if (!SYM) qq[e] = load_pair(q, k0 + e * step);
         }
         Z zs = 0;
 #pragma unroll
         for (int e = 0; e < U; ++e) {
             const double z0 = wide(zz[e].x), z1 = wide(zz[e].y);
             acc[0] += rr[e].x * z0;
-            acc[1] += z0 * qq[e].x;
+            if (!SYM) acc[ZS - 1] += z0 * qq[e].x;
             acc[0] += rr[e].y * z1;
-            acc[1] += z1 * qq[e].y;
-            if (K == 4) {
+            if (!SYM) acc[ZS - 1] += z1 * qq[e].y;
+            if (SING) {
                 zs = e == 0 ? zz[e].x + zz[e].y : zs + (zz[e].x + zz[e].y);
                 acc[K - 1] += rr[e].x;
                 acc[K - 1] += rr[e].y;
             }
         }
-        if (K == 4) acc[K - 2] += wide(zs);
+        if (SING) acc[K - 2] += wide(zs);
     });
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
         const double z0 = wide(z[n - 1]), r0 = r[n - 1];
         acc[0] += r0 * z0;
-        acc[1] += z0 * q[n - 1];
-        if (K == 4) {
+        if (!SYM) acc[ZS - 1] += z0 * q[n - 1];
+        if (SING) {
             acc[K - 2] += z0;
             acc[K - 1] += r0;
         }
     }
     if (grid_reduce<K>(acc, 0u, partials, mb, counter, out) && threadIdx.x == 0 && S) {
-        if (K == 4) S->pcg_rz -= S->pcg_zsum * S->pcg_rsum / (double)n;
+        double rz = out[0];
+        if (SING) S->pcg_rz = rz -= out[K - 2] * out[K - 1] / (double)n;
         const bool first = S->mg_cycles == 0 || S->pcg_rz_old == 0.0;
-        S->pcg_beta = first ? 0.0 : -S->pcg_alpha * S->pcg_zq / S->pcg_rz_old;
+        S->pcg_beta = first ? 0.0 : (SYM ? rz : -S->pcg_alpha * out[ZS - 1]) / S->pcg_rz_old;
     }
 }
 
@@ -2070,7 +2074,7 @@ static impec_status learned_guess(impec_ctx* ctx, double* x) {
     launch_k(ctx->stream, k_cg_apply, blocks, RED_THREADS, 0, F, (const double*)ctx->lrn_d, ctx->lrn_Ad, ctx->partials,
              ctx->max_blocks, ctx->counter, &S->pcg_pq, (DevScalars*)nullptr);
     ++ctx->nlaunch;
-    launch_k(ctx->stream, k_cg_dots<2, double>, flat_blocks((F.n() + 1) / 2, cap), RED_THREADS, 0, F.n(),
+    launch_k(ctx->stream, k_cg_dots<false, false, double>, flat_blocks((F.n() + 1) / 2, cap), RED_THREADS, 0, F.n(),
              (const double*)ctx->lrn_r0, (const double*)ctx->lrn_d, (const double*)ctx->lrn_Ad, ctx->partials, ctx->max_blocks, ctx->counter, &S->pcg_rz, (DevScalars*)nullptr);
     ++ctx->nlaunch;
     launch_k(ctx->stream, k_learn_step, ctx->num_sms * 4, 256, 0, F.n(), x, (const double*)ctx->lrn_d,
@@ -2180,8 +2184,10 @@ impec_status pressure_iteration(impec_ctx* ctx, double tol, cudaGraphConditional
         launch_ks(pdl, ctx->stream, kernel, vblocks(2), RED_THREADS, 0, n, (const double*)r, zz, (const double*)ctx->cg_q, ctx->partials,
                  ctx->max_blocks, ctx->counter, &S->pcg_rz, S);
     };
-    if (mixed) dots(ctx->singular ? k_cg_dots<4, float> : k_cg_dots<2, float>, z32);
-    else dots(ctx->singular ? k_cg_dots<4, double> : k_cg_dots<2, double>, z);
+    const Colours col = colours(ctx);
+    if (mixed) dots(ctx->singular ? k_cg_dots<true, false, float> : k_cg_dots<false, false, float>, z32);
+    else if (ctx->singular && F.kind == FACE5 && col.npre == col.npost) dots(k_cg_dots<true, true, double>, z);
+    else dots(ctx->singular ? k_cg_dots<true, false, double> : k_cg_dots<false, false, double>, z);
     ++ctx->nlaunch;
     if (mixed) launch_ks(pdl, ctx->stream, k_cg_direction<float>, vblocks(8), 256, 0, n, z32, ctx->cg_p, (const DevScalars*)S);
     else launch_ks(pdl, ctx->stream, k_cg_direction<double>, vblocks(8), 256, 0, n, z, ctx->cg_p, (const DevScalars*)S);
