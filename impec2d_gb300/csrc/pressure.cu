@@ -199,15 +199,28 @@ __constant__ int c_off[9][2] = {{0, 0}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}, {1,
 // ---------------------------------------------------------------- coarse operators
 // Five-point coarsening, 2 x 2 cells to one.  A coarse face carries the flux that two coarse cell
 // centres drive through what lies between them: the two fine faces on the interface (conductance
-// s, in parallel) in series with half of each cell's inside, h = 1 / (2 t_in), t_in the sum of
-// the two fine faces inside the cell in that direction:
+// s, in parallel) in series with the part h of either cell's inside that lies on its way:
 //   t = s / (1 + s (h_lo + h_hi)).
-// On a uniform grid that is the rediscretised face (s = 2, h = 1/4, t = 1); across a jump of the
+// t_in is the sum of the two fine faces inside the cell in that direction.  The inside is split between
+// its two sides: half and half in the ordinary case, but where one pair of children conducts far
+// better than the other (CO_MIX) the coarse value is that pair's, and the other side's way takes it
+// all.  t_in counts as a hundredth of what both pairs conduct across at least (CO_DETOUR), a way round
+// the inside through the next cells.  With h = 1 / (2 t_in) alone, a cell on the edge of a nearly
+// impermeable inclusion had hardly any coupling left, although half of it belongs to the well
+// conducting surroundings, and CG hung.  Iterations to 1e-9, FP64, with the half sums and bilinear
+// transfers of plain, with even splits, and now: inclusions of 1e-10 on 64^2 22 / over 400 / 11 and on
+// 130 x 900 36 / over 400 / 25; barriers of 1e-8 crossed by a channel of 1e4, 64^2, 41 / 261 / 13; 15% of the
+// cells at 1e-6, 64^2, 69 / 140 / 22; cells at exp(3 N(0,1)), 513 x 512, 229 / 249 / 67; K11 and K22
+// independent at exp(1.5 N), 513 x 512, 234 / 86 / 101.
+// On a uniform grid the face is the rediscretised one (s = 2, h = 1/4, t = 1); across a jump of the
 // mobility it keeps the harmonic mean that the sum of the fine faces loses.  The same quantities
-// give the transfer weights w = h t <= 1 of a coarse cell towards its four neighbours (planes E, W,
-// N, S): a child's value is the coarse one plus w times the difference to the neighbour on its
-// side, the pressure that the flux t (x_nb - x) loses over the child's half of the cell
-// (prolong5), and the restriction is that interpolation's transpose (k_restrict5).  With symmetric
+// give the transfer weights w = h t <= 1 of a coarse cell towards its four neighbours
+// (planes E, W, N, S): a child's value is the coarse one plus w times the difference to the neighbour on its
+// side, the pressure that the flux t (x_nb - x) loses over the child's side of the cell
+// (prolong5), and the restriction is that interpolation's transpose (k_restrict5).  A child takes one
+// weight in either direction; where two of them add up to more than 1 (children cut off from each
+// other) they are scaled to 1 in the ratio of w / (1 - w), since the child would otherwise take a negative
+// multiple of a value that hardly couples to anything.  With symmetric
 // smoothing the cycle is then symmetric, as CG wants it.  CG iterations to 1e-10 with these
 // coarse operators and transfers against half the sum of the fine faces with bilinear
 // interpolation: 24 -> 14 on a 1024^2 front (M = 41), 52 -> 17 on a 4096^2 lognormal field.
@@ -217,8 +230,12 @@ __constant__ int c_off[9][2] = {{0, 0}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}, {1,
 //
 // A block owns 32 x 8 coarse cells: h of the cells and a one-cell ring in shared memory, then
 // each face of the tile once, then weights, diagonal and 1/diagonal from those faces.  FP64-bound
-// (five divisions per coarse cell).
+// (seven divisions per coarse cell).
 constexpr int CO_C = 32, CO_R = 8;
+// The children's conductances a, b count as a + CO_MIX min(a, b) and b + CO_MIX min(a, b) in the split: contrasts below
+// some ten leave it near one half, where the transfers are exact for linear pressures.
+constexpr double CO_MIX = 10.0;
+constexpr double CO_DETOUR = 0.01;
 __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, const double* __restrict__ txf,
                                                           const double* __restrict__ tyf, int n1c, int n2c,
                                                           double* __restrict__ txc, double* __restrict__ tyc,
@@ -228,7 +245,8 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
                                                           float* __restrict__ diag32, float* __restrict__ idiag32,
                                                           int plain) {
     pdl_enter();
-    __shared__ double hx[CO_R + 2][CO_C], hy[CO_R][CO_C + 2];      // cells (I0 - 1 + r, J0 + q), (I0 + r, J0 - 1 + q)
+    // cells (I0 - 1 + r, J0 + q), (I0 + r, J0 - 1 + q): towards the lower and the higher index
+    __shared__ double hx0[CO_R + 2][CO_C], hx1[CO_R + 2][CO_C], hy0[CO_R][CO_C + 2], hy1[CO_R][CO_C + 2];
     __shared__ double cx[CO_R + 1][CO_C], cy[CO_R][CO_C + 1];      // faces (I0 + r, J0 + q)
     const int t = threadIdx.y * CO_C + threadIdx.x, I0 = blockIdx.y * CO_R, J0 = blockIdx.x * CO_C;
     // fine faces in pairs (the second of a pair may lie outside an odd grid)
@@ -242,14 +260,43 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
         if (2 * I + 1 < n1f) v += tyf[IX(2 * I + 1, fj, n2f + 1)];
         return v;
     };
-    auto half = [&](double in) { return in > 0.0 && !plain ? fmin(0.5 / in, 1e300) : 0.0; };
+    // all three faces across one fine row (column) of a coarse cell
+    auto row_y = [&](int i, int J) {
+        double v = tyf[IX(i, 2 * J, n2f + 1)] + tyf[IX(i, 2 * J + 1, n2f + 1)];
+        if (2 * J + 1 < n2f) v += tyf[IX(i, 2 * J + 2, n2f + 1)];
+        return v;
+    };
+    auto col_x = [&](int I, int j) {
+        double v = txf[IX(2 * I, j, n2f)] + txf[IX(2 * I + 1, j, n2f)];
+        if (2 * I + 1 < n1f) v += txf[IX(2 * I + 2, j, n2f)];
+        return v;
+    };
+    // The inside between children that conduct b0, b1 outwards and t0, t1 across: the parts towards either
+    // side.  One without any conductance counts as none: beyond it lie dead cells, or a known row, whose
+    // couplings are on the diagonal.
+    auto split = [&](double in, double b0, double t0, double b1, double t1, double& h0, double& h1) {
+        if (!(in > 0.0)) return;
+        const double a0 = b0 + t0, a1 = b1 + t1, m = CO_MIX * fmin(a0, a1), s0 = a0 + m, s1 = a1 + m;
+        const double g = fmin(1.0 / fmax(CO_DETOUR * fmin(t0, t1), in), 1e300);
+        const double part = s0 + s1 > 1e-290 ? 1.0 / (s0 + s1) : 0.0;
+        h0 = part > 0.0 ? s1 * part * g : 0.5 * g;
+        h1 = part > 0.0 ? s0 * part * g : 0.5 * g;
+    };
     for (int k = t; k < (CO_R + 2) * CO_C; k += CO_C * CO_R) {
         const int r = k / CO_C, q = k % CO_C, I = I0 - 1 + r, J = J0 + q;
-        hx[r][q] = I >= 0 && J < n2c && 2 * I + 1 < n1f ? half(pair_x(2 * I + 1, J)) : 0.0;
+        double h0 = 0.0, h1 = 0.0;
+        if (!plain && I >= 0 && J < n2c && 2 * I + 1 < n1f)
+            split(pair_x(2 * I + 1, J), pair_x(2 * I, J), row_y(2 * I, J), pair_x(2 * I + 2, J), row_y(2 * I + 1, J), h0, h1);
+        hx0[r][q] = h0;
+        hx1[r][q] = h1;
     }
     for (int k = t; k < CO_R * (CO_C + 2); k += CO_C * CO_R) {
         const int r = k / (CO_C + 2), q = k % (CO_C + 2), I = I0 + r, J = J0 - 1 + q;
-        hy[r][q] = J >= 0 && I < n1c && 2 * J + 1 < n2f ? half(pair_y(I, 2 * J + 1)) : 0.0;
+        double h0 = 0.0, h1 = 0.0;
+        if (!plain && J >= 0 && I < n1c && 2 * J + 1 < n2f)
+            split(pair_y(I, 2 * J + 1), pair_y(I, 2 * J), col_x(I, 2 * J), pair_y(I, 2 * J + 2), col_x(I, 2 * J + 1), h0, h1);
+        hy0[r][q] = h0;
+        hy1[r][q] = h1;
     }
     __syncthreads();
     for (int k = t; k < (CO_R + 1) * CO_C; k += CO_C * CO_R) {
@@ -258,7 +305,7 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
         if (I <= n1c && J < n2c) {
             if (I > 0 && I < n1c) {
                 const double a = pair_x(2 * I, J);
-                v = plain ? 0.5 * a : a / (1.0 + a * (hx[r][q] + hx[r + 1][q]));
+                v = plain ? 0.5 * a : a / (1.0 + a * (hx1[r][q] + hx0[r + 1][q]));
             }
             if (r < CO_R || I == n1c) {  // the face below the tile belongs to the next tile, except the last one
                 txc[IX(I, J, n2c)] = v;
@@ -273,7 +320,7 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
         if (I < n1c && J <= n2c) {
             if (J > 0 && J < n2c) {
                 const double a = pair_y(I, 2 * J);
-                v = plain ? 0.5 * a : a / (1.0 + a * (hy[r][q] + hy[r][q + 1]));
+                v = plain ? 0.5 * a : a / (1.0 + a * (hy1[r][q] + hy0[r][q + 1]));
             }
             if (q < CO_C || J == n2c) {
                 tyc[IX(I, J, n2c + 1)] = v;
@@ -286,12 +333,20 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
     const int r = threadIdx.y, q = threadIdx.x, I = I0 + r, J = J0 + q;
     if (I >= n1c || J >= n2c) return;
     const size_t n = (size_t)n1c * n2c, k = IX(I, J, n2c);
-    const double w[4] = {hx[r + 1][q] * cx[r + 1][q], hx[r + 1][q] * cx[r][q], hy[r][q + 1] * cy[r][q + 1],
-                         hy[r][q + 1] * cy[r][q]};
+    if (w4) {
+        double w[4] = {hx1[r + 1][q] * cx[r + 1][q], hx0[r + 1][q] * cx[r][q], hy1[r][q + 1] * cy[r][q + 1],
+                       hy0[r][q + 1] * cy[r][q]};
+        const double X = fmax(w[0], w[1]), Y = fmax(w[2], w[3]);
+        if (X + Y > 1.0) {
+            const double x = fmax(1.0 - X, 1e-300), y = fmax(1.0 - Y, 1e-300), d = fma(X, y, Y * x);
+            const double fx = y / d, fy = x / d;  // X fx : Y fy = X / (1 - X) : Y / (1 - Y)
+            w[0] *= fx; w[1] *= fx; w[2] *= fy; w[3] *= fy;
+        }
 #pragma unroll
-    for (int e = 0; e < 4 && w4; ++e) {
-        w4[e * n + k] = w[e];
-        if (w432) w432[e * n + k] = (float)w[e];
+        for (int e = 0; e < 4; ++e) {
+            w4[e * n + k] = w[e];
+            if (w432) w432[e * n + k] = (float)w[e];
+        }
     }
     if (diag) store_diag5(k, cx[r][q], cx[r + 1][q], cy[r][q], cy[r][q + 1], diag, idiag, diag32, idiag32);
 }

@@ -322,3 +322,36 @@ def test_diagnostics_on_the_edges(engine, N1, N2):
     d = ctx.diagnostics(dev(c), dev(u), dev(v))
     assert d[3] == np.nanmax(c) and d[4] == np.nanmin(c)
     ctx.close()
+
+
+@pytest.mark.parametrize("N1,N2", [(64, 64), (65, 130), (130, 300)])
+@pytest.mark.parametrize("kind", ["inclusions", "closed", "barriers"])
+@pytest.mark.parametrize("nu", [1.0, 2.0 / 3.0])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_contrasts_inside_coarse_cells(engine, N1, N2, kind, nu, prec):
+    """Nearly impermeable and impermeable inclusions, and thin barriers crossed by a channel: coarse cells
+    that hold both sides of a contrast, on all levels.  CG in 64-bit numpy with these coarse operators takes 10
+    to 12 iterations to 1e-9 on the five-point systems; twice as many are allowed for FP32 cycles and for the
+    nine-point operator's condition number of 1 / nu."""
+    import torch
+
+    from helpers import dev
+    E = engine
+    i, j = np.arange(N1)[:, None], np.arange(N2)[None, :]
+    K = np.ones((N1, N2))
+    if kind == "barriers":
+        K[N1 // 3, :N2 * 2 // 3] = 1e-8
+        K[N1 // 5:N1 // 3, N2 // 2] = 1e-6
+        K[:, N2 // 4] = 1e4
+    else:
+        K[np.sin(0.37 * i) * np.cos(0.29 * j) > 0.5] = 1e-10 if kind == "inclusions" else 0.0
+        K[:3, :3] = K[-3:, -3:] = 1.0
+    P = E.default_params(N1, N2, stype=1, nu=nu, precision=prec, max_cycles=24, x_lb=0.0, x_ub=float(N1), y_lb=0.0,
+                         y_ub=float(N2))
+    ctx = E.Context(P)
+    ctx.set_source(dev(source(oparams(P))))
+    ctx.set_permeability(dev(K), dev(K))
+    p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+    cyc, rr, _ = ctx.pressure_solve(dev(np.zeros((N1, N2))), p, 1e-9)
+    assert rr <= 1e-9, (cyc, rr)
+    ctx.close()
