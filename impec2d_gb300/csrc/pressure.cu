@@ -2046,6 +2046,7 @@ __device__ __forceinline__ void true_check(DevScalars* S, double tol, int max_cy
     if (bad) S->flags |= FLAG_MG_NAN;
     if (!bad && !go && rr > tol) S->flags |= FLAG_MG_NOT_CONVERGED;
     else S->flags &= ~FLAG_MG_NOT_CONVERGED;
+    if (go) S->pcg_rz_old = 0.0;  // the next direction is z alone (k_cg_dots, k_cg_direction)
     S->go = go ? 1 : 0;
     if (use_h) cudaGraphSetConditional(h, go ? 1u : 0u);
 }
@@ -2053,9 +2054,13 @@ __device__ __forceinline__ void true_check(DevScalars* S, double tol, int max_cy
 // End of a CG pass, after k_cg_update, whose check set S->go from the recurrence residual.
 // That residual drifts from the true one by rounding, so a stop (converged, max_cycles or a
 // breakdown) is verified here: the true residual f - A x of the final iterate replaces r (and
-// its FP32 copy), its norm gives the reported relres, and CG continues from it while it is
-// above tol and cycles remain.  On the other passes the kernel only hands S->go to the WHILE
-// condition.  Every thread reads S->go before the last block (the only writer) can change it.
+// its FP32 copy), its norm gives the reported relres, and CG starts again from it while it is
+// above tol and cycles remain: the last direction is conjugate for the residual that was replaced, and
+// (r, z) / (r, z)_old of two unrelated residuals is no coefficient.  Carried on with it, solves asked for a
+// little less than FP64 gives drifted away from their floor (130 x 900, K22 = K11 / 100: from 1.2e-9
+// to 1.1e-4 in 400 iterations); after a breakdown the direction that had failed came back.
+// On the other passes the kernel only hands S->go to the WHILE condition.  Every thread reads
+// S->go before the last block (the only writer) can change it.
 __global__ void __launch_bounds__(RED_THREADS) k_cg_verify(Level F, const double* __restrict__ f,
                                                            const double* __restrict__ x, int pin,
                                                            float* __restrict__ r32, double* __restrict__ r64,

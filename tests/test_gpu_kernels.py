@@ -355,3 +355,34 @@ def test_contrasts_inside_coarse_cells(engine, N1, N2, kind, nu, prec):
     cyc, rr, _ = ctx.pressure_solve(dev(np.zeros((N1, N2))), p, 1e-9)
     assert rr <= 1e-9, (cyc, rr)
     ctx.close()
+
+
+@pytest.mark.parametrize("N1,N2,aniso", [(130, 900, 0.01), (96, 700, 0.02), (200, 200, 0.01)])
+@pytest.mark.parametrize("nu", [1.0, 0.9])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_cg_stays_at_its_floor_when_the_residual_is_replaced(engine, N1, N2, aniso, nu, prec):
+    """A tolerance a little below what FP64 gives: the recurrence residual passes it again and again, and
+    each time the true residual takes its place.  CG must go on from there, not from a search direction that
+    belongs to the old residual: 400 iterations leave the residual within ten times of its floor (the smallest that
+    solves of 60 to 160 iterations reach)."""
+    import torch
+
+    from helpers import dev
+    E = engine
+    i, j = np.arange(N1)[:, None], np.arange(N2)[None, :]
+    K = np.exp(0.7 * np.sin(0.21 * i + 0.05 * j) * np.cos(0.17 * j))
+    c = 1.0 / (1.0 + np.exp((np.hypot(i, j) - 0.35 * math.hypot(N1, N2)) / 3.0))
+
+    def solve(tol, cycles):
+        P = E.default_params(N1, N2, stype=1, nu=nu, precision=prec, max_cycles=cycles, x_lb=0.0, x_ub=float(N1), y_lb=0.0,
+                             y_ub=float(N2))
+        ctx = E.Context(P)
+        ctx.set_source(dev(source(oparams(P))))
+        ctx.set_permeability(dev(K), dev(aniso * K))
+        p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+        rr = ctx.pressure_solve(dev(c), p, tol, check=False)[1]
+        ctx.close()
+        return rr
+    floor = min(solve(1e-16, n) for n in (60, 90, 120, 160))
+    for part in (0.9, 0.75, 0.6, 0.4):
+        assert solve(part * floor, 400) <= 10.0 * floor, part
