@@ -153,21 +153,22 @@ __global__ void __launch_bounds__(RED_THREADS) k_cn_rhs(int n1, int n2, const do
     grid_reduce<1>(acc, 0u, partials, mb, counter, out);
 }
 
-// Two colours of a four-colour Gauss-Seidel sweep, the even and then the odd columns of the rows of
-// one parity.  Rows of one parity do not couple, so a block takes whole rows and orders the two
-// colours with its own barrier: two launches per sweep instead of four, and each plane's sectors,
-// which hold both column parities, are read once instead of twice (1024^2, a sweep: 40 us before, 29
-// now).
+// Colours of a four-colour Gauss-Seidel sweep on the rows of one parity: the even columns, the odd ones, or
+// (both) one after the other.  Rows of one parity do not couple, so a block that takes whole rows
+// orders the two colours with its own barrier: two launches per sweep instead of four, and each
+// plane's sectors, which hold both column parities, are read once instead of twice (1024^2, a
+// sweep: 40 us before, 29 now).  Few long rows make too few blocks for that; there each colour is a launch whose
+// blocks share a row (gridDim.y of them; cn_iteration).
 constexpr int GS_T = 256;
 __global__ void __launch_bounds__(GS_T) k_cn_gs(int n1, int n2, const double* __restrict__ a9,
                                                 const double* __restrict__ idiag, const double* __restrict__ b, double* x,
-                                                int parity) {
+                                                int parity, int first, int last) {
     pdl_enter();
     const int i = 2 * blockIdx.x + parity;
     if (i >= n1) return;
-    for (int cj = 0; cj < 2; ++cj) {
-        if (cj) __syncthreads();
-        for (int j = 2 * threadIdx.x + cj; j < n2; j += 2 * GS_T) {
+    for (int cj = first; cj <= last; ++cj) {
+        if (cj > first) __syncthreads();
+        for (int j = 2 * (blockIdx.y * GS_T + threadIdx.x) + cj; j < n2; j += 2 * GS_T * gridDim.y) {
             const size_t k = IX(i, j, n2);
             x[k] = (b[k] - cn_off(i, j, n1, n2, a9, x)) * idiag[k];
         }
@@ -248,10 +249,21 @@ impec_status cn_check(impec_ctx* ctx, double tol, int inc, cudaGraphConditionalH
 // differs) followed by the new residual (launch only).
 impec_status cn_iteration(impec_ctx* ctx, double* x) {
     const int n1 = ctx->P.N1, n2 = ctx->P.N2, cap = red_cap(ctx->num_sms, ctx->max_blocks);
-    for (int parity = 0; parity < 2; ++parity) {
+    const auto colours = [&](int parity, int first, int last, int blocks) {
         ++ctx->nlaunch;
-        launch_k(ctx->stream, k_cn_gs, (n1 + 1 - parity) / 2, GS_T, 0, n1, n2, (const double*)ctx->cn_a9,
-                 (const double*)ctx->cn_idiag, (const double*)ctx->cn_b, x, parity);
+        launch_k(ctx->stream, k_cn_gs, dim3((n1 + 1 - parity) / 2, blocks), GS_T, 0, n1, n2, (const double*)ctx->cn_a9,
+                 (const double*)ctx->cn_idiag, (const double*)ctx->cn_b, x, parity, first, last);
+    };
+    // Rows shared by several blocks where whole rows would leave SMs idle (us of a solve of three sweeps, whole rows /
+    // shared: 4 x 65536 1935 / 313, 64 x 16384 1002 / 443, 128 x 8192 673 / 446, 304 x 8192 1166 / 848, 512 x 2048
+    // 448 / 437; but 608 x 2048 486 / 493, 1400 x 4096 1776 / 1789, 256 x 1024 230 / 262).
+    const bool shared = n2 >= 2048 && n1 <= 4 * ctx->num_sms;
+    for (int parity = 0; parity < 2; ++parity) {
+        if (shared) {
+            for (int cj = 0; cj < 2; ++cj) colours(parity, cj, cj, (n2 + 2 * GS_T - 1) / (2 * GS_T));
+        } else {
+            colours(parity, 0, 1, 1);
+        }
     }
     ++ctx->nlaunch;
     launch_k(ctx->stream, k_cn_resid, seg_blocks(n1, n2, cap), RED_THREADS, 0, n1, n2, (const double*)ctx->cn_a9,

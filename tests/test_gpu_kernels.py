@@ -386,3 +386,40 @@ def test_cg_stays_at_its_floor_when_the_residual_is_replaced(engine, N1, N2, ani
     floor = min(solve(1e-16, n) for n in (60, 90, 120, 160))
     for part in (0.9, 0.75, 0.6, 0.4):
         assert solve(part * floor, 400) <= 10.0 * floor, part
+
+
+@pytest.mark.parametrize("N1,N2", [(2, 2048), (5, 2049), (3, 2561)])
+def test_cn_sweep_on_few_long_rows(engine, oracle_lib, N1, N2):
+    """Few long rows: each colour of a sweep is a launch of its own whose blocks share the rows (two launches more
+    per sweep than on a short grid).  The same comparison as test_cn_half_step_at_tile_edges, for the same reasons."""
+    import ctypes as C
+
+    import oracle as O
+    from helpers import cell_ghost, dev, host, smooth_field, vel_split
+    E = engine
+
+    def launches(N1, N2):
+        P = E.default_params(N1, N2, diffusion=1, alpha_l=0.5, alpha_t=0.05, Dm=1e-3, para_eps=1e-13, max_cycles=400,
+                             x_lb=0.0, x_ub=float(N1), y_lb=0.0, y_ub=float(N2))
+        OP = oparams(P)
+        v = np.zeros(O.vel_shape(OP))
+        c = np.random.default_rng(6).uniform(0.0, 1.0, (N1, N2))
+        cg = cell_ghost(OP, c)
+        p = smooth_field(N1, N2, 9, -1.0, 1.0) * 0.05
+        oracle_lib.or_calc_velocities(C.byref(OP), O.ptr(cell_ghost(OP, p)), O.ptr(v), O.ptr(cg))
+        u, vv = vel_split(OP, v)
+        dt = 0.5 * oracle_lib.or_max_stable_dt(C.byref(OP), O.ptr(v))
+        its, rr = C.c_int(), C.c_double()
+        assert oracle_lib.or_cn_solve(C.byref(OP), O.ptr(cg), O.ptr(v), dt, 0, 1e-14, C.byref(its), C.byref(rr)) == 0
+        ctx = E.Context(P)
+        d = dev(c)
+        n0 = E.launch_count(ctx)
+        sweeps, rr_d = ctx.dispersion_cn(d, dev(u), dev(vv), dt, 1e-13)
+        n = E.launch_count(ctx) - n0
+        ctx.close()
+        ref = O.interior(OP, cg)
+        assert rr_d <= 1e-13 and np.linalg.norm(host(d) - ref) <= 1e-12 * np.linalg.norm(ref)
+        return n, sweeps
+    n, sweeps = launches(N1, N2)
+    m, short = launches(N1, 64)
+    assert (n - 2) / sweeps == (m - 2) / short + 2  # beside the matrix and the right-hand side
