@@ -246,7 +246,7 @@ struct TileArgs {
 };
 
 // One strip: out[k] = new value of cell k (cells at c + k cs, faces at W + k ws, E at e + k cs', F as W).
-// c[-2 .. 9], W[0 .. 8], E[-1 .. 8], F[0 .. 8] are read.
+// c[-2 .. STRIP + 1], W[0 .. STRIP], E[-1 .. STRIP], F[0 .. STRIP] are read.
 template <int SCHEME>
 __device__ __forceinline__ void sweep_strip(const double* c, int cs, const double* W, const double* E, const double* F,
                                             int ws, double (&out)[STRIP]) {
@@ -438,11 +438,18 @@ static cudaError_t launch_tile(cudaStream_t s, TileArgs A, bool edges) {
     return launch_k(s, k_advect_tile<SCHEME, BC, MODE, TI>, g, Tile<TI, MODE>::THREADS, Tile<TI, MODE>::SMEM, A);
 }
 
+// Tiles of 8 rows instead of 32: where those of 32 would leave SMs without one (symmetric MUSCL, us of a
+// call, 8 / 32 rows: 256^2 36 / 38, 400 x 300 42 / 38, for more of the first sweeps is halo), and where
+// their last rows would be a quarter or more of the grid's tiles beyond it (8 x 16384 42 / 75, 16 x 16384 54 / 75,
+// 33 x 4096 46 / 50, 48 x 4096 50 / 50; WAF 102 / 225, 158 / 258, 121 / 142, 138 / 142; but 96 x 4096 69 / 64).
+static bool tiles_of_8(int n1, int n2) {
+    const int rows8 = (n1 + 7) / 8 * 8, rows32 = (n1 + 31) / 32 * 32;
+    return (size_t)n1 * n2 < 98304 || 3 * (long)rows32 >= 4 * (long)rows8;
+}
+
 template <int SCHEME, int MODE>
 static cudaError_t launch_tile_bc(int bc, cudaStream_t s, const TileArgs& A, bool edges) {
-    // tiles of 8 rows where those of 32 would leave SMs without one (symmetric MUSCL, a call: 256^2 29
-    // against 33 us, 400 x 300 36 against 34: more of the first sweeps is halo)
-    const bool small = (size_t)A.n1 * A.n2 < 98304;
+    const bool small = tiles_of_8(A.n1, A.n2);
     if (bc == IMPEC_BC_PERIODIC)
         return small ? launch_tile<SCHEME, IMPEC_BC_PERIODIC, MODE, 8>(s, A, edges)
                      : launch_tile<SCHEME, IMPEC_BC_PERIODIC, MODE, 32>(s, A, edges);
@@ -548,22 +555,26 @@ static impec_status sweep_cells(impec_ctx* ctx, bool x, const double* cin, doubl
 // 22 / 27; Strang 35 / 41; 256^2: 27 / 27, 43 / 42; 512^2: 48 / 38, 82 / 58).  Upwind sweeps have so
 // little to compute that the tile's copy back costs more than the second launch up to 2^20 cells
 // (512^2: 24 / 26; 1024^2: 42 / 39), in Strang's three tile launches up to 2^18 (360^2: 33 / 34;
-// 512^2: 37 / 36).
+// 512^2: 37 / 36).  Rows of the last tiles that lie beyond the grid count against tiles (33 x 2000, WAF:
+// 49 / 53); grids of five or fewer rows always go cell by cell (4 x 65536: 53 / 64, Strang 93 / 106, WAF
+// 105 / 140 and 188 / 302).
 static bool by_cells(const impec_params& P) {
-    const size_t n = (size_t)P.N1 * P.N2;
+    const size_t n = (size_t)P.N1 * P.N2, rows8 = (size_t)(P.N1 + 7) / 8 * 8;
     const bool upwind = P.hmtype != IMPEC_MUSCL && P.hmtype != IMPEC_WAFSPLIT && P.hmtype != IMPEC_WAF;
-    return n < (size_t)1 << (!upwind ? 16 : P.dim_splitting == IMPEC_STRANG ? 18 : 20);
+    return 2 * rows8 > 3 * (size_t)P.N1 || n * P.N1 < rows8 << (!upwind ? 16 : P.dim_splitting == IMPEC_STRANG ? 18 : 20);
 }
+// A single sweep: also wherever its tiles would be of 8 rows (33 x 4096, X: 32 / 31, WAF 46 / 52; 256^2 28 / 29, 34 / 37).
+static bool sweep_by_cells(const impec_params& P) { return by_cells(P) || tiles_of_8(P.N1, P.N2); }
 
 impec_status advect_x_dev(impec_ctx* ctx, const double* cin, double* cout, const double* u, double dt_scale,
                           const double* dt_dev) {
-    if (by_cells(ctx->P)) return sweep_cells(ctx, true, cin, cout, u, dt_scale, dt_dev);
+    if (sweep_by_cells(ctx->P)) return sweep_cells(ctx, true, cin, cout, u, dt_scale, dt_dev);
     return advect_tiles<MODE_X>(ctx, cin, cout, u, nullptr, dt_scale, 0.0, dt_dev);
 }
 
 impec_status advect_y_dev(impec_ctx* ctx, const double* cin, double* cout, const double* v, double dt_scale,
                           const double* dt_dev) {
-    if (by_cells(ctx->P)) return sweep_cells(ctx, false, cin, cout, v, dt_scale, dt_dev);
+    if (sweep_by_cells(ctx->P)) return sweep_cells(ctx, false, cin, cout, v, dt_scale, dt_dev);
     return advect_tiles<MODE_Y>(ctx, cin, cout, nullptr, v, 0.0, dt_scale, dt_dev);
 }
 

@@ -423,3 +423,42 @@ def test_cn_sweep_on_few_long_rows(engine, oracle_lib, N1, N2):
     n, sweeps = launches(N1, N2)
     m, short = launches(N1, 64)
     assert (n - 2) / sweeps == (m - 2) / short + 2  # beside the matrix and the right-hand side
+
+
+@pytest.mark.parametrize("N1,N2,launches", [(4, 20000, 2), (5, 13200, 2), (6, 14000, 2), (8, 13000, 1), (33, 2010, 2), (40, 2500, 1),
+                                            (24, 4100, 1), (7000, 24, 1)])
+@pytest.mark.parametrize("scheme", [4, 1])  # MUSCL, WAF split
+def test_sweeps_of_thin_grids(engine, oracle_lib, N1, N2, launches, scheme):
+    """Grids of few rows: X, then Y cell by cell (two launches) where the tiles' rows would lie beyond the
+    grid for the most part, else tiles of 8 rows; Strang, symmetric and single sweeps take the same rules.  Against the
+    oracle, with the tolerance of test_sweep_tiles for its reasons (the single sweeps against each other: 1e-13 too)."""
+    import ctypes as C
+
+    import oracle as O
+    from helpers import cell_ghost, dev, host, rel_err, smooth_field, vel_split
+    E = engine
+    c = np.random.default_rng(5).uniform(0.0, 1.0, (N1, N2))
+    p = smooth_field(N1, N2, 9, -1.0, 1.0) * 0.05
+    for mode in (1, 3, 4):  # X first, Strang, symmetric
+        P = E.default_params(N1, N2, hmtype=scheme, dim_splitting=mode, porosity=0.7)
+        OP = oparams(P)
+        v = np.zeros(O.vel_shape(OP))
+        cg = cell_ghost(OP, c)
+        oracle_lib.or_calc_velocities(C.byref(OP), O.ptr(cell_ghost(OP, p)), O.ptr(v), O.ptr(cg))
+        u, vv = vel_split(OP, v)
+        dt = 0.8 * oracle_lib.or_max_stable_advection_dt(C.byref(OP), O.ptr(v)) * OP.porosity
+        pfs = C.c_int(1)
+        oracle_lib.or_advect_split(C.byref(OP), O.ptr(cg), O.ptr(v), dt, C.byref(pfs))
+        ctx = E.Context(P)
+        d = dev(c)
+        n0 = E.launch_count(ctx)
+        ctx.advect_split(d, dev(u), dev(vv), dt, 1)
+        n = E.launch_count(ctx) - n0
+        assert rel_err(host(d), O.interior(OP, cg)) <= 1e-13
+        if mode == 1:
+            assert n == launches
+            s = dev(c)
+            ctx.advect_x(s, dev(u), dt)
+            ctx.advect_y(s, dev(vv), dt)
+            assert rel_err(host(s), host(d)) <= 1e-13
+        ctx.close()
