@@ -1277,8 +1277,8 @@ static bool wgrad_boxes_ok(int cin, int cout) {
 }
 
 // Boxes of 64 pixels of several rows or images (k_conv_wgrad_tma), for images of at most 16 columns that
-// tile them; all other images go by rows, whose segments of 64 columns are mostly empty there.  64 images,
-// us by boxes / by rows: 32^2, 32 to 32 channels 63 / 50, 256 to 256 256 / 247; 16^2: 44 / 37 and 110 / 161.
+// tile them; other images of more than six columns go by rows, whose segments of 64 columns are mostly
+// empty there.  64 images, us by boxes / by rows: 32^2, 32 to 32 channels 63 / 50, 256 to 256 256 / 247; 16^2: 44 / 37 and 110 / 161.
 static bool wgrad_tma_plan(int B, int H, int W, int cin, int cout, int* wb, int* hb, int* bb) {
     if (!wgrad_boxes_ok(cin, cout) || W > 16 || WG_PIX % W || ((long long)B * H * W) % WG_PIX) return false;
     const int r = WG_PIX / W;
@@ -1384,7 +1384,10 @@ impec_status launch_wgrad(const __nv_bfloat16* dZ, const __nv_bfloat16* X, int B
     int wb, hb, bb;
     const bool a64 = cout % 64 == 0, b64 = cin % 64 == 0;  // 8-channel operands take 32-channel boxes
     const bool boxes = wgrad_tma_plan(B, H, W_, cin, cout, &wb, &hb, &bb);
-    if (wgrad_boxes_ok(cin, cout) && !boxes) {
+    // Rows of at most six columns fill less than a tenth of their segments: the general kernel, whose units are
+    // 64 pixels in a row (us, by rows / general: 64 images of 33 x 3, 8 to 32 channels 46 / 36, 256 to 256 257 / 144;
+    // 256 of 40 x 6, 32 to 128 162 / 122, 256 to 256 1071 / 861; but 64 of 33 x 7, 128 to 64 62 / 82, 256 to 256 251 / 246).
+    if (wgrad_boxes_ok(cin, cout) && !boxes && W_ > 6) {
         if (a64 && b64) return launch_wgrad_rows<64, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);
         if (a64) return launch_wgrad_rows<64, 32>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);
         if (b64) return launch_wgrad_rows<32, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, s);

@@ -462,3 +462,11 @@ def test_sweeps_of_thin_grids(engine, oracle_lib, N1, N2, launches, scheme):
             ctx.advect_y(s, dev(vv), dt)
             assert rel_err(host(s), host(d)) <= 1e-13
         ctx.close()
+
+
+@pytest.mark.parametrize("W", [3, 6, 7])
+@pytest.mark.parametrize("cin,cout", [(8, 32), (32, 128), (256, 256)])
+def test_weight_gradient_of_narrow_images(engine, W, cin, cout):
+    """Either side of six columns, where the general kernel gives way to image rows.  The comparison of
+    test_weight_gradient_by_rows, for its reasons."""
+    test_weight_gradient_by_rows(engine, 48, 33, W, cin, cout)
