@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/impec2d.h"
+#include "perdevice.h"
 
 namespace impec {
 
@@ -122,6 +123,18 @@ inline cudaError_t launch_ks(bool pdl, cudaStream_t s, void (*k)(KArgs...), dim3
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(cudaStream_t s, void (*k)(KArgs...), dim3 g, dim3 b, size_t smem, Args&&... args) {
     return launch_ks(pdl_enabled(), s, k, g, b, smem, std::forward<Args>(args)...);
+}
+
+// Lets Kernel use `bytes` of dynamic shared memory (above the default limit) on the current device; a set
+// attribute stays.
+template <auto Kernel>
+inline cudaError_t allow_smem(int bytes) {
+    static OncePerDevice once;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return once.do_once(dev, cudaSuccess,
+                        [&] { return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
 }
 
 // Device-resident scalars of a step (so a step needs no host round trip).

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 #include <string>
 
 #include "learned.cuh"
@@ -1047,23 +1048,24 @@ void launch_wt_transpose(const __nv_bfloat16* W, int cin, int cout, __nv_bfloat1
     k_conv_wt_transpose<<<128, 256, 0, s>>>(W, cin, cout, conv_kp(cin), Wd, conv_kp(cout));
 }
 
+// The flag that the kernels' waits set when they give up: one on each device, kept for the process.
 int* device_error_flag() {
-    static int* flag = nullptr;
-    if (!flag) {
-        if (cudaMalloc((void**)&flag, sizeof(int)) != cudaSuccess) return nullptr;
-        cudaMemset(flag, 0, sizeof(int));
+    static std::mutex mu;
+    static int* flags[64] = {nullptr};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!flags[dev]) {
+        if (cudaMalloc((void**)&flags[dev], sizeof(int)) != cudaSuccess) return nullptr;
+        cudaMemset(flags[dev], 0, sizeof(int));
     }
-    return flag;
+    return flags[dev];
 }
 
 impec_status gemm_bf16_tn(int M, int N, int K, const void* A, int lda, const void* B, int ldb, float* C, int ldc,
                           cudaStream_t s, int* err) {
-    static bool attr = false;
     const int smem = 2 * GB_TILE_BYTES + 1024;
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_gemm_bf16_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY(allow_smem<k_gemm_bf16_tn>(smem));
     dim3 g((N + GB_N - 1) / GB_N, (M + GB_M - 1) / GB_M);
     k_gemm_bf16_tn<<<g, GB_THREADS, smem, s>>>(M, N, K, (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)B, ldb,
                                                  C, ldc, err);
@@ -1075,12 +1077,8 @@ int conv_kp(int cin) { return (9 * cin + GB_K - 1) / GB_K * GB_K; }
 
 template <int BN>
 static impec_status launch_conv_bn(const ConvArgs& a, cudaStream_t s) {
-    static bool attr = false;
     const int smem = conv_smem_bytes<BN>();
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv3x3<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY(allow_smem<k_conv3x3<BN>>(smem));
     const int M = a.B * a.H * a.W_;
     dim3 g((a.cout + BN - 1) / BN, (M + GB_M - 1) / GB_M);
     k_conv3x3<BN><<<g, CV_THREADS, smem, s>>>(a);
@@ -1142,12 +1140,7 @@ static bool conv_tma_plan(const ConvArgs& a, int BN, ConvTmaPlan& p) {
 
 template <int BN, int KS>
 static impec_status launch_conv_tma(const ConvArgs& a, const ConvTmaPlan& p, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv3x3_tma<BN, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            200 * 1024 + 1024));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY((allow_smem<k_conv3x3_tma<BN, KS>>(200 * 1024 + 1024)));
     TmapEncodeFn enc = tmap_encoder();
     const CUtensorMapSwizzle sw = KS == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     CUtensorMap tx, tw;
@@ -1187,11 +1180,7 @@ static impec_status launch_conv_tma(const ConvArgs& a, const ConvTmaPlan& p, cud
 template <int BN, int CIN>
 static impec_status launch_conv_halo(const ConvArgs& a, cudaStream_t s) {
     constexpr int smem = halo_smem<BN, CIN>();
-    static bool attr = false;
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv3x3_halo<BN, CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY((allow_smem<k_conv3x3_halo<BN, CIN>>(smem)));
     TmapEncodeFn enc = tmap_encoder();
     const CUtensorMapSwizzle sw = CIN == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
                                             : (CIN == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
@@ -1299,11 +1288,7 @@ static impec_status launch_wgrad_tma(const __nv_bfloat16* dZ, const __nv_bfloat1
                                      cudaStream_t s) {
     constexpr int STAGE = 128 * WG_PIX * 2 * 2;
     const int smem = WG_STAGES * STAGE + 1024;
-    static bool attr = false;
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv_wgrad_tma<CA, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY((allow_smem<k_conv_wgrad_tma<CA, CB>>(smem)));
     TmapEncodeFn enc = tmap_encoder();
     const cuuint32_t es[4] = {1, 1, 1, 1};
     const int P = B * H * W_, Kp = conv_kp(cin);
@@ -1342,11 +1327,7 @@ static impec_status launch_wgrad_rows(const __nv_bfloat16* dZ, const __nv_bfloat
                                       int cout, float* dW, int* err, int num_sms, cudaStream_t s) {
     using G = WgRows<CA, CB>;
     constexpr int SMEM = 216 * 1024;
-    static bool attr = false;
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv_wgrad_rows<CA, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY((allow_smem<k_conv_wgrad_rows<CA, CB>>(SMEM)));
     const cuuint32_t es[4] = {1, 1, 1, 1};
     auto encode = [&](CUtensorMap* m, const void* p, int c, int box, int pix) {
         const cuuint64_t d[4] = {(cuuint64_t)c, (cuuint64_t)W_, (cuuint64_t)H, (cuuint64_t)B};
@@ -1399,12 +1380,8 @@ impec_status launch_wgrad(const __nv_bfloat16* dZ, const __nv_bfloat16* X, int B
         if (b64) return launch_wgrad_tma<32, 64>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, wb, hb, bb, s);
         return launch_wgrad_tma<32, 32>(dZ, X, B, H, W_, cin, cout, dW, err, num_sms, wb, hb, bb, s);
     }
-    static bool attr = false;
     const int smem = 2 * GB_TILE_BYTES + 1024;
-    if (!attr) {
-        IMPEC_CUDA_TRY(cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
-    }
+    IMPEC_CUDA_TRY(allow_smem<k_conv_wgrad>(smem));
     const int P = B * H * W_, Kp = conv_kp(cin);
     const int nt = (9 * cin + GB_N - 1) / GB_N, mt = (cout + GB_M - 1) / GB_M;
     int splits = (2 * num_sms + nt * mt - 1) / (nt * mt);  // about two waves of CTAs

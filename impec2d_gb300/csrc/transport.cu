@@ -411,8 +411,7 @@ __global__ void __launch_bounds__(Tile<TI, MODE>::THREADS) k_advect_tile(const T
     }
 }
 
-// Launches one tile kernel.  Its shared memory is above the default limit, which each device has
-// to be told once per kernel (a set attribute stays; setting it again does no harm).
+// Launches one tile kernel, whose shared memory is above the default limit.
 template <int SCHEME, int BC, int MODE, int TI>
 static cudaError_t launch_tile(cudaStream_t s, TileArgs A, bool edges) {
     int rows = (A.n1 + TI - 1) / TI;
@@ -420,20 +419,8 @@ static cudaError_t launch_tile(cudaStream_t s, TileArgs A, bool edges) {
         A.row0 = rows - 3;
         rows = 3;
     }
-    static std::mutex mu;
-    static unsigned long long done = 0;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = allow_smem<k_advect_tile<SCHEME, BC, MODE, TI>>((int)Tile<TI, MODE>::SMEM);
     if (e != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev >= 64 || !(done >> dev & 1)) {
-            e = cudaFuncSetAttribute(k_advect_tile<SCHEME, BC, MODE, TI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)Tile<TI, MODE>::SMEM);
-            if (e != cudaSuccess) return e;
-            if (dev < 64) done |= 1ull << dev;
-        }
-    }
     const dim3 g((A.n2 + TJ - 1) / TJ, rows);
     return launch_k(s, k_advect_tile<SCHEME, BC, MODE, TI>, g, Tile<TI, MODE>::THREADS, Tile<TI, MODE>::SMEM, A);
 }
