@@ -17,8 +17,8 @@
 // Levels nd .. nl-1 have rows[l] = n1[l]: CTA 0 owns all of them.
 //
 // What bounds it: latency.  A phase is one dependent chain of 5 to 10 FP64 operations per cell
-// (at 128^2 also 1,300 cycles of FP64 issue per colour on 16 SMs) behind a barrier, some forty of
-// them.  So a five-point band keeps the neighbours' edge rows in halo rows of its own, which the
+// (at 128^2 also 1,300 cycles of FP64 issue per colour on 16 SMs) behind a barrier: some forty phases, 26 of them
+// behind a cluster barrier at 128^2, the others on CTA 0 alone.  So a five-point band keeps the neighbours' edge rows in halo rows of its own, which the
 // neighbour writes when it updates its edge cell (the store's way to the other SM overlaps the
 // rest of the phase) instead of being read from there at the start of the next one, and cells are
 // found without an integer division.
@@ -43,10 +43,11 @@
 constexpr int CL_MAXL = 10;
 constexpr int CL_THREADS = 512;
 constexpr int CL_MAX_CTAS = 16;
-// shared arrays of a level.  Five-point: X, P, Q and the four planes of W have a halo row above and
-// below the band (plane stride (rows + 2) * n2).  A nine-point level keeps its nine planes at CL_TX (plane
-// stride rows * n2) and has no CL_TY / CL_DG (the diagonal is plane 0), no halo rows, no W, P, Q.
-enum { CL_TX = 0, CL_TY, CL_ID, CL_DG, CL_X, CL_B, CL_W, CL_P, CL_Q, CL_ARRAYS };
+// shared arrays of a level.  Five-point: X, P, Q, P2, Q2 and the four planes of W have a halo row above and
+// below the band (plane stride (rows + 2) * n2); plain transfers have no W, and only a restriction that
+// takes both colours has P2, Q2.  A nine-point level keeps its nine planes at CL_TX (plane stride rows * n2) and has
+// no CL_TY / CL_DG (the diagonal is plane 0), no halo rows and none of the last five.
+enum { CL_TX = 0, CL_TY, CL_ID, CL_DG, CL_X, CL_B, CL_W, CL_P, CL_Q, CL_P2, CL_Q2, CL_ARRAYS };
 
 template <class T>
 struct ClusterArgs {
@@ -55,8 +56,9 @@ struct ClusterArgs {
     int dn;
     int npre, npost;  // smoother colours before / after the coarse correction
     int post_first;   // five-point: colour of the first one after it
-    int zero_color;   // five-point: restriction skips cells of this colour (their residual is ~0)
+    int zero_color;   // five-point: restriction skips cells of this colour (their residual is ~0), -1: none
     int zero0;        // five-point: level 0 starts from x = 0 (x0 is not read)
+    int plain;        // five-point: transfers without weights (as k_restrict5 and prolong_cell without w4)
     int n1[CL_MAXL], n2[CL_MAXL], rows[CL_MAXL];
     float rhalf[CL_MAXL], rn2[CL_MAXL];       // 1 / ((n2 + 1) / 2), 1 / n2
     unsigned off[CL_MAXL][CL_ARRAYS];  // shared-memory offsets (elements of T)
@@ -144,14 +146,14 @@ __device__ void cl_sweep(const cooperative_groups::cluster_group& cl, T* sm, int
 // First half of the restriction: the residual of every band cell of the colour that the sweep
 // before it did not update last, to the CTA that owns its coarse row: P for the child on the even
 // fine row, Q for the one on the odd row (each coarse cell has one of each), with the halo rows of
-// that CTA's neighbours.
-template <class T>
+// that CTA's neighbours.  Where no colour is skipped, the black cells' go there and the red ones' to P2, Q2.
+template <class T, bool ANY>
 __device__ void cl_residual(const cooperative_groups::cluster_group& cl, T* sm, int rank, const ClusterArgs<T>& A,
                             int l) {
     int lo, cnt;
     cl_band(A, l, rank, lo, cnt);
     if (cnt == 0) return;
-    const int n1 = A.n1[l], n2 = A.n2[l], half = (n2 + 1) / 2, col = 1 - A.zero_color;
+    const int n1 = A.n1[l], n2 = A.n2[l], half = (n2 + 1) / 2, both = ANY && A.zero_color < 0;
     const int c1 = A.n1[l + 1], c2 = A.n2[l + 1], R = A.rows[l + 1];
     const bool spread = l + 1 < A.nd;
     const T* x = sm + A.off[l][CL_X] + n2;
@@ -159,7 +161,8 @@ __device__ void cl_residual(const cooperative_groups::cluster_group& cl, T* sm, 
     const T* tx = sm + A.off[l][CL_TX];
     const T* ty = sm + A.off[l][CL_TY];
     const T* dg = sm + A.off[l][CL_DG];
-    for (int k = threadIdx.x; k < cnt * half; k += CL_THREADS) {
+    for (int t = threadIdx.x; t < cnt * half * (1 + both); t += CL_THREADS) {
+        const int second = t >= cnt * half, k = t - second * cnt * half, col = both ? 1 - second : 1 - A.zero_color;
         const int li = cl_div(k, A.rhalf[l]), i = lo + li, j = 2 * (k - li * half) + ((i + col) & 1);
         T r = 0;
         if (j < n2) {
@@ -179,15 +182,16 @@ __device__ void cl_residual(const cooperative_groups::cluster_group& cl, T* sm, 
             if (spread && ro == 0 && I > 0) cl.map_shared_rank(base + (size_t)(R + 1) * c2, (unsigned)(o - 1))[0] = v;
             if (spread && ro == R - 1 && I < c1 - 1) cl.map_shared_rank(base, (unsigned)(o + 1))[0] = v;
         };
-        put((i & 1) ? CL_Q : CL_P, r);
-        if (i == n1 - 1 && !(i & 1)) put(CL_Q, T(0));  // odd n1: no child on the odd row
+        put(((i & 1) ? CL_Q : CL_P) + 2 * second, r);
+        if (i == n1 - 1 && !(i & 1)) put(CL_Q + 2 * second, T(0));  // odd n1: no child on the odd row
     }
 }
 
 // Second half: coarse right-hand side of the rows this CTA owns from its own and the
 // neighbouring children (the arithmetic of k_restrict5), and the coarse sweep's first colour from
-// x = 0 (red: x = b * idiag).  The dense coarsest level (last) takes no sweep.
-template <class T>
+// x = 0 (red: x = b * idiag), or x = 0 where no sweep precedes the correction.  The dense coarsest level
+// (last) takes neither.
+template <class T, bool ANY>
 __device__ void cl_gather(const cooperative_groups::cluster_group& cl, T* sm, int rank, const ClusterArgs<T>& A,
                           int l, bool last) {
     int lo, cnt;
@@ -203,18 +207,30 @@ __device__ void cl_gather(const cooperative_groups::cluster_group& cl, T* sm, in
     const T *wE = sm + A.off[l][CL_W] + n2, *wW = wE + ps, *wN = wW + ps, *wS = wN + ps;
     // which child lies east, west, north, south: the black ones (zero_color 0) or the red ones
     const T *north = A.zero_color == 1 ? Q : P, *south = A.zero_color == 1 ? P : Q;
+    // or all four (P: row 0, column 1; Q: 1, 0; P2: 0, 0; Q2: 1, 1)
+    const bool both = ANY && A.zero_color < 0;
+    const T *P2 = sm + A.off[l][CL_P2] + n2, *Q2 = sm + A.off[l][CL_Q2] + n2;
+    auto east = [&](int k) { return both ? Q[k] + Q2[k] : Q[k]; };
+    auto west = [&](int k) { return both ? P2[k] + P[k] : P[k]; };
+    auto nort = [&](int k) { return both ? P[k] + Q2[k] : north[k]; };
+    auto sout = [&](int k) { return both ? P2[k] + Q[k] : south[k]; };
     T *up, *dn;
     cl_halo(cl, sm, rank, A, l, CL_X, lo, cnt, up, dn);
     for (int k = threadIdx.x; k < cnt * n2; k += CL_THREADS) {
         const int li = cl_div(k, A.rn2[l]), j = k - li * n2, i = lo + li;
-        T v = restrict_sum<T>(Q[k], P[k], north[k], south[k], wE[k], wW[k], wN[k], wS[k]);
-        if (i > 0) v = fma(wE[k - n2], Q[k - n2], v);
-        if (i < n1 - 1) v = fma(wW[k + n2], P[k + n2], v);
-        if (j > 0) v = fma(wN[k - 1], north[k - 1], v);
-        if (j < n2 - 1) v = fma(wS[k + 1], south[k + 1], v);
+        const T e = east(k), w = west(k);
+        T v = e + w;
+        if (!ANY || !A.plain) {
+            v = restrict_sum<T>(e, w, nort(k), sout(k), wE[k], wW[k], wN[k], wS[k]);
+            if (i > 0) v = fma(wE[k - n2], east(k - n2), v);
+            if (i < n1 - 1) v = fma(wW[k + n2], west(k + n2), v);
+            if (j > 0) v = fma(wN[k - 1], nort(k - 1), v);
+            if (j < n2 - 1) v = fma(wS[k + 1], sout(k + 1), v);
+        }
         b[k] = v;
-        if (last || ((i + j) & 1)) continue;
-        v = v * id[k];
+        const bool sweep = !ANY || A.npre > 0;
+        if (last || (sweep && ((i + j) & 1))) continue;
+        v = sweep ? v * id[k] : T(0);
         x[k] = v;
         if (li == 0 && up) up[j] = v;
         if (li == cnt - 1 && dn) dn[j] = v;
@@ -223,7 +239,7 @@ __device__ void cl_gather(const cooperative_groups::cluster_group& cl, T* sm, in
 
 // Prolongation of the coarse iterate to the band's cells of the colour that the post-smoothing
 // does not overwrite first, or to all of them (colour -1): the arithmetic of k_prolong.
-template <class T>
+template <class T, bool ANY>
 __device__ void cl_prolong5(const cooperative_groups::cluster_group& cl, T* sm, int rank, const ClusterArgs<T>& A,
                             int l, int col) {
     int lo, cnt;
@@ -262,7 +278,15 @@ __device__ void cl_prolong5(const cooperative_groups::cluster_group& cl, T* sm, 
             w1 = o1 == rank ? c : cl.map_shared_rank(c, (unsigned)o1);
         }
         const int c = li * n2 + j;
-        const T v = prolong5<T>(x[c], r1[J], r2[J], r1[J2], w1[ex * ps + J], w1[ey * ps + J]);
+        T v = x[c];
+        if (ANY && A.plain) {
+            v += T(0.5625) * r1[J];
+            v += T(0.1875) * r2[J];
+            v += T(0.1875) * r1[J2];
+            v += T(0.0625) * r2[J2];
+        } else {
+            v = prolong5<T>(v, r1[J], r2[J], r1[J2], w1[ex * ps + J], w1[ey * ps + J]);
+        }
         x[c] = v;
         if (li == 0 && up) up[j] = v;
         if (li == cnt - 1 && dn) dn[j] = v;
@@ -367,8 +391,10 @@ __device__ void cl_prolong9(const cooperative_groups::cluster_group& cl, T* sm, 
     }
 }
 
-// KIND: FACE5 or EXP9 (every level of the cycle).
-template <class T, int KIND>
+// KIND: FACE5 or EXP9 (every level of the cycle).  ANY: any schedule and transfers of five-point levels; without
+// it a skipped colour, weighted transfers and a sweep before the correction are taken for granted, as a CG solve has them by
+// default (decided at run time they cost that solve 5%: 128^2 step 1020 / 1066 us).
+template <class T, int KIND, bool ANY>
 __global__ void __launch_bounds__(CL_THREADS) k_cluster_vcycle(const __grid_constant__ ClusterArgs<T> A) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -388,7 +414,7 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_vcycle(const __grid_cons
         T* id = sm + A.off[l][CL_ID];
         T* dg = sm + A.off[l][CL_DG];
         if (KIND == FACE5) {
-            if (l > 0) {
+            if (l > 0 && !(ANY && A.plain)) {
                 // the gather reads the rows above and below too
                 T* w = sm + A.off[l][CL_W];
                 const int first = lo > 0 ? 0 : n2, last = (lo + cnt < A.n1[l] ? cnt + 2 : cnt + 1) * n2;
@@ -439,36 +465,36 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_vcycle(const __grid_cons
     const int L = A.nl - 1;
     if (KIND == FACE5) {
         const int keep = A.npost > 0 ? 1 - A.post_first : -1;  // cells that the prolongation corrects
-        // down: the first colour of a level below the first was done with its right-hand side
+        // down: the first colour of a level below the first was done with its right-hand side (cl_gather)
         for (int l = 0; l < A.nd; ++l) {
             for (int s = l > 0 ? 1 : 0; s < A.npre; ++s) {
                 cl_sweep(cl, sm, rank, A, l, s & 1, A.zero0 && s == 0);
                 cl.sync();
             }
-            cl_residual(cl, sm, rank, A, l);
+            cl_residual<T, ANY>(cl, sm, rank, A, l);
             cl.sync();
             if (l + 1 < A.nd) {
-                cl_gather(cl, sm, rank, A, l + 1, false);
+                cl_gather<T, ANY>(cl, sm, rank, A, l + 1, false);
                 cl.sync();
             }
         }
         // the small levels and the dense solve on CTA 0
         if (rank == 0) {
             for (int l = A.nd; l < L; ++l) {
-                cl_gather(cl, sm, 0, A, l, false);
+                cl_gather<T, ANY>(cl, sm, 0, A, l, false);
                 __syncthreads();
                 for (int s = 1; s < A.npre; ++s) {
                     cl_sweep(cl, sm, 0, A, l, s & 1);
                     __syncthreads();
                 }
-                cl_residual(cl, sm, 0, A, l);
+                cl_residual<T, ANY>(cl, sm, 0, A, l);
                 __syncthreads();
             }
-            cl_gather(cl, sm, 0, A, L, true);
+            cl_gather<T, ANY>(cl, sm, 0, A, L, true);
             __syncthreads();
             dense_coarse_apply<T>(A.dn, dinv, sm + A.off[L][CL_B], sm + A.off[L][CL_X] + A.n2[L]);
             for (int l = L - 1; l >= A.nd; --l) {
-                cl_prolong5(cl, sm, 0, A, l, keep);
+                cl_prolong5<T, ANY>(cl, sm, 0, A, l, keep);
                 __syncthreads();
                 for (int s = 0; s < A.npost; ++s) {
                     cl_sweep(cl, sm, 0, A, l, (A.post_first + s) & 1);
@@ -479,7 +505,7 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_vcycle(const __grid_cons
         cl.sync();
         // up: levels spread over the cluster
         for (int l = A.nd - 1; l >= 0; --l) {
-            cl_prolong5(cl, sm, rank, A, l, keep);
+            cl_prolong5<T, ANY>(cl, sm, rank, A, l, keep);
             cl.sync();
             for (int s = 0; s < A.npost; ++s) {
                 cl_sweep(cl, sm, rank, A, l, (A.post_first + s) & 1);

@@ -1053,7 +1053,7 @@ constexpr size_t MG_CLUSTER_SMEM = 200 * 1024;
 
 // CTAs per cluster for k_cluster_vcycle: 16 where the device can co-schedule such a cluster
 // with the kernel's shared memory, else 8, else 0 (the per-level path is used).
-template <class T, int KIND>
+template <class T, int KIND, bool ANY>
 static int cluster_size_for(int want) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(want);
@@ -1067,7 +1067,7 @@ static int cluster_size_for(int want) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, k_cluster_vcycle<T, KIND>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&num, k_cluster_vcycle<T, KIND, ANY>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -1202,11 +1202,13 @@ impec_status pressure_alloc(impec_ctx* ctx) {
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cls) == cudaSuccess &&
                cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     };
-    if (f5 ? allow(k_cluster_vcycle<double, FACE5>) && allow(k_cluster_vcycle<float, FACE5>)
-           : allow(k_cluster_vcycle<double, EXP9>))
+    if (f5 ? allow(k_cluster_vcycle<double, FACE5, false>) && allow(k_cluster_vcycle<float, FACE5, false>) &&
+                 allow(k_cluster_vcycle<double, FACE5, true>) && allow(k_cluster_vcycle<float, FACE5, true>)
+           : allow(k_cluster_vcycle<double, EXP9, false>))
         for (int cs = want < CL_MAX_CTAS ? want : CL_MAX_CTAS; cs >= 2 && !ctx->cl_size; cs /= 2)
-            if (f5 ? cluster_size_for<double, FACE5>(cs) && cluster_size_for<float, FACE5>(cs)
-                   : cluster_size_for<double, EXP9>(cs))
+            if (f5 ? cluster_size_for<double, FACE5, false>(cs) && cluster_size_for<float, FACE5, false>(cs) &&
+                         cluster_size_for<double, FACE5, true>(cs) && cluster_size_for<float, FACE5, true>(cs)
+                   : cluster_size_for<double, EXP9, false>(cs))
                 ctx->cl_size = cs;
     cudaGetLastError();
     return IMPEC_OK;
@@ -1545,8 +1547,7 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
     A.npost = f5 ? col.npost : 4 * (int)ctx->tune.post;
     A.post_first = col.post_first;
     A.zero_color = restrict_zero_color(ctx, ctx->L[ls]);
-    // five-point levels: its restriction knows one colour's residuals and weighted transfers only
-    if (f5 && (A.zero_color < 0 || !ctx->krylov)) return false;
+    A.plain = ctx->krylov ? 0 : 1;
     A.dn = ctx->dense_n;
     A.dinv = ctx->dense_inv;
     size_t off = 0;
@@ -1567,7 +1568,8 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
         const size_t ops = k + 1 < nl ? r * n2 : 0;  // the dense level keeps no operator
         const size_t halo = f5 ? (r + 2) * n2 : r * n2, tr = f5 && k > 0 ? halo : 0;
         const size_t sz[CL_ARRAYS] = {f5 ? (ops ? (r + 1) * n2 : 0) : 9 * ops, f5 && ops ? r * (n2 + 1) : 0, ops,
-                                      f5 ? ops : 0, halo, r * n2, 4 * tr, tr, tr};
+                                      f5 ? ops : 0, halo, r * n2, A.plain ? 0 : 4 * tr, tr, tr, A.zero_color < 0 ? tr : 0,
+                                      A.zero_color < 0 ? tr : 0};
         for (int a = 0; a < CL_ARRAYS; ++a) {
             A.off[k][a] = (unsigned)off;
             off += sz[a];
@@ -1632,8 +1634,12 @@ static void launch_cluster(impec_ctx* ctx, size_t ls, bool zero) {
     cfg.attrs = at;
     cfg.numAttrs = 2;  // always with programmatic serialisation (mgcluster.cuh: staging)
     ++ctx->nlaunch;
-    if (ctx->L[ls].kind == FACE5) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5>, A);
-    else if constexpr (sizeof(T) == 8) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, EXP9>, A);
+    if (ctx->L[ls].kind == FACE5) {
+        if (A.plain || A.zero_color < 0) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, true>, A);
+        else cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, false>, A);
+    } else if constexpr (sizeof(T) == 8) {
+        cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, EXP9, false>, A);
+    }
 }
 
 // Whether a five-point V-cycle at level l started from x = 0 needs no zero fill of the level's

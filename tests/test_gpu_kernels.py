@@ -470,3 +470,35 @@ def test_weight_gradient_of_narrow_images(engine, W, cin, cout):
     """Either side of six columns, where the general kernel gives way to image rows.  The comparison of
     test_weight_gradient_by_rows, for its reasons."""
     test_weight_gradient_by_rows(engine, 48, 33, W, cin, cout)
+
+
+@pytest.mark.parametrize("N1,N2", [(37, 29), (100, 100), (300, 130), (65, 257)])
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("env", [{"IMPEC_MG_KRYLOV": "0"}, {"IMPEC_MG_RB_RESID": "0"}, {"IMPEC_MG_PRE": "0", "IMPEC_MG_POST": "2"},
+                                 {"IMPEC_MG_KRYLOV": "0", "IMPEC_MG_RB_RESID": "0"}, {"IMPEC_MG_PRE": "2", "IMPEC_MG_POST": "0"}],
+                         ids=["stationary", "all residuals", "no pre-smoothing", "stationary, all residuals", "no post-smoothing"])
+def test_cluster_takes_every_schedule(engine, monkeypatch, N1, N2, prec, env):
+    """Stationary cycles (plain transfers), restrictions that take both colours' residuals and one-sided smoothing run
+    their coarse levels in the cluster launch too, with the bits of the per-level launches."""
+    import torch
+
+    from helpers import dev, host
+    E = engine
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    c = np.random.default_rng(9).uniform(0.0, 1.0, (N1, N2))
+    out = []
+    for cluster in ("0", "1"):
+        monkeypatch.setenv("IMPEC_MG_CLUSTER", cluster)
+        P = E.default_params(N1, N2, stype=1, nu=1.0, precision=prec, max_cycles=200, x_lb=0.0, x_ub=float(N1), y_lb=0.0,
+                             y_ub=float(N2))
+        ctx = E.Context(P)
+        ctx.set_source(dev(source(oparams(P))))
+        p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+        n0 = E.launch_count(ctx)
+        cyc, rr, _ = ctx.pressure_solve(dev(c), p, 1e-9, check=False)
+        out.append((cyc, rr, host(p), E.launch_count(ctx) - n0))
+        ctx.close()
+    assert np.isfinite(out[0][1]) and out[0][:2] == out[1][:2]
+    assert np.array_equal(out[0][2], out[1][2])
+    assert out[1][3] < out[0][3]
