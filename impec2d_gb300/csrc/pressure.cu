@@ -230,7 +230,7 @@ __constant__ int c_off[9][2] = {{0, 0}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}, {1,
 //
 // A block owns 32 x 8 coarse cells: h of the cells and a one-cell ring in shared memory, then
 // each face of the tile once, then weights, diagonal and 1/diagonal from those faces.  FP64-bound
-// (seven divisions per coarse cell).
+// (five divisions per coarse cell) on large levels, bound by the latency of that chain on small ones.
 constexpr int CO_C = 32, CO_R = 8;
 // The children's conductances a, b count as a + CO_MIX min(a, b) and b + CO_MIX min(a, b) in the split: contrasts below
 // some ten leave it near one half, where the transfers are exact for linear pressures.
@@ -273,64 +273,79 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
     };
     // The inside between children that conduct b0, b1 outwards and t0, t1 across: the parts towards either
     // side.  One without any conductance counts as none: beyond it lie dead cells, or a known row, whose
-    // couplings are on the diagonal.
+    // couplings are on the diagonal.  One division unless the operands are far out of the ordinary.
     auto split = [&](double in, double b0, double t0, double b1, double t1, double& h0, double& h1) {
         if (!(in > 0.0)) return;
-        const double a0 = b0 + t0, a1 = b1 + t1, m = CO_MIX * fmin(a0, a1), s0 = a0 + m, s1 = a1 + m;
-        const double g = fmin(1.0 / fmax(CO_DETOUR * fmin(t0, t1), in), 1e300);
-        const double part = s0 + s1 > 1e-290 ? 1.0 / (s0 + s1) : 0.0;
-        h0 = part > 0.0 ? s1 * part * g : 0.5 * g;
-        h1 = part > 0.0 ? s0 * part * g : 0.5 * g;
+        const double a0 = b0 + t0, a1 = b1 + t1, m = CO_MIX * fmin(a0, a1), s0 = a0 + m, s1 = a1 + m, s = s0 + s1;
+        const double g = fmax(CO_DETOUR * fmin(t0, t1), in), d = s * g;
+        if (d > 1e-290 && d < 1e290) {
+            const double e = 1.0 / d;
+            h0 = s1 * e;
+            h1 = s0 * e;
+        } else {
+            const double e = fmin(1.0 / g, 1e300), part = s > 1e-290 ? s1 / s : 0.5;
+            h0 = part * e;
+            h1 = e - h0;
+        }
     };
-    for (int k = t; k < (CO_R + 2) * CO_C; k += CO_C * CO_R) {
-        const int r = k / CO_C, q = k % CO_C, I = I0 - 1 + r, J = J0 + q;
-        double h0 = 0.0, h1 = 0.0;
+    auto half_x = [&](int I, int J, double& h0, double& h1) {
+        h0 = h1 = 0.0;
         if (!plain && I >= 0 && J < n2c && 2 * I + 1 < n1f)
             split(pair_x(2 * I + 1, J), pair_x(2 * I, J), row_y(2 * I, J), pair_x(2 * I + 2, J), row_y(2 * I + 1, J), h0, h1);
-        hx0[r][q] = h0;
-        hx1[r][q] = h1;
-    }
-    for (int k = t; k < CO_R * (CO_C + 2); k += CO_C * CO_R) {
-        const int r = k / (CO_C + 2), q = k % (CO_C + 2), I = I0 + r, J = J0 - 1 + q;
-        double h0 = 0.0, h1 = 0.0;
+    };
+    auto half_y = [&](int I, int J, double& h0, double& h1) {
+        h0 = h1 = 0.0;
         if (!plain && J >= 0 && I < n1c && 2 * J + 1 < n2f)
             split(pair_y(I, 2 * J + 1), pair_y(I, 2 * J), col_x(I, 2 * J), pair_y(I, 2 * J + 2), col_x(I, 2 * J + 1), h0, h1);
-        hy0[r][q] = h0;
-        hy1[r][q] = h1;
+    };
+    // each thread its own cell, then some a cell of the ring (the small levels are bound by latency: two short
+    // chains side by side and one more instead of four in a row)
+    const int r = threadIdx.y, q = threadIdx.x, I = I0 + r, J = J0 + q;
+    half_x(I, J, hx0[r + 1][q], hx1[r + 1][q]);
+    half_y(I, J, hy0[r][q + 1], hy1[r][q + 1]);
+    if (t < 2 * CO_C) {
+        const int a = t / CO_C * (CO_R + 1), c = t % CO_C;
+        half_x(I0 - 1 + a, J0 + c, hx0[a][c], hx1[a][c]);
+    } else if (t < 2 * CO_C + 2 * CO_R) {
+        const int a = (t - 2 * CO_C) % CO_R, c = (t - 2 * CO_C) / CO_R * (CO_C + 1);
+        half_y(I0 + a, J0 - 1 + c, hy0[a][c], hy1[a][c]);
     }
     __syncthreads();
-    for (int k = t; k < (CO_R + 1) * CO_C; k += CO_C * CO_R) {
-        const int r = k / CO_C, q = k % CO_C, I = I0 + r, J = J0 + q;
+    auto face_x = [&](int r, int q, bool store) {  // a face on the far side of the tile is the next tile's, except the last one
+        const int I = I0 + r, J = J0 + q;
         double v = 0.0;
         if (I <= n1c && J < n2c) {
             if (I > 0 && I < n1c) {
                 const double a = pair_x(2 * I, J);
                 v = plain ? 0.5 * a : a / (1.0 + a * (hx1[r][q] + hx0[r + 1][q]));
             }
-            if (r < CO_R || I == n1c) {  // the face below the tile belongs to the next tile, except the last one
+            if (store || I == n1c) {
                 txc[IX(I, J, n2c)] = v;
                 if (txc32) txc32[IX(I, J, n2c)] = (float)v;
             }
         }
         cx[r][q] = v;
-    }
-    for (int k = t; k < CO_R * (CO_C + 1); k += CO_C * CO_R) {
-        const int r = k / (CO_C + 1), q = k % (CO_C + 1), I = I0 + r, J = J0 + q;
+    };
+    auto face_y = [&](int r, int q, bool store) {
+        const int I = I0 + r, J = J0 + q;
         double v = 0.0;
         if (I < n1c && J <= n2c) {
             if (J > 0 && J < n2c) {
                 const double a = pair_y(I, 2 * J);
                 v = plain ? 0.5 * a : a / (1.0 + a * (hy1[r][q] + hy0[r][q + 1]));
             }
-            if (q < CO_C || J == n2c) {
+            if (store || J == n2c) {
                 tyc[IX(I, J, n2c + 1)] = v;
                 if (tyc32) tyc32[IX(I, J, n2c + 1)] = (float)v;
             }
         }
         cy[r][q] = v;
-    }
+    };
+    face_x(r, q, true);
+    face_y(r, q, true);
+    if (t < CO_C) face_x(CO_R, t, false);
+    else if (t < CO_C + CO_R) face_y(t - CO_C, CO_C, false);
     __syncthreads();
-    const int r = threadIdx.y, q = threadIdx.x, I = I0 + r, J = J0 + q;
     if (I >= n1c || J >= n2c) return;
     const size_t n = (size_t)n1c * n2c, k = IX(I, J, n2c);
     if (w4) {
