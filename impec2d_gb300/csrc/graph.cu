@@ -360,7 +360,9 @@ extern "C" impec_status impec_ensemble_create(impec_ctx* const* members, int n, 
         impec_ctx* c = e->m[i];
         ce = cudaStreamWaitEvent(c->cap_stream, e->fork, 0);
         if (ce != cudaSuccess) break;
+        c->crowd = n > 1;
         s = capture_step_into(c, 0);  // the variant a single context replays (non-alternating splitting)
+        c->crowd = false;
         if (s != IMPEC_OK) break;
         ce = cudaEventRecord(e->join[i], c->cap_stream);
         if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->stream, e->join[i], 0);

@@ -250,6 +250,9 @@ struct impec_ctx {
     // live ensembles whose captured graph holds this context's buffers: calls that would free
     // or move a buffer are refused while it is non-zero
     int ensembles = 0;
+    // being captured as one of several branches of an ensemble's graph: no programmatic launches, whose blocks
+    // would wait on SMs that the other members have work for
+    bool crowd = false;
 };
 
 namespace impec {

@@ -1647,7 +1647,7 @@ static void launch_cluster(impec_ctx* ctx, size_t ls, bool zero) {
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 2;  // always with programmatic serialisation (mgcluster.cuh: staging)
+    cfg.numAttrs = ctx->crowd ? 1 : 2;  // with programmatic serialisation (mgcluster.cuh: staging) unless in a crowd
     ++ctx->nlaunch;
     if (ctx->L[ls].kind == FACE5) {
         if (A.plain || A.zero_color < 0) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, true>, A);
@@ -2259,7 +2259,7 @@ impec_status pressure_iteration(impec_ctx* ctx, double tol, cudaGraphConditional
     // On small grids an iteration's vector kernels are short beside the launches between them, which programmatic
     // serialisation overlaps; on larger ones the waiting blocks take the running kernel's places (us without / with:
     // 128^2 step 1007 / 990, 300 x 130 solve 1520 / 1415, 256^2 step 918 / 929, 513 x 777 step 2820 / 2970).
-    const bool pdl = pdl_enabled() || n < (size_t)3 << 14;
+    const bool pdl = pdl_enabled() || (n < (size_t)3 << 14 && !ctx->crowd);
     const auto dots = [&](auto kernel, auto* zz) {
         ++ctx->nlaunch;
         launch_ks(pdl, ctx->stream, kernel, vblocks(2), RED_THREADS, 0, n, (const double*)r, zz, (const double*)ctx->cg_q, ctx->partials,
