@@ -204,14 +204,14 @@ __constant__ int c_off[9][2] = {{0, 0}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}, {1,
 // t_in is the sum of the two fine faces inside the cell in that direction.  The inside is split between
 // its two sides: half and half in the ordinary case, but where one pair of children conducts far
 // better than the other (CO_MIX) the coarse value is that pair's, and the other side's way takes it
-// all.  t_in counts as a hundredth of what both pairs conduct across at least (CO_DETOUR), a way round
-// the inside through the next cells.  With h = 1 / (2 t_in) alone, a cell on the edge of a nearly
+// all.  t_in counts as a fiftieth at least of what both pairs conduct across and the better one outwards
+// (CO_DETOUR), a way round the inside through the next cells.  With h = 1 / (2 t_in) alone, a cell on the edge of a nearly
 // impermeable inclusion had hardly any coupling left, although half of it belongs to the well
 // conducting surroundings, and CG hung.  Iterations to 1e-9, FP64, with the half sums and bilinear
 // transfers of plain, with even splits, and now: inclusions of 1e-10 on 64^2 22 / over 400 / 11 and on
-// 130 x 900 36 / over 400 / 25; barriers of 1e-8 crossed by a channel of 1e4, 64^2, 41 / 261 / 13; 15% of the
-// cells at 1e-6, 64^2, 69 / 140 / 22; cells at exp(3 N(0,1)), 513 x 512, 229 / 249 / 67; K11 and K22
-// independent at exp(1.5 N), 513 x 512, 234 / 86 / 101.
+// 130 x 900 36 / over 400 / 37; barriers of 1e-8 crossed by a channel of 1e4, 64^2, 41 / 261 / 13; 15% of the
+// cells at 1e-6, 64^2, 69 / 140 / 22; cells at exp(3 N(0,1)), 513 x 512, 229 / 249 / 65; K11 and K22
+// independent at exp(1.5 N), 513 x 512, 234 / 86 / 85.
 // On a uniform grid the face is the rediscretised one (s = 2, h = 1/4, t = 1); across a jump of the
 // mobility it keeps the harmonic mean that the sum of the fine faces loses.  The same quantities
 // give the transfer weights w = h t <= 1 of a coarse cell towards its four neighbours
@@ -234,8 +234,31 @@ __constant__ int c_off[9][2] = {{0, 0}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}, {1,
 constexpr int CO_C = 32, CO_R = 8;
 // The children's conductances a, b count as a + CO_MIX min(a, b) and b + CO_MIX min(a, b) in the split: contrasts below
 // some ten leave it near one half, where the transfers are exact for linear pressures.
-constexpr double CO_MIX = 10.0;
-constexpr double CO_DETOUR = 0.01;
+constexpr float CO_MIX = 10.0f;
+constexpr float CO_DETOUR = 0.02f;
+// The leading bits (20 of the mantissa) of v >= 0 as v 2^-(top - 1022), top being an exponent field at least v's: below
+// 1, zero when more than 2^126 smaller.  By integer operations: the ratios of conductances that decide a
+// split need no more, and sixty FP64 operations a cell for them were as many as all the others (2048^2, set-up and
+// residual of a solve: 976 us so, 859 now, 847 with even splits).
+__device__ __forceinline__ float lead_bits(double v, int top) {
+    const int hi = __double2hiint(v), e = (hi >> 20) - top + 126;
+    return e > 0 && hi >= 0x00100000 ? __int_as_float(e << 23 | (hi & 0xfffff) << 3) : 0.0f;
+}
+
+// The parts h0, h1 of a cell's inside towards either side.  in: its conductance; the rest are lead_bits: inf the same,
+// b0, b1 what the two pairs of children conduct outwards, t0, t1 across.  An inside without any conductance
+// counts as none: beyond it lie dead cells, or a known row, whose couplings are on the diagonal.
+__device__ __forceinline__ void co_split(double in, float inf, float b0, float t0, float b1, float t1, int top, double& h0,
+                                         double& h1) {
+    if (__double2hiint(in) <= 0) return;
+    const float a0 = b0 + t0, a1 = b1 + t1, m = CO_MIX * fminf(a0, a1), s0 = a0 + m, s1 = a1 + m, s = s0 + s1;
+    const float part = s > 0.0f ? s1 / s : 0.5f, detour = CO_DETOUR * fminf(fminf(t0, t1), fmaxf(b0, b1));
+    if (inf < detour && top < 2045) in = (double)detour * __hiloint2double((top + 1) << 20, 0);
+    const double g = __double2hiint(in) > 0x01a56e1f ? 1.0 / in : 1e300;  // in above 1e-300
+    h0 = (double)part * g;
+    h1 = (double)(1.0f - part) * g;
+}
+
 __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, const double* __restrict__ txf,
                                                           const double* __restrict__ tyf, int n1c, int n2c,
                                                           double* __restrict__ txc, double* __restrict__ tyc,
@@ -260,55 +283,49 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
         if (2 * I + 1 < n1f) v += tyf[IX(2 * I + 1, fj, n2f + 1)];
         return v;
     };
-    // all three faces across one fine row (column) of a coarse cell
-    auto row_y = [&](int i, int J) {
-        double v = tyf[IX(i, 2 * J, n2f + 1)] + tyf[IX(i, 2 * J + 1, n2f + 1)];
-        if (2 * J + 1 < n2f) v += tyf[IX(i, 2 * J + 2, n2f + 1)];
-        return v;
-    };
-    auto col_x = [&](int I, int j) {
-        double v = txf[IX(2 * I, j, n2f)] + txf[IX(2 * I + 1, j, n2f)];
-        if (2 * I + 1 < n1f) v += txf[IX(2 * I + 2, j, n2f)];
-        return v;
-    };
-    // The inside between children that conduct b0, b1 outwards and t0, t1 across: the parts towards either
-    // side.  One without any conductance counts as none: beyond it lie dead cells, or a known row, whose
-    // couplings are on the diagonal.  One division unless the operands are far out of the ordinary.
-    auto split = [&](double in, double b0, double t0, double b1, double t1, double& h0, double& h1) {
-        if (!(in > 0.0)) return;
-        const double a0 = b0 + t0, a1 = b1 + t1, m = CO_MIX * fmin(a0, a1), s0 = a0 + m, s1 = a1 + m, s = s0 + s1;
-        const double g = fmax(CO_DETOUR * fmin(t0, t1), in), d = s * g;
-        if (d > 1e-290 && d < 1e290) {
-            const double e = 1.0 / d;
-            h0 = s1 * e;
-            h1 = s0 * e;
-        } else {
-            const double e = fmin(1.0 / g, 1e300), part = s > 1e-290 ? s1 / s : 0.5;
-            h0 = part * e;
-            h1 = e - h0;
-        }
-    };
-    auto half_x = [&](int I, int J, double& h0, double& h1) {
-        h0 = h1 = 0.0;
-        if (!plain && I >= 0 && J < n2c && 2 * I + 1 < n1f)
-            split(pair_x(2 * I + 1, J), pair_x(2 * I, J), row_y(2 * I, J), pair_x(2 * I + 2, J), row_y(2 * I + 1, J), h0, h1);
-    };
-    auto half_y = [&](int I, int J, double& h0, double& h1) {
-        h0 = h1 = 0.0;
-        if (!plain && J >= 0 && I < n1c && 2 * J + 1 < n2f)
-            split(pair_y(I, 2 * J + 1), pair_y(I, 2 * J), col_x(I, 2 * J), pair_y(I, 2 * J + 2), col_x(I, 2 * J + 1), h0, h1);
+    // the parts of a coarse cell's inside towards either side, in x and in y
+    auto split = [&](int I, int J, double& x0, double& x1, double& y0, double& y1) {
+        x0 = x1 = y0 = y1 = 0.0;
+        if (plain || I < 0 || J < 0 || I >= n1c || J >= n2c) return;
+        const bool two_i = 2 * I + 1 < n1f, two_j = 2 * J + 1 < n2f;
+        double X[3][2], Y[2][3];  // the cell's fine faces: x-faces 2 I + e of its columns, y-faces 2 J + e of its rows
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int f = 0; f < 2; ++f) {
+                X[e][f] = (e < 2 || two_i) && (f == 0 || two_j) ? txf[IX(2 * I + e, 2 * J + f, n2f)] : 0.0;
+                Y[f][e] = (f == 0 || two_i) && (e < 2 || two_j) ? tyf[IX(2 * I + f, 2 * J + e, n2f + 1)] : 0.0;
+            }
+        int top = 0;  // the largest exponent
+        float x[3][2], y[2][3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int f = 0; f < 2; ++f) top = max(top, max(__double2hiint(X[e][f]), __double2hiint(Y[f][e])));
+        top >>= 20;
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int f = 0; f < 2; ++f) {
+                x[e][f] = lead_bits(X[e][f], top);
+                y[f][e] = lead_bits(Y[f][e], top);
+            }
+        const float tx0 = y[0][0] + y[0][1] + y[0][2], tx1 = y[1][0] + y[1][1] + y[1][2];
+        const float ty0 = x[0][0] + x[1][0] + x[2][0], ty1 = x[0][1] + x[1][1] + x[2][1];
+        if (two_i) co_split(X[1][0] + X[1][1], x[1][0] + x[1][1], x[0][0] + x[0][1], tx0, x[2][0] + x[2][1], tx1, top, x0, x1);
+        if (two_j) co_split(Y[0][1] + Y[1][1], y[0][1] + y[1][1], y[0][0] + y[1][0], ty0, y[0][2] + y[1][2], ty1, top, y0, y1);
     };
     // each thread its own cell, then some a cell of the ring (the small levels are bound by latency: two short
     // chains side by side and one more instead of four in a row)
     const int r = threadIdx.y, q = threadIdx.x, I = I0 + r, J = J0 + q;
-    half_x(I, J, hx0[r + 1][q], hx1[r + 1][q]);
-    half_y(I, J, hy0[r][q + 1], hy1[r][q + 1]);
+    split(I, J, hx0[r + 1][q], hx1[r + 1][q], hy0[r][q + 1], hy1[r][q + 1]);
+    double unused0, unused1;
     if (t < 2 * CO_C) {
         const int a = t / CO_C * (CO_R + 1), c = t % CO_C;
-        half_x(I0 - 1 + a, J0 + c, hx0[a][c], hx1[a][c]);
+        split(I0 - 1 + a, J0 + c, hx0[a][c], hx1[a][c], unused0, unused1);
     } else if (t < 2 * CO_C + 2 * CO_R) {
         const int a = (t - 2 * CO_C) % CO_R, c = (t - 2 * CO_C) / CO_R * (CO_C + 1);
-        half_y(I0 + a, J0 - 1 + c, hy0[a][c], hy1[a][c]);
+        split(I0 + a, J0 - 1 + c, unused0, unused1, hy0[a][c], hy1[a][c]);
     }
     __syncthreads();
     auto face_x = [&](int r, int q, bool store) {  // a face on the far side of the tile is the next tile's, except the last one
@@ -351,8 +368,9 @@ __global__ void __launch_bounds__(CO_C * CO_R) k_coarsen5(int n1f, int n2f, cons
     if (w4) {
         double w[4] = {hx1[r + 1][q] * cx[r + 1][q], hx0[r + 1][q] * cx[r][q], hy1[r][q + 1] * cy[r][q + 1],
                        hy0[r][q + 1] * cy[r][q]};
-        const double X = fmax(w[0], w[1]), Y = fmax(w[2], w[3]);
-        if (X + Y > 1.0) {
+        const float wf[4] = {lead_bits(w[0], 1023), lead_bits(w[1], 1023), lead_bits(w[2], 1023), lead_bits(w[3], 1023)};
+        if (fmaxf(wf[0], wf[1]) + fmaxf(wf[2], wf[3]) > 0.5f) {  // halves: lead_bits scales by 1 / 2
+            const double X = fmax(w[0], w[1]), Y = fmax(w[2], w[3]);
             const double x = fmax(1.0 - X, 1e-300), y = fmax(1.0 - Y, 1e-300), d = fma(X, y, Y * x);
             const double fx = y / d, fy = x / d;  // X fx : Y fy = X / (1 - X) : Y / (1 - Y)
             w[0] *= fx; w[1] *= fx; w[2] *= fy; w[3] *= fy;
