@@ -2485,7 +2485,7 @@ extern "C" impec_status impec_time_kernel_cold(impec_ctx* ctx, int which, int re
                                                double* ms, double* ms_min, double* bytes) {
     if (!ctx || reps <= 0 || which < 0 || which > 1 || !flush || !flush_bytes) return IMPEC_ERR_ARG;
     Level& F = ctx->L[0];
-    if (F.kind != FACE5) return IMPEC_ERR_ARG;
+    if (F.kind != FACE5 || F.a9) return IMPEC_ERR_ARG;  // five-point systems only
     const double n = (double)F.n();
     if (which == 1 && ctx->P.precision != IMPEC_PREC_MIXED) {  // FP32 copies of the fine level
         const int nb = ctx->num_sms * 4;

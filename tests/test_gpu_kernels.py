@@ -502,3 +502,19 @@ def test_cluster_takes_every_schedule(engine, monkeypatch, N1, N2, prec, env):
     assert np.isfinite(out[0][1]) and out[0][:2] == out[1][:2]
     assert np.array_equal(out[0][2], out[1][2])
     assert out[1][3] < out[0][3]
+
+
+@pytest.mark.parametrize("nu,ok", [(1.0, True), (0.9, False), (0.5, False), (0.25, False)])
+def test_cold_sweep_timing_is_for_five_point_systems(engine, nu, ok):
+    """Nine-point systems are refused, whatever levels precondition them."""
+    import ctypes as C
+
+    import torch
+    E = engine
+    ctx = E.Context(E.default_params(96, 96, stype=1, nu=nu))
+    flush = torch.zeros(1 << 20, device="cuda")
+    ms, best, b = C.c_double(), C.c_double(), C.c_double()
+    st = E.lib().impec_time_kernel_cold(ctx.h, 0, 1, C.c_void_p(flush.data_ptr()), flush.numel() * 4, C.byref(ms), C.byref(best),
+                                        C.byref(b))
+    assert (st == 0) == ok
+    ctx.close()
