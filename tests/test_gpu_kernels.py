@@ -518,3 +518,32 @@ def test_cold_sweep_timing_is_for_five_point_systems(engine, nu, ok):
                                         C.byref(b))
     assert (st == 0) == ok
     ctx.close()
+
+
+@pytest.mark.parametrize("N1,N2,stype", [(300, 130, 1), (515, 333, 1), (97, 70, 2), (1024, 1024, 1)])
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("pre,post", [(2, 2), (1, 1), (2, 1)])
+def test_one_launch_sweeps_under_cg(engine, monkeypatch, N1, N2, stype, prec, pre, post):
+    """The default schedule of a CG solve runs half cycles in one launch; with any other one the levels sweep by colour or, from
+    the tile thresholds on, both colours in one launch (from x = 0 as well).  Either way the same bits."""
+    import torch
+
+    from helpers import dev, host
+    E = engine
+    monkeypatch.setenv("IMPEC_MG_PRE", str(pre))
+    monkeypatch.setenv("IMPEC_MG_POST", str(post))
+    c = np.random.default_rng(12).uniform(0.0, 1.0, (N1, N2))
+    out = []
+    for tile in ("0", "1"):
+        monkeypatch.setenv("IMPEC_MG_TILE_CELLS", tile)
+        monkeypatch.setenv("IMPEC_MG_TILE_CELLS32", tile)
+        P = E.default_params(N1, N2, stype=stype, nu=1.0, precision=prec, max_cycles=200)
+        ctx = E.Context(P)
+        ctx.set_source(dev(source(oparams(P))))
+        p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+        n0 = E.launch_count(ctx)
+        cyc, rr, _ = ctx.pressure_solve(dev(c), p, 1e-10)
+        out.append((cyc, rr, host(p), E.launch_count(ctx) - n0))
+        ctx.close()
+    assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
+    assert out[1][3] < out[0][3]
