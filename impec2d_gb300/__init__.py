@@ -159,12 +159,14 @@ def time_kernel(ctx, which: int, reps: int = 20):
 
 def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = None, traffic_path: str | None = None,
                    reps: int = 20):
-    """Achieved bandwidth of a red-black sweep of the finest level (two colours by the per-level sweep
-    kernels; inside a CG solve the half-cycle kernels do the same arithmetic) against the measured HBM copy bandwidth, and its FP64 operation rate against the measured DFMA rate.
+    """Achieved bandwidth of the finest level's two half cycles (pre-smoothing, residual and restriction;
+    prolongation and post-smoothing), the dominant kernels of a pressure solve, against the measured HBM
+    copy bandwidth, and their FP64 operation rate against the measured DFMA rate.  Where a solve runs that
+    level otherwise (grids of one cluster launch, other schedules) a red-black sweep by the per-level kernels stands in.
     Each repetition is timed cold: L2 is overwritten first (``flush``, a CUDA tensor larger
-    than L2), then CUDA events on the engine's stream bracket the sweep.  Algorithmic bytes
-    follow the five-point model: x read and written, b, and the two face planes (40 B per cell in
-    FP64).  ``traffic`` (DRAM bytes per sweep) comes from the ncu capture recorded in
+    than L2), then CUDA events on the engine's stream bracket the launches.  Algorithmic bytes:
+    104 B per cell in FP64 for the half cycles (both read b, 1/diag, both face planes and the transfer weights), 40
+    for a sweep.  ``traffic`` (DRAM bytes) comes from the ncu capture recorded in
     profiles/traffic.json when that file names the kernel and grid."""
     import json
     which = 1 if precision == "mixed" else 0
@@ -181,8 +183,13 @@ def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = 
         import torch
         flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
     ms, ms_min, b = C.c_double(), C.c_double(), C.c_double()
-    _chk(lib().impec_time_kernel_cold(ctx.h, which, reps, C.c_void_p(flush.data_ptr()), flush.numel() * flush.element_size(),
-                                      C.byref(ms), C.byref(ms_min), C.byref(b)), "time_kernel_cold")
+
+    def cold(w):
+        return lib().impec_time_kernel_cold(ctx.h, w, reps, C.c_void_p(flush.data_ptr()), flush.numel() * flush.element_size(),
+                                            C.byref(ms), C.byref(ms_min), C.byref(b))
+    half = cold(which + 2) == 0
+    if not half:
+        _chk(cold(which), "time_kernel_cold")
     ms, ms_min, b = ms.value, ms_min.value, b.value
     peak, src = 6800.0, "fallback"
     path = peaks_path or os.path.join(os.path.dirname(HERE), "MEASURED_PEAKS.json")
@@ -197,11 +204,19 @@ def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = 
         tile = ctx.get_tuning("tile_cells32")
     one_launch = tile > 0 and P.N1 * P.N2 >= tile
     t = "double" if which == 0 else "float"
-    name = (f"k_rb_tile<{t}> (fine red-black sweep, both colours in one launch)" if one_launch
-            else f"k_rb_face5<{t}> (fine red-black sweep, one launch per colour)")
+    march = which == 1 and P.N1 * P.N2 >= 3 << 18
+    if half:
+        name = (f"k_down5{'_march' if march else f'<{t}>'} and k_up5{'_march' if march else f'<{t}>'} "
+                "(the finest level's half cycles)")
+    elif one_launch:
+        name = f"k_rb_tile<{t}> (fine red-black sweep, both colours in one launch)"
+    else:
+        name = f"k_rb_face5<{t}> (fine red-black sweep, one launch per colour)"
+    model = "down: b, 1/diag, tx, ty, half the diagonal, weights; half x and coarse b written; up: the same with half x read " \
+        "and x written" if half else "x r+w, b, tx, ty"
     out = {"bound": "hbm", "kernel": name, "grid": f"{P.N1}x{P.N2}", "achieved": ach, "peak": peak, "unit": "GB/s",
-           "frac": ach / peak, "peak_source": src, "bytes_per_launch": b, "bytes_model": "x r+w, b, tx, ty",
-           "ms_per_launch": ms, "ms_per_launch_min": ms_min, "timing": "cold (L2 overwritten before each sweep)",
+           "frac": ach / peak, "peak_source": src, "bytes_per_launch": b, "bytes_model": model,
+           "ms_per_launch": ms, "ms_per_launch_min": ms_min, "timing": "cold (L2 overwritten before each repetition)",
            "traffic": None}
     tpath = traffic_path or os.path.join(os.path.dirname(HERE), "profiles", "traffic.json")
     if os.path.exists(tpath):
@@ -213,7 +228,9 @@ def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = 
         except Exception:  # noqa: BLE001
             pass
     if which == 0:
-        ops = 5.0 * float(P.N1) * float(P.N2)  # 4 DFMA + 1 DMUL per cell (ncu instruction counts)
+        # a sweep: 4 DFMA + 1 DMUL per cell; half cycles: 10.25 (a colour from zero, two colours, half a residual, the
+        # restriction) and 10 (half a prolongation, three colours), without what the tiles' halos repeat
+        ops = (20.25 if half else 5.0) * float(P.N1) * float(P.N2)
         fma = measure_fp64()
         out["fp64"] = {"achieved_ops_per_s": ops / (ms * 1e-3), "peak_ops_per_s": fma,
                        "frac": ops / (ms * 1e-3) / fma, "ops_per_launch": ops,

@@ -1693,6 +1693,12 @@ static bool fused_level(impec_ctx* ctx, size_t l) {
            ctx->tune.rb_resid != 0;
 }
 
+// Whether a CG solve runs level l in half cycles: not inside the cluster or the single-CTA cycle.
+template <class T>
+static bool half_cycles(impec_ctx* ctx, size_t l) {
+    return fused_level<T>(ctx, l) && l + 1 < ctx->L.size() && l < coarse_start<T>(ctx) && l < cluster_start<T>(ctx);
+}
+
 template <class T, int TR, int TC>
 static void launch_down_up(impec_ctx* ctx, Level& F, Level& C, bool down, T* xc, const unsigned char* mask) {
     const T *tx, *ty, *a9, *id, *tx_, *ty_, *a9_, *id_;
@@ -2483,17 +2489,24 @@ using namespace impec;
 // runs between two events on that stream.  *ms: mean over the repetitions, *ms_min: the fastest.
 extern "C" impec_status impec_time_kernel_cold(impec_ctx* ctx, int which, int reps, void* flush, size_t flush_bytes,
                                                double* ms, double* ms_min, double* bytes) {
-    if (!ctx || reps <= 0 || which < 0 || which > 1 || !flush || !flush_bytes) return IMPEC_ERR_ARG;
+    if (!ctx || reps <= 0 || which < 0 || which > 3 || !flush || !flush_bytes) return IMPEC_ERR_ARG;
     Level& F = ctx->L[0];
     if (F.kind != FACE5 || F.a9) return IMPEC_ERR_ARG;  // five-point systems only
+    const bool half = which >= 2;
+    if (half && !(which == 2 ? half_cycles<double>(ctx, 0) : half_cycles<float>(ctx, 0))) return IMPEC_ERR_ARG;
     const double n = (double)F.n();
-    if (which == 1 && ctx->P.precision != IMPEC_PREC_MIXED) {  // FP32 copies of the fine level
+    if (which % 2 == 1 && ctx->P.precision != IMPEC_PREC_MIXED) {  // FP32 copies of the fine level
         const int nb = ctx->num_sms * 4;
         launch_k(ctx->stream, k_to_float, nb, 256, 0, (size_t)(F.n1 + 1) * F.n2, F.tx, F.tx32);
         launch_k(ctx->stream, k_to_float, nb, 256, 0, (size_t)F.n1 * (F.n2 + 1), F.ty, F.ty32);
         launch_k(ctx->stream, k_to_float, nb, 256, 0, F.n(), F.idiag, F.idiag32);
         launch_k(ctx->stream, k_to_float, nb, 256, 0, F.n(), F.b, F.b32);
         launch_k(ctx->stream, k_to_float, nb, 256, 0, F.n(), F.x, F.x32);
+        if (half) {
+            Level& C = ctx->L[1];
+            launch_k(ctx->stream, k_to_float, nb, 256, 0, F.n(), F.diag, F.diag32);
+            launch_k(ctx->stream, k_to_float, nb, 256, 0, 4 * C.n(), C.w4, C.w432);
+        }
         IMPEC_LAUNCH_CHECK();
     }
     cudaEvent_t e0, e1;
@@ -2504,7 +2517,12 @@ extern "C" impec_status impec_time_kernel_cold(impec_ctx* ctx, int which, int re
         IMPEC_CUDA_TRY(cudaMemsetAsync(flush, r & 0xff, flush_bytes, ctx->stream));
         IMPEC_CUDA_TRY(cudaEventRecord(e0, ctx->stream));
         if (which == 0) smooth<double>(ctx, F, 2, 0);
-        else smooth<float>(ctx, F, 2, 0);
+        else if (which == 1) smooth<float>(ctx, F, 2, 0);
+        else
+            for (int down = 1; down >= 0; --down) {
+                if (which == 2) launch_half<double>(ctx, F, ctx->L[1], down != 0, nullptr, nullptr);
+                else launch_half<float>(ctx, F, ctx->L[1], down != 0, nullptr, nullptr);
+            }
         IMPEC_CUDA_TRY(cudaEventRecord(e1, ctx->stream));
         IMPEC_CUDA_TRY(cudaEventSynchronize(e1));
         float t = 0;
@@ -2516,8 +2534,11 @@ extern "C" impec_status impec_time_kernel_cold(impec_ctx* ctx, int which, int re
     cudaEventDestroy(e1);
     if (ms) *ms = tot / reps;
     if (ms_min) *ms_min = best;
-    // algorithmic bytes of one five-point sweep: x read and written, b, and the two face planes
-    if (bytes) *bytes = n * (which == 0 ? 8.0 : 4.0) * 5.0;
+    // algorithmic bytes in values per cell.  A five-point sweep: x read and written, b, and the two face planes.
+    // Half cycles: both read b, 1/diag, the face planes and four weights of a quarter as many cells; down also
+    // half the diagonal, and writes half the iterate and the coarse right-hand side; up reads half the iterate and
+    // the coarse iterate, and writes the iterate.
+    if (bytes) *bytes = n * (which % 2 == 0 ? 8.0 : 4.0) * (half ? 6.25 + 6.75 : 5.0);
     return IMPEC_OK;
 }
 

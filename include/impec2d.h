@@ -264,12 +264,13 @@ impec_status impec_learned_target(impec_ctx* ctx, float* T);
 /* Step length of the last solve's learned correction (0: rejected). */
 impec_status impec_learned_alpha(impec_ctx* ctx, double* alpha);
 
-/* Cold timing of one fine-level smoother sweep (which 0: FP64, 1: FP32; five-point levels):
- * before each of `reps` repetitions `flush_bytes` of the device buffer `flush` are overwritten
- * on the context's stream, so the sweep's data comes from HBM; each repetition is timed with
- * events on that stream.  *ms: mean, *ms_min: fastest, *bytes: the sweep's algorithmic bytes (x
- * read and written, b, the two face planes).  A benchmark probe; no counterpart in the
- * reference. */
+/* Cold timing on the finest level of a five-point system: one smoother sweep (which 0: FP64, 1: FP32)
+ * or the two half cycles that a CG solve of the default schedule runs there, down and up (which 2: FP64,
+ * 3: FP32; an argument error where such a solve runs the level otherwise).  Before each of `reps` repetitions
+ * `flush_bytes` of the device buffer `flush` are overwritten on the context's stream, so the data comes
+ * from HBM; each repetition is timed with events on that stream.  *ms: mean, *ms_min: fastest,
+ * *bytes: the algorithmic bytes (a sweep: x read and written, b, the two face planes; half cycles: 13 values
+ * per cell).  A benchmark probe; no counterpart in the reference. */
 impec_status impec_time_kernel_cold(impec_ctx* ctx, int which, int reps, void* flush, size_t flush_bytes,
                                     double* ms, double* ms_min, double* bytes);
 
