@@ -50,7 +50,7 @@ def parse():
     ap.add_argument("--later-after", type=int, default=1000,
                     help="time a second window of --steps steps after this many IMPES steps (0: skip)")
     ap.add_argument("--no-large-roofline", action="store_true",
-                    help="skip the 4096^2 roofline probe of the finest level's half cycles")
+                    help="skip the 4096^2 roofline probe of the finest level's sweeps")
     ap.add_argument("--no-learned", action="store_true",
                     help="skip the in-run training of the warm-start network for the pressure-solve line")
     ap.add_argument("--no-graph", action="store_true",
@@ -357,7 +357,8 @@ def study_pressure(args):
 def study_sweep(args):
     """The finest level of the bench workload at --n (default 4096): one pressure solve on the
     workload's initial state (kernel by kernel, so profilers see each launch), then the cold roofline
-    probe: the half cycles of the default schedule, and for V(2,2) the one-launch and the two-launch sweeps."""
+    probe: the default (half cycles, or one-launch sweeps where the FP64 level streams from HBM), half cycles, and
+    for V(2,2) the one-launch and the two-launch sweeps."""
     import numpy as np
     import torch
 
@@ -367,7 +368,7 @@ def study_sweep(args):
     N = args.n or 4096
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
     out = {"study": "sweep", "grid": f"{N}x{N}", "precision": args.precision}
-    for name, sched in (("half_cycles", {}), ("one_launch", {"mg_pre": 2, "mg_post": 2}),
+    for name, sched in (("default", {}), ("half_cycles", {"tile_cells": 0}), ("one_launch", {"mg_pre": 2, "mg_post": 2}),
                         ("two_launch", {"mg_pre": 2, "mg_post": 2, "tile_cells": 0})):
         P = workload_params(E, N, args.precision, args.nu)
         ctx = E.Context(P)
@@ -793,9 +794,10 @@ def main():
     pressure = pressure_solves(E, ctx, N, q, args, flush)
 
     roof_small = E.roofline_probe(ctx, P, args.precision, flush=flush)
-    # The dominant kernels' HBM roofline: the finest level's FP64 half cycles where their data cannot stay
-    # in L2, at 4096^2 (the mixed-precision case's grid).  Inside the 1024^2 step they run from
-    # L2 (the whole hierarchy, ~150 MB, is about L2's size); their cold figure is kept beside it.
+    # The HBM roofline of the finest level's FP64 kernels where their data cannot stay in L2, at 4096^2
+    # (the mixed-precision case's grid): the one-launch sweeps that a solve runs there.  Inside the 1024^2
+    # step that level runs its half cycles from L2 (the whole hierarchy, ~150 MB, is about L2's size);
+    # their cold figure is kept beside it.
     roof_large = None
     if not args.no_large_roofline and args.nu == 1.0:
         NL = 4096
@@ -819,7 +821,7 @@ def main():
             "pressure_solve_1e-10": pressure, "gpu_launches": int(launches), "clocks": clk,
             "roofline": roof_large or roof_small}
     if roof_large:
-        roof_large["why_this_grid"] = ("HBM can bound these kernels only where their level does not fit L2; inside the "
+        roof_large["why_this_grid"] = ("HBM can bound the finest level only where it does not fit L2; inside the "
                                        f"{N}^2 step the level is L2-resident (roofline_{N} holds its cold figure)")
         line[f"roofline_{N}"] = roof_small
     if e2e:

@@ -162,7 +162,8 @@ def roofline_probe(ctx, P, precision: str, flush=None, peaks_path: str | None = 
     """Achieved bandwidth of the finest level's two half cycles (pre-smoothing, residual and restriction;
     prolongation and post-smoothing), the dominant kernels of a pressure solve, against the measured HBM
     copy bandwidth, and their FP64 operation rate against the measured DFMA rate.  Where a solve runs that
-    level otherwise (grids of one cluster launch, other schedules) a red-black sweep by the per-level kernels stands in.
+    level otherwise (large FP64 levels, grids of one cluster launch, other schedules) a red-black sweep by the
+    per-level kernels stands in.
     Each repetition is timed cold: L2 is overwritten first (``flush``, a CUDA tensor larger
     than L2), then CUDA events on the engine's stream bracket the launches.  Algorithmic bytes:
     104 B per cell in FP64 for the half cycles (both read b, 1/diag, both face planes and the transfer weights), 40

@@ -173,12 +173,13 @@ struct Tuning {
     long rb_skip = 1;  // five-point levels: no zero fill before pre-smoothing, red-only prolongation
     long rb_resid = 1;  // five-point levels: restriction sums the red residuals only (black ones are ~0)
     // FP64 five-point levels of at least this many cells sweep both colours in one launch (k_rb_tile,
-    // ping-pong iterate) where a half cycle is not one launch anyway (pressure.cu, fused_level: CG with
-    // the default schedule): every coefficient is read once per sweep instead of once per colour, which
-    // pays where the level streams from HBM (4096^2 sweep 185 against 240 us cold) and costs where it sits
-    // in L2 (1024^2 solve 2.23 against 2.08 ms with every level so swept); 0 disables
+    // ping-pong iterate) instead of running half cycles (pressure.cu, fused_level): every coefficient is read once
+    // per sweep instead of once per colour, which pays where the level streams from HBM (4096^2 sweep 185
+    // against 240 us cold) and costs where it sits in L2 (1024^2 solve 2.23 against 2.08 ms with
+    // every level so swept); 0 disables
     long tile_cells = 1L << 22;
-    // the same for FP32 levels (mixed precision): 4096^2 cold sweep 110 against 130 us
+    // the same for FP32 levels (mixed precision) that do not run half cycles anyway: 4096^2 cold sweep 110
+    // against 130 us
     long tile_cells32 = 1L << 22;
 };
 }  // namespace impec

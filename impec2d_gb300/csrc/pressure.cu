@@ -1686,8 +1686,12 @@ static bool zero_start_free(impec_ctx* ctx, size_t l) {
 
 // Whether a half cycle of level l is one launch (mglevel.cuh): per-level five-point kernels with the
 // default three colours on either side, starting from x = 0 (CG), with both red-black shortcuts.
+// FP64 levels that stream from HBM keep the one-launch sweeps (use_tile): there the halo's repeated operations
+// cost more than the saved traffic (FP64 solve, half cycles / sweeps: 4096^2 21.1 / 20.0 ms from a uniform field and
+// 24.6 / 23.4 from a front; 2048^2 6.49 / 6.49).
 template <class T>
 static bool fused_level(impec_ctx* ctx, size_t l) {
+    if (sizeof(T) == 8 && use_tile<T>(ctx, l)) return false;
     const Colours c = colours(ctx);
     return ctx->krylov && ctx->L[l].kind == FACE5 && c.npre == LV_N && c.npost == LV_N && ctx->tune.rb_skip != 0 &&
            ctx->tune.rb_resid != 0;
