@@ -6,9 +6,14 @@
 // every non-pinned row has zero row sum, so with b~ = b except b~(pin) = -sum_{k != pin} b(k)
 // the singular Neumann system A_N x = b~ is consistent; any solution shifted by
 // (p_pin - x_pin) satisfies all rows of the pinned system.  The consistent singular system is
-// solved by geometric multigrid (cell-centred, Galerkin coarse operators from 2x2
-// aggregation scaled by 1/2, red-black / four-colour Gauss-Seidel, summed restriction,
-// bilinear prolongation, dense coarsest solve with one unknown fixed).
+// solved by conjugate gradients with one geometric multigrid cycle as preconditioner (cell-centred, 2x2
+// aggregation, a dense pseudo-inverse on the coarsest level):
+//   five-point levels (nu = 1, and the preconditioner of nu >= 1/2): coarse faces as series conductances,
+//     flux-weighted prolongation and its transpose (k_coarsen5), red-black Gauss-Seidel, a symmetric cycle;
+//   nine-point levels (nu < 1/2, Dirichlet rows): Galerkin sums scaled by 1/2 (k_exp9_coarsen), summed
+//     restriction, bilinear prolongation, four-colour Gauss-Seidel;
+// or by stationary cycles (IMPEC_MG_KRYLOV=0), whose five-point levels take half the sums of the fine faces,
+// summed restriction and bilinear prolongation.
 //
 // Internally the operator is stored in integrated form with positive diagonal:
 // A_int = -dA * A_ref, f = dA * q, so that ||f - A_int x|| / ||f|| equals the reference's
@@ -1634,8 +1639,9 @@ static bool cluster_plan(impec_ctx* ctx, size_t ls, ClusterArgs<T>& A, size_t& s
 template <class T>
 static size_t cluster_start(impec_ctx* ctx) {
     if (ctx->cl_size < 2 || ctx->tune.cluster == 0) return SIZE_MAX;
-    // FP32 cycles of nine-point systems keep their per-level and single-CTA kernels (with nine-point
-    // levels the cluster costs more: mixed solve at 1024^2, nu = 2/3: 5.10 against 4.76 ms)
+    // FP32 cycles of nine-point systems keep their per-level and single-CTA kernels: with nine-point
+    // levels the cluster costs more (mixed solve at 1024^2, nu = 2/3: 5.10 against 4.76 ms).  With the five-point
+    // levels of nu >= 1/2 neither side has been measured.
     if (sizeof(T) == 4 && ctx->L[0].a9) return SIZE_MAX;
     const long cells = ctx->tune.cl_cells;
     ClusterArgs<T> A;
