@@ -57,12 +57,16 @@ impec_status hyperbolic_capture(impec_ctx* ctx, double* c, const double* u, cons
     return hyperbolic_parts(ctx, c, u, v, dt_dev, pfs, [&](const double* a, double* x) { return capture_cn_solve(ctx, a, x); });
 }
 
-// Host driven.
+// Host driven.  After a failed CN solve c holds the iterate it stopped at.
 impec_status hyperbolic_solve_dev(impec_ctx* ctx, double* c, const double* u, const double* v, const double* dt_dev,
                                   int* pfs) {
     IMPEC_CUDA_TRY(cudaMemsetAsync(&ctx->dscal->flags, 0, sizeof(int), ctx->stream));
-    return hyperbolic_parts(ctx, c, u, v, dt_dev, pfs,
-                            [&](const double* a, double* x) { return cn_solve_host(ctx, a, x, ctx->P.para_eps); });
+    return hyperbolic_parts(ctx, c, u, v, dt_dev, pfs, [&](const double* a, double* x) -> impec_status {
+        const impec_status s = cn_solve_host(ctx, a, x, ctx->P.para_eps);
+        if (s != IMPEC_OK && x != c)
+            IMPEC_CUDA_TRY(cudaMemcpyAsync(c, x, (size_t)ctx->P.N1 * ctx->P.N2 * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+        return s;
+    });
 }
 
 // FP64 maxima and minima by integer comparison: the value's words mapped so that signed order is theirs.

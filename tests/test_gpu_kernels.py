@@ -547,3 +547,26 @@ def test_one_launch_sweeps_under_cg(engine, monkeypatch, N1, N2, stype, prec, pr
         ctx.close()
     assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
     assert out[1][3] < out[0][3]
+
+
+@pytest.mark.parametrize("N1,N2", [(33, 40), (3, 2100)])
+def test_hyperbolic_solve_leaves_the_iterate_of_a_failed_dispersion_solve(engine, N1, N2):
+    """A CN solve that does not converge ends the update; c holds the iterate it stopped at, the one that the
+    dispersion entry point leaves for the same half step (without wells nothing precedes it): the same bits."""
+    import torch
+
+    from helpers import dev, host
+    E = engine
+    rng = np.random.default_rng(3)
+    c, u, v = rng.uniform(0.0, 1.0, (N1, N2)), rng.normal(size=(N1 + 1, N2)), rng.normal(size=(N1, N2 + 1))
+    P = E.default_params(N1, N2, diffusion=1, alpha_l=0.5, alpha_t=0.05, Dm=1e-3, para_eps=1e-30, max_cycles=2)
+    out = []
+    for call in ("hyperbolic_solve", "dispersion_cn"):
+        ctx = E.Context(P)
+        d, dt = dev(c), 1e-4
+        with pytest.raises(E.ImpecError) as e:
+            getattr(ctx, call)(d, dev(u), dev(v), dt if call == "hyperbolic_solve" else 0.5 * dt)
+        torch.cuda.synchronize()
+        out.append((e.value.status, host(d).copy()))
+        ctx.close()
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1]) and not np.array_equal(out[0][1], c)
