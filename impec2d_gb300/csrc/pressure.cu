@@ -1091,7 +1091,7 @@ constexpr size_t MG_CLUSTER_SMEM = 200 * 1024;
 
 // CTAs per cluster for k_cluster_vcycle: 16 where the device can co-schedule such a cluster
 // with the kernel's shared memory, else 8, else 0 (the per-level path is used).
-template <class T, int KIND, bool ANY>
+template <class T, int KIND>
 static int cluster_size_for(int want) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(want);
@@ -1105,7 +1105,7 @@ static int cluster_size_for(int want) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, k_cluster_vcycle<T, KIND, ANY>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&num, k_cluster_vcycle<T, KIND, false>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -1240,13 +1240,12 @@ impec_status pressure_alloc(impec_ctx* ctx) {
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cls) == cudaSuccess &&
                cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     };
-    if (f5 ? allow(k_cluster_vcycle<double, FACE5, false>) && allow(k_cluster_vcycle<float, FACE5, false>) &&
-                 allow(k_cluster_vcycle<double, FACE5, true>) && allow(k_cluster_vcycle<float, FACE5, true>)
+    // (shared memory allows one CTA per SM of either instance: the default one stands for both)
+    if (f5 ? allow(k_cluster_vcycle<double, FACE5, false>) && allow(k_cluster_vcycle<float, FACE5, false>)
            : allow(k_cluster_vcycle<double, EXP9, false>))
         for (int cs = want < CL_MAX_CTAS ? want : CL_MAX_CTAS; cs >= 2 && !ctx->cl_size; cs /= 2)
-            if (f5 ? cluster_size_for<double, FACE5, false>(cs) && cluster_size_for<float, FACE5, false>(cs) &&
-                         cluster_size_for<double, FACE5, true>(cs) && cluster_size_for<float, FACE5, true>(cs)
-                   : cluster_size_for<double, EXP9, false>(cs))
+            if (f5 ? cluster_size_for<double, FACE5>(cs) && cluster_size_for<float, FACE5>(cs)
+                   : cluster_size_for<double, EXP9>(cs))
                 ctx->cl_size = cs;
     cudaGetLastError();
     return IMPEC_OK;
@@ -1674,8 +1673,17 @@ static void launch_cluster(impec_ctx* ctx, size_t ls, bool zero) {
     cfg.numAttrs = ctx->crowd ? 1 : 2;  // with programmatic serialisation (mgcluster.cuh: staging) unless in a crowd
     ++ctx->nlaunch;
     if (ctx->L[ls].kind == FACE5) {
-        if (A.plain || A.zero_color < 0) cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, true>, A);
-        else cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, false>, A);
+        if (A.plain || A.zero_color < 0) {
+            static OncePerDevice once;  // its limits are raised here: few contexts ever launch it
+            once.do_once(ctx->device, cudaSuccess, [] {
+                const auto k = k_cluster_vcycle<T, FACE5, true>;
+                const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MG_CLUSTER_SMEM);
+                return e != cudaSuccess ? e : cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            });
+            cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, true>, A);
+        } else {
+            cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, FACE5, false>, A);
+        }
     } else if constexpr (sizeof(T) == 8) {
         cudaLaunchKernelEx(&cfg, k_cluster_vcycle<T, EXP9, false>, A);
     }
