@@ -570,3 +570,36 @@ def test_hyperbolic_solve_leaves_the_iterate_of_a_failed_dispersion_solve(engine
         out.append((e.value.status, host(d).copy()))
         ctx.close()
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1]) and not np.array_equal(out[0][1], c)
+
+
+@pytest.mark.parametrize("N1,N2,stype", [(515, 333, 1), (1024, 1024, 1), (600, 410, 2)])
+def test_one_launch_sweeps_above_half_cycles(engine, monkeypatch, N1, N2, stype):
+    """A finest FP64 level that streams from HBM sweeps in one launch while the levels below it run half cycles: the bits
+    of half cycles throughout, from the host and from the captured solve."""
+    import torch
+
+    from helpers import dev, host
+    E = engine
+    c = np.random.default_rng(12).uniform(0.0, 1.0, (N1, N2))
+    cg = np.zeros((N1 + 4, N2 + 4))
+    cg[2:-2, 2:-2] = c
+    out = []
+    for tile in (0, N1 * N2):
+        monkeypatch.setenv("IMPEC_MG_TILE_CELLS", str(tile))
+        P = E.default_params(N1, N2, stype=stype, nu=1.0, precision=0, max_cycles=200, eps=1e-10)
+        ctx = E.Context(P)
+        q = source(oparams(P))
+        ctx.set_source(dev(q))
+        p = torch.zeros((N1, N2), dtype=torch.float64, device="cuda")
+        n0 = E.launch_count(ctx)
+        cyc, rr, _ = ctx.pressure_solve(dev(c), p, 1e-10)
+        n = E.launch_count(ctx) - n0
+        ctx.upload(cg, q, ghost=2)
+        res = [ctx.pressure_solve_resident() for _ in range(3)]
+        pr = np.zeros((N1 + 4, N2 + 4))
+        ctx.download(None, pr, None, ghost=2)
+        out.append((cyc, rr, host(p), res, pr, n))
+        ctx.close()
+    assert out[0][:2] == out[1][:2] and out[0][3] == out[1][3]
+    assert np.array_equal(out[0][2], out[1][2]) and np.array_equal(out[0][4], out[1][4])
+    assert out[1][5] > out[0][5]
